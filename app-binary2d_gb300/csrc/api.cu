@@ -18,7 +18,9 @@
 #include "runtime.cuh"
 
 namespace b2d {
-cudaError_t launch_stage_f64(int nf, const StageArgs& a, int grid, int tw, size_t smem, cudaStream_t s);
+cudaError_t launch_stage_f64(int nf, const StageArgs& a, int grid, size_t smem, cudaStream_t s);
+cudaError_t launch_buffer_rate(const RunDev* runs, int run, int N, double* out, cudaStream_t s);
+size_t stage_f64_smem(int nf, int th, int tw);
 cudaError_t launch_stage_f32(int nf, int store, const StageArgs& a, int grid, int tw, size_t smem, cudaStream_t s);
 int stage_ctas_per_sm(int nf, int store, int nruns, int tw);
 void host_block_vertices(const b2d_config* c, int b, double* xv);
@@ -258,6 +260,7 @@ struct RunHost {
     unsigned* counter = nullptr;
     double *xc = nullptr, *xv = nullptr;
     float *xcf = nullptr, *xvf = nullptr, *xvgf = nullptr;
+    double* buffer = nullptr;   // FP64: the buffer's rate of every zone
     double* stage_time = nullptr;
     double* orbit = nullptr;
     double* stage_ds = nullptr;
@@ -281,6 +284,7 @@ struct StagePlan {
 struct b2d_ctx {
     int nruns = 0, nf = 3, precision = 0, hydro = 0, rk = 2;
     int tw = 64, th = 64;
+    int sub_h = 16, sub_w = 32;   // FP64 kernel: the largest sub-tile (f64_sub_tile)
     int strip_rows = 0;   // > 0: the paired FP32 kernel covers column strips in row chunks of at most this many rows
     // a slab advance in progress (b2d_slab_begin .. b2d_slab_end)
     std::vector<StagePlan> slab_plan;
@@ -321,8 +325,6 @@ struct b2d_ctx {
     double stage_ms_total = 0.0;
     long long stage_count = 0;
 };
-
-static int rsize_of(int precision) { return precision == B2D_PREC_FP64 ? 8 : 4; }
 
 static size_t stage_smem_bytes(int nf, int rsize, int tw)
 {
@@ -416,6 +418,54 @@ static int default_tile_w(int bs)
     return bs;
 }
 
+// The FP64 kernel's largest sub-tile for runs of the given block sizes and
+// block counts: the shape whose sub-tiles, dealt evenly to the SMs, take the
+// busiest SM the fewest FP64 operations.  The kernel is bound by each SM's FP64
+// pipe, so large sub-tiles (few guard zones) win until the mesh is too small to
+// give every SM the same share of them.  The weights are the kernel's FP64
+// operations per guard-including zone, slope zone, face and updated zone, and
+// 4000 for a sub-tile's latency between phases; a
+// 16 x 32 sub-tile of Euler zones leaves room for one CTA per SM only, which
+// costs 5 % (1024^2: 1.568 against 1.490 ms a stage).  Measured per stage, by
+// shape 16x32 / 12x32 / 8x32 / 8x16 / 4x16: isothermal 2048^2 3.21 / 3.30 / 3.56
+// / 4.16 / 5.80 ms, 384^2 140 / 182 / 152 / 173 / 236 us; Euler 256^2 129 / 167 /
+// 135 / 149 / 193 us, 128^2 127 / 93 / 79 / 49 / 58 us.
+struct BlockCount { int bs; long long blocks; };
+static void f64_sub_tile(int nf, const std::vector<BlockCount>& runs, int* th, int* tw)
+{
+    constexpr int SMS = 152;
+    const int shapes[5][2] = {{16, 32}, {12, 32}, {8, 32}, {8, 16}, {4, 16}};
+    double best = 1e300;
+    for (const auto& s : shapes) {
+        long long n = 0;
+        double cost = 0.0;
+        for (const BlockCount& r : runs) {
+            const int ni = (r.bs + s[0] - 1) / s[0], nj = (r.bs + s[1] - 1) / s[1];
+            const int h = (r.bs + ni - 1) / ni, w = (r.bs + nj - 1) / nj;
+            n += r.blocks * ni * nj;
+            auto whole = [](int k) { return (k + 31) / 32 * 32; };   // lanes of whole warps
+            cost = std::max(cost, 4000.0 + 15 * whole((h + 4) * (w + 4)) + 31 * whole((h + 2) * (w + 2)) +
+                                      105 * (whole((h + 1) * w) + whole(h * (w + 1))) + 95 * whole(h * w));
+        }
+        if (nf == 4 && s[0] == 16) cost *= 1.05;
+        cost *= n < 8 * SMS ? (double)((n + SMS - 1) / SMS) : (double)n / SMS;
+        if (cost < best) {
+            best = cost;
+            *th = s[0];
+            *tw = s[1];
+        }
+    }
+}
+
+// Split blocks of bs x bs zones evenly into sub-tiles of at most th x tw.
+static void split_blocks(RunDev& d, int bs, int th, int tw, int per_cta)
+{
+    d.sub_i = (bs + th - 1) / th;
+    d.sub_j = (bs + tw - 1) / tw;
+    d.sub_per_cta = per_cta;
+    d.tiles_per_block = (d.sub_i * d.sub_j + per_cta - 1) / per_cta;
+}
+
 static bool tile_ok(const b2d_ctx* ctx, int tw, int th)
 {
     // the paired FP32 kernels' 128-, 256- and 512-column tiles may also span
@@ -443,7 +493,7 @@ static void free_ctx(b2d_ctx* ctx)
         const size_t ri = &r - ctx->runs.data();
         if (ri < ctx->rdev_h.size())
             for (int s = 0; s < NSLOTS; ++s) cudaFree(ctx->rdev_h[ri].tracers[s]);
-        cudaFree(r.bg); cudaFree(r.partial); cudaFree(r.counter);
+        cudaFree(r.buffer); cudaFree(r.bg); cudaFree(r.partial); cudaFree(r.counter);
         cudaFree(r.xc); cudaFree(r.xv); cudaFree(r.xcf); cudaFree(r.xvf); cudaFree(r.xvgf);
         cudaFree(r.stage_time); cudaFree(r.orbit); cudaFree(r.stage_ds); cudaFree(r.stage_de);
     }
@@ -505,6 +555,11 @@ static b2d_status sync_rundev(b2d_ctx* ctx)
         else
             for (int b = 0; b < r.nb; ++b) most = std::max(most, chunks_in_block_row(b, r.bs, r.N, d.chunks));
         d.tiles_per_block = most * std::max(r.bs / ctx->tw, 1);
+        if (ctx->precision == B2D_PREC_FP64) {
+            // the FP64 kernel's CTAs take sub-tiles block by block
+            split_blocks(d, r.bs, ctx->sub_h, ctx->sub_w, 1);
+            d.ntiles = (d.slab_hi > 0 ? d.slab_hi - d.slab_lo : r.nb) * r.nb * d.tiles_per_block;
+        }
         base += d.ntiles;
         CUDA_TRY(cudaFree(r.partial));
         r.partial = nullptr;
@@ -684,7 +739,27 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
         free_ctx(ctx);
         return nullptr;
     }
+    std::vector<BlockCount> counts;
+    for (const RunHost& r : ctx->runs) counts.push_back({r.bs, r.nblocks});
+    f64_sub_tile(ctx->nf, counts, &ctx->sub_h, &ctx->sub_w);
     if (sync_rundev(ctx) != B2D_OK) { *status = B2D_ERR_CUDA; free_ctx(ctx); return nullptr; }
+    if (precision == B2D_PREC_FP64) {
+        // the buffer's rate depends on the zone's place only, and takes an
+        // FP64 root, division and tanh: a table, 8 bytes a zone beside the
+        // run's 144 or 192 (without the memory for it, the stages compute it)
+        for (int i = 0; i < nruns; ++i) {
+            RunHost& r = ctx->runs[i];
+            if (cudaMalloc(&r.buffer, sizeof(double) * (size_t)r.N * r.N) != cudaSuccess) {
+                cudaGetLastError();
+                r.buffer = nullptr;
+                continue;
+            }
+            CREATE_TRY(launch_buffer_rate(ctx->rdev, i, r.N, r.buffer, ctx->stream));
+            ctx->rdev_h[i].buffer = r.buffer;
+        }
+        CREATE_TRY(cudaStreamSynchronize(ctx->stream));
+        CREATE_TRY(cudaMemcpy(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * nruns, cudaMemcpyHostToDevice));
+    }
     if (ensure_stage_capacity(ctx, 16) != B2D_OK) { *status = B2D_ERR_CUDA; free_ctx(ctx); return nullptr; }
     *status = B2D_OK;
     return ctx;
@@ -1065,10 +1140,12 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
     a.err_key = ctx->d_err_key;
     a.timeout_flag = ctx->d_timeout;
     a.pf1 = ctx->rdev_h[0].pf;
-    size_t smem = stage_smem_bytes(ctx->nf, rsize_of(ctx->precision), ctx->tw);
     cudaError_t e;
-    if (ctx->precision == B2D_PREC_FP64) e = launch_stage_f64(ctx->nf, a, ctx->total_tiles, ctx->tw, smem, ctx->stream);
-    else e = launch_stage_f32(ctx->nf, store_of(ctx), a, ctx->total_tiles, ctx->tw, smem, ctx->stream);
+    if (ctx->precision == B2D_PREC_FP64)
+        e = launch_stage_f64(ctx->nf, a, ctx->total_tiles, stage_f64_smem(ctx->nf, ctx->sub_h, ctx->sub_w), ctx->stream);
+    else
+        e = launch_stage_f32(ctx->nf, store_of(ctx), a, ctx->total_tiles, ctx->tw, stage_smem_bytes(ctx->nf, 4, ctx->tw),
+                             ctx->stream);
     if (e != cudaSuccess) return fail(B2D_ERR_CUDA, std::string("stage kernel launch: ") + cudaGetErrorString(e));
     return B2D_OK;
 }
@@ -1645,12 +1722,16 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
     b2d_status st = ensure_stage_capacity(ctx, fold);
     if (st != B2D_OK) return st;
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    const int max_w = ctx->precision == B2D_PREC_FP64 || ctx->precision == B2D_PREC_FP32_COMP ? 256 : 128;
+    const int max_w = ctx->precision == B2D_PREC_FP32_COMP ? 256 : 128;
     int best_w = ctx->tw, best_h = ctx->th, best_rows = 0;
     double best = 1e300;
     ctx->strip_rows = 0;
+    if (ctx->precision == B2D_PREC_FP64) {   // one tiling, whatever the tile shape
+        st = time_tile(ctx, fold, reps, &best);
+        if (st != B2D_OK) return st;
+    }
     for (int w : {32, 64, 128, 256}) {
-        if (w > max_w) continue;
+        if (w > max_w || ctx->precision == B2D_PREC_FP64) continue;
         for (int h : {8, 16, 32, 64, 128}) {
             if (!tile_ok(ctx, w, h)) continue;
             ctx->tw = w;
@@ -1877,20 +1958,29 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     cudaStream_t stream = (cudaStream_t)stream_ptr;
     const int nf = cfg->hydro_kind == B2D_EULER ? 4 : 3;
     const int bs = cfg->block_size, nb = cfg->num_blocks, N = bs * nb, nblocks = nb * nb;
-    int tw = default_tile_w(bs), th = std::min(64, bs);
-    while (bs % th) th /= 2;
-    // one thread per tile column: a block width that is not a multiple of 32
-    // is its own tile, which the FP64 kernel's 256-thread bound must hold
-    if (tw > 256)
+    if (bs % 32 != 0 && bs > 256)
         return fail(B2D_ERR_INVALID, "b2d_stage_noalloc: block_size " + std::to_string(bs) +
                                          " must be a multiple of 32 or at most 256");
-    const int tiles_per_block = (bs / th) * (bs / tw);
-    const int ntiles = (N / th) * (N / tw);
 
-    // scratch layout: run descriptor | control words | counters | tile partials
+    // scratch layout: run descriptor | control words | counters | ledger pieces | geometry tables.  A CTA takes
+    // several sub-tiles of a block where one piece per sub-tile would not fit.
     const size_t off_run = 0, off_ctl = 2048, off_cnt = 2304;
     const size_t off_part = off_cnt + ((sizeof(unsigned) * (size_t)nblocks + 255) / 256) * 256;
-    const size_t need = off_part + sizeof(double) * (size_t)nblocks * tiles_per_block * NITEMS * nf;
+    const size_t geo_bytes = sizeof(double) * ((size_t)N + (size_t)nb * (bs + 1));
+    int sub_h, sub_w;
+    f64_sub_tile(nf, {{bs, nblocks}}, &sub_h, &sub_w);
+    RunDev rd;
+    memset(&rd, 0, sizeof rd);
+    // the meshes taken are those whose pieces would fit at one per default tile
+    int tile_h = std::min(64, bs);
+    while (bs % tile_h) tile_h /= 2;
+    size_t need = off_part + sizeof(double) * (size_t)nblocks * (bs / tile_h) * (bs / default_tile_w(bs)) * NITEMS * nf;
+    const bool fits = (need + 255) / 256 * 256 + geo_bytes <= B2D_NOALLOC_SCRATCH_BYTES;
+    for (int per_cta = 1; fits; per_cta *= 2) {
+        split_blocks(rd, bs, sub_h, sub_w, per_cta);
+        need = off_part + sizeof(double) * (size_t)nblocks * rd.tiles_per_block * NITEMS * nf;
+        if (rd.tiles_per_block == 1 || (need + 255) / 256 * 256 + geo_bytes <= B2D_NOALLOC_SCRATCH_BYTES) break;
+    }
     static_assert(sizeof(RunDev) <= 2048, "run descriptor outgrew its scratch slot");
     if (need > B2D_NOALLOC_SCRATCH_BYTES)
         return fail(B2D_ERR_INVALID, "b2d_stage_noalloc: this mesh needs " + std::to_string(need) +
@@ -1926,12 +2016,8 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     double* d_xc = (double*)(base + off_geo);
     double* d_xv = d_xc + xc.size();
 
-    RunDev rd;
-    memset(&rd, 0, sizeof rd);
     rd.N = N; rd.bs = bs; rd.nb = nb; rd.nblocks = nblocks;
-    rd.tiles_i = N / th; rd.tiles_j = N / tw; rd.ntiles = ntiles; rd.tile_base = 0;
-    rd.chunks = rd.tiles_i; rd.chunk0 = 0;
-    rd.tiles_per_block = tiles_per_block;
+    rd.ntiles = nblocks * rd.tiles_per_block;
     rd.xc = d_xc; rd.xv = d_xv;
     rd.slot[0] = (void*)d_in; rd.slot[1] = (void*)d_base; rd.slot[2] = d_out; rd.slot[3] = d_out;
     rd.bg = d_background;
@@ -1958,7 +2044,7 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     StageArgs a;
     a.runs = d_run;
     a.nruns = 1;
-    a.th = th;
+    a.th = sub_h;
     a.in_slot = 0;
     a.base_slot = d_base ? 1 : -1;
     a.out_slot = 2;
@@ -1969,7 +2055,7 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     a.bff = split_df(a.bf);
     a.err_key = err_key;
     a.timeout_flag = timeout;
-    cudaError_t e = launch_stage_f64(nf, a, ntiles, tw, stage_smem_bytes(nf, 8, tw), stream);
+    cudaError_t e = launch_stage_f64(nf, a, rd.ntiles, stage_f64_smem(nf, sub_h, sub_w), stream);
     if (e != cudaSuccess) return fail(B2D_ERR_CUDA, std::string("stage kernel launch: ") + cudaGetErrorString(e));
     if (d_max_speed) CUDA_TRY(cudaMemcpyAsync(d_max_speed, amax, sizeof(double), cudaMemcpyDeviceToDevice, stream));
 

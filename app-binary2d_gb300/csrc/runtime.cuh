@@ -21,6 +21,9 @@ struct RunDev {
                                  // speed and the orbital-element ledger cover only the slab
     int chunks, pad_;            // row chunks per column strip of the whole run (C of chunk_start);
                                  // tiles_i of them, from chunk0, are launched
+    int sub_i, sub_j;        // FP64 kernel: sub-tiles per block along rows and columns
+    int sub_per_cta;         // and how many of a block's sub-tiles (row-major) one CTA takes, the last one fewer
+    const double* buffer;    // FP64 kernel: [N][N] buffer rate (nullptr: computed where it is used)
     const double* xc;        // [N] cell centres by global index (block formula, mesh.rs:49-54)
     const double* xv;        // [nb][bs+1] block vertices (mesh.rs:42-47)
     const float* xcf;

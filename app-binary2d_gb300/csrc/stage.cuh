@@ -1,4 +1,6 @@
-// stage.cuh — the fused RK-stage kernel.
+// stage.cuh — state access and double-float arithmetic of the stage kernels,
+// and the generic fused RK-stage kernel (FP32 stencil, blocks narrower than a
+// warp or of a ragged width).
 //
 // One launch performs one call of try_advance_rk (src/scheme.rs:88-173) for
 // every run of a context: cons→prim (phase A), PLM slopes and HLLE + viscous

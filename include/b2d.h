@@ -287,7 +287,8 @@ b2d_status b2d_initial_state(const b2d_config* cfg, const b2d_disk_model* model,
  * multiple of 32 dividing block_size) and height along i (dividing
  * block_size).  The paired-column FP32 kernel (precision FP32_COMP,
  * isothermal) also takes 128-, 256- or 512-column tiles that span whole
- * blocks of 64 columns or more side by side.  0 keeps the current value. */
+ * blocks of 64 columns or more side by side.  The FP64 kernel cuts blocks into
+ * sub-tiles of its own and takes any shape here.  0 keeps the current value. */
 b2d_status b2d_set_tile(b2d_ctx* ctx, int32_t tile_w, int32_t tile_h);
 b2d_status b2d_get_tile(const b2d_ctx* ctx, int32_t* tile_w, int32_t* tile_h);
 
@@ -304,8 +305,9 @@ b2d_status b2d_get_tile(const b2d_ctx* ctx, int32_t* tile_w, int32_t* tile_h);
 b2d_status b2d_set_strip_rows(b2d_ctx* ctx, int32_t rows);
 b2d_status b2d_get_strip_rows(const b2d_ctx* ctx, int32_t* rows);
 
-/* Tile autotuner: times every tile shape that divides the block size (width
- * 32..128, or 256 for FP64; height 8..128), the paired FP32 kernel's tiles
+/* Tile autotuner (of the FP32 precisions; an FP64 context is timed once, as it
+ * is): times every tile shape that divides the block size (width
+ * 32..128; height 8..128), the paired FP32 kernel's tiles
  * that span blocks (128, 256 or 512 columns) and, where that kernel runs, the
  * strip rows that fill one, two or three whole waves of its resident CTAs, over `reps` advances of `fold` steps with CUDA events; keeps
  * the fastest (b2d_get_tile and b2d_get_strip_rows report it).  The
