@@ -5,8 +5,8 @@ into app-binary2d_gb300/_build/libb2d.so.  Flags per unit:
 
   kernels_f64.cu   --fmad=false   FP64 parity kernels: every operation rounds as written
   api.cu           --fmad=false   Kepler solve and time bookkeeping in exact FP64
-  kernels_f32.cu   fast FP32      -ftz, approximate division and square root
-  kernels_f32e.cu  fast FP32      the paired Euler kernel, same flags
+  kernels_f32.cu   fast FP32      -ftz, approximate division and square root: the isothermal system
+  kernels_f32e.cu  fast FP32      the Euler system, same flags
   host_ic.cpp      g++ -ffp-contract=off   geometry and initial states
 """
 import concurrent.futures as cf

@@ -21,8 +21,10 @@ namespace b2d {
 cudaError_t launch_stage_f64(int nf, const StageArgs& a, int grid, size_t smem, cudaStream_t s);
 cudaError_t launch_buffer_rate(const RunDev* runs, int run, int N, double* out, cudaStream_t s);
 size_t stage_f64_smem(int nf, int th, int tw);
-cudaError_t launch_stage_f32(int nf, int store, const StageArgs& a, int grid, int tw, size_t smem, cudaStream_t s);
-int stage_ctas_per_sm(int nf, int store, int nruns, int tw);
+cudaError_t launch_stage_f32_iso(int store, bool even, const StageArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_stage_f32_euler(int store, bool even, const StageArgs& a, int grid, cudaStream_t s);
+int resident_f32_iso(int store, bool even, int nruns);
+int resident_f32_euler(int store, bool even, int nruns);
 void host_block_vertices(const b2d_config* c, int b, double* xv);
 void host_cell_centers(const b2d_config* c, int b, double* xc);
 }  // namespace b2d
@@ -259,7 +261,7 @@ struct RunHost {
     double* partial = nullptr;
     unsigned* counter = nullptr;
     double *xc = nullptr, *xv = nullptr;
-    float *xcf = nullptr, *xvf = nullptr, *xvgf = nullptr;
+    float *xcf = nullptr, *xvgf = nullptr;
     double* buffer = nullptr;   // FP64: the buffer's rate of every zone
     double* stage_time = nullptr;
     double* orbit = nullptr;
@@ -285,7 +287,7 @@ struct b2d_ctx {
     int nruns = 0, nf = 3, precision = 0, hydro = 0, rk = 2;
     int tw = 64, th = 64;
     int sub_h = 16, sub_w = 32;   // FP64 kernel: the largest sub-tile (f64_sub_tile)
-    int strip_rows = 0;   // > 0: the paired FP32 kernel covers column strips in row chunks of at most this many rows
+    int strip_rows = 0;   // > 0: the FP32 kernel's strips are cut into row chunks of at most this many rows
     // a slab advance in progress (b2d_slab_begin .. b2d_slab_end)
     std::vector<StagePlan> slab_plan;
     int slab_fold = 0, slab_start = -1, slab_final = -1, slab_next = -1;
@@ -299,7 +301,6 @@ struct b2d_ctx {
     long long* d_iter = nullptr;      // [nruns][NSLOTS]
     unsigned long long* d_amax = nullptr;  // [nruns]
     unsigned long long* d_err_key = nullptr;  // failure key (~0: none)
-    unsigned* d_timeout = nullptr;            // a bounded wait gave up
     long long* d_adv_count = nullptr;       // advances begun without a pending failure
     long long adv_base = 0;
     std::vector<std::pair<int, std::vector<StagePlan>>> window;  // advances since the last check
@@ -325,15 +326,6 @@ struct b2d_ctx {
     double stage_ms_total = 0.0;
     long long stage_count = 0;
 };
-
-static size_t stage_smem_bytes(int nf, int rsize, int tw)
-{
-    int cw = 3 * nf + 4;
-    size_t elems = 4 * (size_t)(tw + 4) * nf + 3 * (size_t)(tw + 2) * cw + 2 * (size_t)(tw + 1) * nf;
-    size_t bytes = elems * rsize;
-    size_t red = (size_t)tw * 8;
-    return std::max(bytes, red);
-}
 
 template <class T> static DevParamsT<T> make_params(const b2d_config& c)
 {
@@ -494,11 +486,11 @@ static void free_ctx(b2d_ctx* ctx)
         if (ri < ctx->rdev_h.size())
             for (int s = 0; s < NSLOTS; ++s) cudaFree(ctx->rdev_h[ri].tracers[s]);
         cudaFree(r.buffer); cudaFree(r.bg); cudaFree(r.partial); cudaFree(r.counter);
-        cudaFree(r.xc); cudaFree(r.xv); cudaFree(r.xcf); cudaFree(r.xvf); cudaFree(r.xvgf);
+        cudaFree(r.xc); cudaFree(r.xv); cudaFree(r.xcf); cudaFree(r.xvgf);
         cudaFree(r.stage_time); cudaFree(r.orbit); cudaFree(r.stage_ds); cudaFree(r.stage_de);
     }
     cudaFree(ctx->rdev); cudaFree(ctx->d_dt); cudaFree(ctx->d_time); cudaFree(ctx->d_iter);
-    cudaFree(ctx->d_amax); cudaFree(ctx->d_err_key); cudaFree(ctx->d_adv_count); cudaFree(ctx->d_timeout); cudaFree(ctx->d_staging);
+    cudaFree(ctx->d_amax); cudaFree(ctx->d_err_key); cudaFree(ctx->d_adv_count); cudaFree(ctx->d_staging);
     for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->up_stream) cudaStreamDestroy(ctx->up_stream);
@@ -512,29 +504,27 @@ static void free_ctx(b2d_ctx* ctx)
     delete ctx;
 }
 
-// Rebuild the tile bookkeeping for the current tile shape and push the run
-// descriptors to the device.
-// The stage kernel the context launches takes row chunks: a paired-column
-// kernel or the TMA-staged one (launch_stage_f32 makes the same choice), not
-// the FP64 or the generic kernel.
-static bool chunk_kernel(const b2d_ctx* ctx)
-{
-    if (ctx->precision == B2D_PREC_FP64) return false;
-    if (ctx->precision == B2D_PREC_FP32_COMP &&
-        (ctx->tw == 64 || ctx->tw == 128 || ctx->tw == 256 || ctx->tw == 512))
-        return true;
-    return ctx->tw % 32 == 0 && ctx->tw <= 128;
-}
+constexpr int TABLE_PAD = 4;     // entries of the FP32 position tables beyond either end
+constexpr int STRIP_COLS = 60;   // SW_COLS of the FP32 kernel (stagew.cuh)
 
 // Row chunks per column strip of a run: block-aligned tiles of height th, or,
-// with strip rows set and a chunk-taking kernel launched, ceil(N / rows)
-// chunks that may cross one block boundary each.
+// with strip rows set, ceil(N / rows) chunks that may cross block boundaries.
 static int row_chunks(const b2d_ctx* ctx, const RunHost& r)
 {
-    if (ctx->strip_rows > 0 && chunk_kernel(ctx)) return (r.N + ctx->strip_rows - 1) / ctx->strip_rows;
+    if (ctx->strip_rows > 0) return (r.N + ctx->strip_rows - 1) / ctx->strip_rows;
     return r.N / ctx->th;
 }
 
+// Every run has an even number of columns: the FP32 kernel stages pairs of them as one word.
+static bool even_columns(const b2d_ctx* ctx)
+{
+    for (const RunHost& r : ctx->runs)
+        if (r.N % 2) return false;
+    return true;
+}
+
+// Rebuild the tile bookkeeping for the current tile shape and push the run
+// descriptors to the device.
 static b2d_status sync_rundev(b2d_ctx* ctx)
 {
     int base = 0;
@@ -545,25 +535,30 @@ static b2d_status sync_rundev(b2d_ctx* ctx)
         d.chunks = d.slab_hi > 0 ? r.N / ctx->th : row_chunks(ctx, r);
         d.chunk0 = d.slab_hi > 0 ? d.slab_lo * (r.bs / ctx->th) : 0;
         d.tiles_i = d.slab_hi > 0 ? (d.slab_hi - d.slab_lo) * (r.bs / ctx->th) : d.chunks;
-        d.tiles_j = r.N / ctx->tw;
-        d.ntiles = d.tiles_i * d.tiles_j;
         d.tile_base = base;
-        // partial slots of the block with the most chunk pieces (every block:
-        // bs / th for block-aligned tiles)
-        int most = 0;
-        if (d.slab_hi > 0) most = r.bs / ctx->th;   // a slab's tiles are block-aligned
-        else
-            for (int b = 0; b < r.nb; ++b) most = std::max(most, chunks_in_block_row(b, r.bs, r.N, d.chunks));
-        d.tiles_per_block = most * std::max(r.bs / ctx->tw, 1);
         if (ctx->precision == B2D_PREC_FP64) {
             // the FP64 kernel's CTAs take sub-tiles block by block
             split_blocks(d, r.bs, ctx->sub_h, ctx->sub_w, 1);
             d.ntiles = (d.slab_hi > 0 ? d.slab_hi - d.slab_lo : r.nb) * r.nb * d.tiles_per_block;
+            base += d.ntiles;
+        } else {
+            // the FP32 kernel's one-warp CTAs take strips x row chunks
+            d.tiles_j = (r.N + STRIP_COLS - 1) / STRIP_COLS;
+            d.ntiles = d.tiles_i * d.tiles_j;
+            base += d.ntiles;
+            // ledger pieces of the block with the most: the chunks of its rows times the strips of its columns
+            int rows = 0, cols = 0;
+            for (int b = 0; b < r.nb; ++b) {
+                rows = std::max(rows, chunks_in_block_row(b, r.bs, r.N, d.chunks));
+                cols = std::max(cols, (b * r.bs + r.bs - 1) / STRIP_COLS - b * r.bs / STRIP_COLS + 1);
+            }
+            d.tiles_per_block = rows * cols;
         }
-        base += d.ntiles;
         CUDA_TRY(cudaFree(r.partial));
         r.partial = nullptr;
-        CUDA_TRY(cudaMalloc(&r.partial, sizeof(double) * r.nblocks * d.tiles_per_block * NITEMS * ctx->nf));
+        const size_t partial_bytes = sizeof(double) * r.nblocks * d.tiles_per_block * NITEMS * ctx->nf;
+        CUDA_TRY(cudaMalloc(&r.partial, partial_bytes));
+        CUDA_TRY(cudaMemset(r.partial, 0, partial_bytes));   // the words of items that are always zero are never written
         d.partial = r.partial;
     }
     ctx->total_tiles = base;
@@ -645,8 +640,6 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
     CREATE_TRY(cudaMalloc(&ctx->d_amax, sizeof(unsigned long long) * nruns));
     CREATE_TRY(cudaMalloc(&ctx->d_err_key, sizeof(unsigned long long)));
     CREATE_TRY(cudaMalloc(&ctx->d_adv_count, sizeof(long long)));
-    CREATE_TRY(cudaMalloc(&ctx->d_timeout, sizeof(unsigned)));
-    CREATE_TRY(cudaMemset(ctx->d_timeout, 0, sizeof(unsigned)));
     CREATE_TRY(cudaMemset(ctx->d_adv_count, 0, sizeof(long long)));
     CREATE_TRY(cudaMemset(ctx->d_time, 0, sizeof(double) * nruns * NSLOTS));
     CREATE_TRY(cudaMemset(ctx->d_iter, 0, sizeof(long long) * nruns * NSLOTS));
@@ -687,24 +680,28 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
             host_block_vertices(&cfgs[i], b, xv.data() + (size_t)b * (r.bs + 1));
         }
         std::vector<float> xcf(xc.begin(), xc.end()), xvf(xv.begin(), xv.end());
+        auto pad = [](std::vector<float>& v) {   // TABLE_PAD entries beyond either end, for row positions read ahead
+            v.insert(v.begin(), TABLE_PAD, v.front());
+            v.insert(v.end(), TABLE_PAD, v.back());
+        };
         // row faces by global index: face k of block k / bs, the last block's top face last
         std::vector<float> xvgf((size_t)r.N + 1);
         for (int k = 0; k < r.N; ++k) xvgf[k] = xvf[(size_t)(k / r.bs) * (r.bs + 1) + k % r.bs];
         xvgf[r.N] = xvf[(size_t)(r.nb - 1) * (r.bs + 1) + r.bs];
+        pad(xcf);
+        pad(xvgf);
         r.hxc = xc;
         CREATE_TRY(cudaMalloc(&r.xc, sizeof(double) * xc.size()));
         CREATE_TRY(cudaMalloc(&r.xv, sizeof(double) * xv.size()));
-        CREATE_TRY(cudaMalloc(&r.xcf, sizeof(float) * xc.size()));
-        CREATE_TRY(cudaMalloc(&r.xvf, sizeof(float) * xv.size()));
+        CREATE_TRY(cudaMalloc(&r.xcf, sizeof(float) * xcf.size()));
         CREATE_TRY(cudaMalloc(&r.xvgf, sizeof(float) * xvgf.size()));
         CREATE_TRY(cudaMemcpy(r.xc, xc.data(), sizeof(double) * xc.size(), cudaMemcpyHostToDevice));
         CREATE_TRY(cudaMemcpy(r.xv, xv.data(), sizeof(double) * xv.size(), cudaMemcpyHostToDevice));
-        CREATE_TRY(cudaMemcpy(r.xcf, xcf.data(), sizeof(float) * xc.size(), cudaMemcpyHostToDevice));
-        CREATE_TRY(cudaMemcpy(r.xvf, xvf.data(), sizeof(float) * xv.size(), cudaMemcpyHostToDevice));
+        CREATE_TRY(cudaMemcpy(r.xcf, xcf.data(), sizeof(float) * xcf.size(), cudaMemcpyHostToDevice));
         CREATE_TRY(cudaMemcpy(r.xvgf, xvgf.data(), sizeof(float) * xvgf.size(), cudaMemcpyHostToDevice));
 
         d.N = r.N; d.bs = r.bs; d.nb = r.nb; d.nblocks = r.nblocks;
-        d.xc = r.xc; d.xv = r.xv; d.xcf = r.xcf; d.xvf = r.xvf; d.xvgf = r.xvgf;
+        d.xc = r.xc; d.xv = r.xv; d.xcf = r.xcf + TABLE_PAD; d.xvgf = r.xvgf + TABLE_PAD;
         for (int s = 0; s < NSLOTS; ++s) {
             d.slot[s] = r.slot[s];
             d.ledger[s] = r.ledger[s];
@@ -1135,17 +1132,17 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
     a.stage = stage;
     a.amax_flag = amax_flag;
     a.bf = sp.bf;
+    a.half_avg = sp.bf == 0.5;
     a.w1f = split_df(-sp.bf + 1.0);
     a.bff = split_df(sp.bf);
     a.err_key = ctx->d_err_key;
-    a.timeout_flag = ctx->d_timeout;
     a.pf1 = ctx->rdev_h[0].pf;
     cudaError_t e;
     if (ctx->precision == B2D_PREC_FP64)
         e = launch_stage_f64(ctx->nf, a, ctx->total_tiles, stage_f64_smem(ctx->nf, ctx->sub_h, ctx->sub_w), ctx->stream);
     else
-        e = launch_stage_f32(ctx->nf, store_of(ctx), a, ctx->total_tiles, ctx->tw, stage_smem_bytes(ctx->nf, 4, ctx->tw),
-                             ctx->stream);
+        e = (ctx->nf == 3 ? launch_stage_f32_iso : launch_stage_f32_euler)(store_of(ctx), even_columns(ctx), a,
+                                                                           ctx->total_tiles, ctx->stream);
     if (e != cudaSuccess) return fail(B2D_ERR_CUDA, std::string("stage kernel launch: ") + cudaGetErrorString(e));
     return B2D_OK;
 }
@@ -1478,8 +1475,6 @@ static b2d_status finish_advance(b2d_ctx* ctx, int final_slot, double* dt_out, b
     long long count = 0;
     CUDA_TRY(cudaMemcpyAsync(&key, ctx->d_err_key, sizeof key, cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_TRY(cudaMemcpyAsync(&count, ctx->d_adv_count, sizeof count, cudaMemcpyDeviceToHost, ctx->stream));
-    unsigned tmo = 0;
-    CUDA_TRY(cudaMemcpyAsync(&tmo, ctx->d_timeout, sizeof tmo, cudaMemcpyDeviceToHost, ctx->stream));
     std::vector<double> dts(ctx->nruns);
     CUDA_TRY(cudaMemcpyAsync(dts.data(), ctx->d_dt, sizeof(double) * ctx->nruns, cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -1488,11 +1483,6 @@ static b2d_status finish_advance(b2d_ctx* ctx, int final_slot, double* dt_out, b
     const long long base = ctx->adv_base;
     ctx->adv_base = count;
     if (dt_out) memcpy(dt_out, dts.data(), sizeof(double) * ctx->nruns);
-    if (tmo) {
-        CUDA_TRY(cudaMemsetAsync(ctx->d_timeout, 0, sizeof(unsigned), ctx->stream));
-        CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        return fail(B2D_ERR_TIMEOUT, "a bounded wait on a staging barrier gave up; the step's results are invalid");
-    }
     if (key != ~0ull) {
         // the failing advance is the last one whose prologue ran
         long long k = count - 1 - base;
@@ -1683,29 +1673,38 @@ static b2d_status time_tile(b2d_ctx* ctx, int fold, int reps, double* ms)
     return B2D_OK;
 }
 
-// Strip rows for the chunk-taking kernel at the context's tile width: for the
-// fewest whole waves of resident CTAs that chunks of at most a block's rows
-// fill, and the next two, the shortest chunks that still fit in them.
+// CTAs of the FP32 stage kernel that the GPU holds at once.
+static long long resident_ctas(const b2d_ctx* ctx)
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return (long long)sms * (ctx->nf == 3 ? resident_f32_iso : resident_f32_euler)(store_of(ctx), even_columns(ctx), ctx->nruns);
+}
+
+// CTAs of a launch with row chunks of at most `rows` rows.
+static long long chunk_ctas(const b2d_ctx* ctx, int rows)
+{
+    long long n = 0;
+    for (const RunHost& r : ctx->runs)
+        n += (long long)((r.N + rows - 1) / rows) * ((r.N + STRIP_COLS - 1) / STRIP_COLS);
+    return n;
+}
+
+// Strip rows to try: for the fewest whole waves of resident CTAs that chunks of
+// at most a block's rows fill, and the next two, the shortest chunks that
+// still fit in them.
 static std::vector<int> strip_row_candidates(const b2d_ctx* ctx)
 {
     std::vector<int> out;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return out;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return out;
-    const int per_sm = stage_ctas_per_sm(ctx->nf, store_of(ctx), ctx->nruns, ctx->tw);
-    if (sms <= 0 || per_sm <= 0) return out;
-    const long long slots = (long long)sms * per_sm;
+    const long long slots = resident_ctas(ctx);
+    if (slots <= 0) return out;
     int min_bs = 1 << 30;
     for (const RunHost& r : ctx->runs) min_bs = std::min(min_bs, r.bs);
-    auto ctas = [&](int rows) {
-        long long n = 0;
-        for (const RunHost& r : ctx->runs) n += (long long)((r.N + rows - 1) / rows) * (r.N / ctx->tw);
-        return n;
-    };
-    long long waves = (ctas(min_bs) + slots - 1) / slots;
+    long long waves = (chunk_ctas(ctx, min_bs) + slots - 1) / slots;
     for (int c = 0; c < 3; ++c, ++waves) {
         int best = 0;
-        for (int rows = min_bs; rows >= 8 && ctas(rows) <= waves * slots; --rows) best = rows;
+        for (int rows = min_bs; rows >= 8 && chunk_ctas(ctx, rows) <= waves * slots; --rows) best = rows;
         if (best && std::find(out.begin(), out.end(), best) == out.end()) out.push_back(best);
     }
     return out;
@@ -1722,48 +1721,38 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
     b2d_status st = ensure_stage_capacity(ctx, fold);
     if (st != B2D_OK) return st;
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    const int max_w = ctx->precision == B2D_PREC_FP32_COMP ? 256 : 128;
     int best_w = ctx->tw, best_h = ctx->th, best_rows = 0;
     double best = 1e300;
-    ctx->strip_rows = 0;
+    auto trial = [&](int th, int rows) -> b2d_status {
+        ctx->th = th;
+        ctx->strip_rows = rows;
+        b2d_status s = sync_rundev(ctx);
+        double ms = 0;
+        if (s == B2D_OK) s = time_tile(ctx, fold, reps, &ms);
+        if (s == B2D_OK && ms < best * AUTOTUNE_MARGIN) { best = ms; best_h = th; best_rows = rows; }
+        return s;
+    };
     if (ctx->precision == B2D_PREC_FP64) {   // one tiling, whatever the tile shape
-        st = time_tile(ctx, fold, reps, &best);
+        st = trial(ctx->th, 0);
         if (st != B2D_OK) return st;
-    }
-    for (int w : {32, 64, 128, 256}) {
-        if (w > max_w || ctx->precision == B2D_PREC_FP64) continue;
-        for (int h : {8, 16, 32, 64, 128}) {
-            if (!tile_ok(ctx, w, h)) continue;
-            ctx->tw = w;
-            ctx->th = h;
-            st = sync_rundev(ctx);
+    } else {
+        // block-aligned chunks: every height that divides the blocks, but not
+        // so many chunks that they queue up behind one another
+        const long long slots = resident_ctas(ctx);
+        int max_bs = 0;
+        for (const RunHost& r : ctx->runs) max_bs = std::max(max_bs, r.bs);
+        for (int h = 1; h <= std::min(max_bs, 128); ++h) {
+            if (!tile_ok(ctx, ctx->tw, h)) continue;
+            if (h < 16 && 2 * h <= max_bs && chunk_ctas(ctx, h) > 2 * slots) continue;
+            st = trial(h, 0);
             if (st != B2D_OK) return st;
-            double ms = 0;
-            st = time_tile(ctx, fold, reps, &ms);
-            if (st != B2D_OK) return st;
-            if (ms < best * AUTOTUNE_MARGIN) { best = ms; best_w = w; best_h = h; }
         }
-    }
-    // row chunks of the FP32 kernels, at each tile width that takes them (the
-    // widest first: the fewest halo warps)
-    for (int w : {512, 256, 128, 64, 32}) {
-        int h = 0;
-        for (int hh : {64, 32, 16, 8})
-            if (!h && tile_ok(ctx, w, hh)) h = hh;
-        if (!h) continue;
-        ctx->tw = w;
-        ctx->th = h;
-        if (!chunk_kernel(ctx)) continue;
+        // chunks that cross block rows and fill whole waves
+        const int h = best_h;
         for (int rows : strip_row_candidates(ctx)) {
-            ctx->strip_rows = rows;
-            st = sync_rundev(ctx);
+            st = trial(h, rows);
             if (st != B2D_OK) return st;
-            double ms = 0;
-            st = time_tile(ctx, fold, reps, &ms);
-            if (st != B2D_OK) return st;
-            if (ms < best * AUTOTUNE_MARGIN) { best = ms; best_w = w; best_h = h; best_rows = rows; }
         }
-        ctx->strip_rows = 0;
     }
     // discard what the trial advances left behind
     long long count = 0;
@@ -1771,7 +1760,6 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
     ctx->adv_base = count;
     ctx->window.clear();
     CUDA_TRY(cudaMemset(ctx->d_err_key, 0xff, sizeof(unsigned long long)));
-    CUDA_TRY(cudaMemset(ctx->d_timeout, 0, sizeof(unsigned)));
     ctx->tw = best_w;
     ctx->th = best_h;
     ctx->strip_rows = best_rows;
@@ -1998,7 +1986,6 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     long long* iters = (long long*)(orbit + 16);           // 4 (unused by the stage)
     unsigned long long* amax = (unsigned long long*)(orbit + 20);
     unsigned long long* err_key = amax + 1;
-    unsigned* timeout = (unsigned*)(err_key + 1);
     unsigned* counter = (unsigned*)(base + off_cnt);
     double* partial = (double*)(base + off_part);
 
@@ -2037,7 +2024,6 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned) * nblocks, stream));
     CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(unsigned long long), stream));
     CUDA_TRY(cudaMemsetAsync(err_key, 0xff, sizeof(unsigned long long), stream));
-    CUDA_TRY(cudaMemsetAsync(timeout, 0, sizeof(unsigned), stream));
     noalloc_setup_kernel<<<1, 32, 0, stream>>>(d_run, time, dt);
     CUDA_TRY(cudaGetLastError());
 
@@ -2051,10 +2037,10 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     a.stage = 0;
     a.amax_flag = d_max_speed ? 1 : 0;
     a.bf = d_base ? bf : 0.0;
+    a.half_avg = a.bf == 0.5;
     a.w1f = split_df(-a.bf + 1.0);
     a.bff = split_df(a.bf);
     a.err_key = err_key;
-    a.timeout_flag = timeout;
     cudaError_t e = launch_stage_f64(nf, a, rd.ntiles, stage_f64_smem(nf, sub_h, sub_w), stream);
     if (e != cudaSuccess) return fail(B2D_ERR_CUDA, std::string("stage kernel launch: ") + cudaGetErrorString(e));
     if (d_max_speed) CUDA_TRY(cudaMemcpyAsync(d_max_speed, amax, sizeof(double), cudaMemcpyDeviceToDevice, stream));

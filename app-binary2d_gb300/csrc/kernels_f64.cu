@@ -22,7 +22,7 @@ __global__ void buffer_rate_kernel(const RunDev* runs, int run, double* out)
     const size_t nn = (size_t)rd.N * rd.N;
     for (size_t z = blockIdx.x * (size_t)blockDim.x + threadIdx.x; z < nn; z += (size_t)gridDim.x * blockDim.x) {
         const unsigned i = (unsigned)z / (unsigned)rd.N, j = (unsigned)z - i * (unsigned)rd.N;
-        out[z] = buffer_rate<double>(rd.p, rd.xc[i], rd.xc[j]);
+        out[z] = buffer_rate(rd.p, rd.xc[i], rd.xc[j]);
     }
 }
 

@@ -26,8 +26,7 @@ struct RunDev {
     const double* buffer;    // FP64 kernel: [N][N] buffer rate (nullptr: computed where it is used)
     const double* xc;        // [N] cell centres by global index (block formula, mesh.rs:49-54)
     const double* xv;        // [nb][bs+1] block vertices (mesh.rs:42-47)
-    const float* xcf;
-    const float* xvf;
+    const float* xcf;        // FP32 centres; like xvgf, 4 entries longer than the mesh at either end
     const float* xvgf;       // [N+1] row faces by global index, FP32 (a block's first vertex at its lower boundary)
     void* slot[NSLOTS];      // conserved state per slot (STORE layout)
     const void* bg;          // BlockData::initial_conserved (STORE layout)
@@ -59,10 +58,10 @@ struct StageArgs {
     int stage;
     int amax_flag;
     double bf;               // weight of the RK base state (br of godunov-core)
+    int half_avg;            // bf is 1/2
     b2d::df32w w1f, bff;     // 1 - bf and bf as double-float
     DevParamsF pf1;          // FP32 parameters of a single-run context, read as kernel arguments
     unsigned long long* err_key;  // failure key, ~0 when no zone failed
-    unsigned* timeout_flag;       // set when a bounded wait gave up
 };
 
 // Row chunks of a column strip.  A run's N rows split into C chunks; chunk c

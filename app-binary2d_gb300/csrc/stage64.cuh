@@ -131,7 +131,7 @@ __device__ __noinline__ double minmod_nan(double x, double y, double z)
     return fmax(fmin(fmin(x, y), z), 0.0) + fmin(fmax(fmax(x, y), z), 0.0);
 }
 
-// The limiter of plm_gradient (physics.cuh) on x, y / 2 and z: the one of
+// The limiter of plm_gradient (godunov-core, restated) on x, y / 2 and z: the one of
 // smallest magnitude if all share a sign, else 0.  Halving takes one off the
 // exponent; NaN, infinite and subnormal arguments take the general form.
 __device__ __forceinline__ double minmod_bits(double x, double y, double z)
@@ -147,7 +147,7 @@ __device__ __forceinline__ double minmod_bits(double x, double y, double z)
     return (long long)((a ^ b) | (a ^ c)) < 0 ? 0.0 : from_bits(m | (a & D_SIGN));
 }
 
-// Sum K values (a power of two, K <= 32) over a warp: see warp_sum_items (stage2.cuh).
+// Sum K values (a power of two, K <= 32) over the warp by recursive halving.
 template <int K> __device__ __forceinline__ double warp_sum_doubles(double (&v)[K], int lane)
 {
 #pragma unroll
@@ -278,7 +278,7 @@ template <int NF> __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kern
         // Phase 1: primitives of the sub-tile and its 2-zone halo; the geometry tables.
         for (int e = t; e < PS; e += NT) {
             const int r = e / PW - 2, c = e % PW - 2;
-            const int gi = wrap(i0 + r, N), gj = wrap(j0 + c, N);
+            const int gi = wrap(wrap(i0 + r, N), N), gj = wrap(wrap(j0 + c, N), N);   // (twice: a mesh may be one zone wide)
             const size_t idx = (size_t)gi * N + gj;
             double u[NF], p[NF];
 #pragma unroll
@@ -555,7 +555,7 @@ template <int NF> __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kern
             const double* q = gr + 7 * r;
             const double* w = gc + 7 * c;
             const double s1 = q[0] + w[0], s2 = q[1] + w[1];
-            const double br = rd.buffer ? __ldg(rd.buffer + idx) : buffer_rate<double>(P, q[2], w[2]);
+            const double br = rd.buffer ? __ldg(rd.buffer + idx) : buffer_rate(P, q[2], w[2]);
             const double* fx = sFX + r * TW + c;
             const double* fy = sFY + r * FW + c;
 
@@ -637,8 +637,8 @@ template <int NF> __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kern
                     const PointMass<double> b1{orb[0], orb[1], orb[2], orb[3], orb[4]};
                     const PointMass<double> b2{orb[5], orb[6], orb[7], orb[8], orb[9]};
                     double x1, y1, x2, y2;
-                    torque_free_velocity<double>(P, b1, q[2], w[2], vx, vy, x1, y1);
-                    torque_free_velocity<double>(P, b2, q[2], w[2], vx, vy, x2, y2);
+                    torque_free_velocity(P, b1, q[2], w[2], vx, vy, x1, y1);
+                    torque_free_velocity(P, b2, q[2], w[2], vx, vy, x2, y2);
                     a1[0] = a2[0] = u[0];
                     a1[1] = u[0] * x1; a1[2] = u[0] * y1;
                     a2[1] = u[0] * x2; a2[2] = u[0] * y2;

@@ -1,0 +1,1017 @@
+// stagew.cuh — the FP32 RK-stage kernel: every warp marches down a strip of
+// its own.
+//
+// One launch performs one call of try_advance_rk (src/scheme.rs:88-173) for
+// every run of a context, on the FP64 state or on the compensated FP32 state:
+// cons→prim (scheme.rs:185-199), PLM slopes and HLLE + viscous fluxes
+// (scheme.rs:216-268), flux divergence + sources + RK average
+// (scheme.rs:290-305, state.rs:183-199), the per-block source ledger
+// (scheme.rs:288-313) and, on the last stage of an advance, the max signal
+// speed of the next dt (state.rs:121-133).
+//
+//  * A warp is on its own: it is a CTA, so that its loop and addresses are
+//    uniform.  It owns 60 columns of a row chunk, two adjacent columns a lane
+//    (lanes 0 and 31 are the two guard pairs on either side), and goes down its
+//    rows without a barrier: neighbouring columns come by shuffle, the rows
+//    above from registers, and the guard columns are computed again by the
+//    next strip's warp (2 of 32 lanes).  The twelve warps of an SM drift apart
+//    and fill each other's stalls.
+//  * Packed arithmetic.  Every per-column quantity is a float2 and the
+//    arithmetic runs as Blackwell's packed FADD2 / FMUL2 / FFMA2; min / max,
+//    compares, selects and the special-function unit stay per column.
+//  * Row staging.  Every lane copies its own two columns of the rows ahead into
+//    a ring in shared memory by asynchronous copies (8 bytes, or 16 of an FP64
+//    state; a mesh of odd side takes single words), one group per row: the
+//    stage input a row ahead of its use, and what the update reads besides (low
+//    words, background, RK base).  Lanes read back only what they copied
+//    themselves, so nothing waits but the lane.  The periodic edge is a matter
+//    of a lane's column.  (Bulk copies (TMA) cost more here: a warp's row is 15
+//    planes of 240 bytes, each an instruction of its own with uniform
+//    addresses, 180 of 970 instructions a row.)
+//  * Constants that packed instructions take are kept twice, as a pair, in
+//    shared memory: one load instead of two moves per use.
+//  * Pipeline.  Iteration n converts row n, forms slopes and stresses of row
+//    g = n - 1, its upper x faces and its y faces, and updates row g - 1.
+//  * Ledger.  The items that are live everywhere are summed per column in
+//    registers; a block's part is reduced over the warp at the last row of
+//    each block row and at the chunk's end, one piece per strip and chunk,
+//    and the last piece of a block folds them in order.
+//
+// What bounds it: instruction issue (681 warp instructions per row of 60
+// columns and isothermal first stage, about 390 of them arithmetic; issue 52 %
+// busy at 12 warps per SM), not memory (about 2.7 of 6.7 TB/s).  Measured per
+// stage against the kernels it took the place of: isothermal 2048^2 0.127 ->
+// 0.109 ms (a CTA of 10 warps marching in step over 512 columns), 384^2 33 -> 22
+// us, the 64-run sweep 1.05 -> 0.69 ms, Euler 4096^2 0.65 -> 0.55 ms, 768^2 48
+// -> 42 us, blocks of 50^2 (RK3, alpha viscosity) 163 -> 25 us (one thread per
+// column of a block), FP64 state 1024^2 106 -> 94 us.
+#pragma once
+
+#include "stage.cuh"
+
+namespace b2d {
+
+constexpr int SW_COLS = 60;              // columns of a strip
+constexpr int SW_CTAS = 12;              // one-warp CTAs per SM: 168 registers a thread
+constexpr int SW_SLOTS = 4;              // stencil ring: rows n - 2 (for its update) to n + 1
+constexpr int SW_USLOTS = 2;             // update rows: one in use, one ahead
+
+// Shared memory of one warp.
+template <int NF, int STORE> struct SWShape {
+    using E = typename std::conditional<STORE == 1, float, double>::type;
+    static constexpr int NU = (STORE == 1 ? 4 : 2) * NF;  // update planes: (lo,) bg, base hi (, base lo)
+    static constexpr int ITEMS = NF == 3 ? 16 : 19;       // ledger rows: everywhere, sinks, fake mass
+    static constexpr int SINKS_AT = NF == 3 ? 7 : 11, FAKE_AT = 13;
+    static constexpr int STENCIL = NF * 64;               // elements of a staged row
+    static constexpr int UPDATE = NU * 64;
+    static constexpr int BYTES = (SW_SLOTS * STENCIL + SW_USLOTS * UPDATE) * (int)sizeof(E) + ITEMS * 64 * 4;
+};
+
+// Constants as pairs.
+enum {
+    C_THETA, C_HALF, C_NHALF, C_INV_DX, C_LAMBDA, C_NU, C_INV_MACH2, C_M1, C_M2, C_NM1DT, C_NM2DT, C_Y1, C_Y2, C_SOFT2,
+    C_RADIUS, C_BUF_SLOPE, C_BUF_RATE, C_NDT_DX, C_43, C_N23, C_GAMMA, C_GM1, C_INV_GM1, C_COOL, C_ALPHA, C_ONE, C_COUNT
+};
+
+// ---------------------------------------------------------------------------
+// Packed FP32x2 arithmetic (sm_100+ FADD2 / FMUL2 / FFMA2, round to nearest).
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+// a - b as b * (-1) + a: one rounding, the same value as a subtraction
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)); }
+__device__ __forceinline__ float2 sqrt2(float2 a) { return make_float2(sqrtf(a.x), sqrtf(a.y)); }
+__device__ __forceinline__ float2 rsqrt2(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
+
+// Knuth TwoSum / Dekker Fast2Sum on pairs (the compensated state update).
+struct df2 { float2 hi, lo; };
+
+__device__ __forceinline__ df2 fast_two_sum2(float2 a, float2 b)
+{
+    const float2 s = add2(a, b);
+    return {s, sub2(b, sub2(s, a))};
+}
+
+__device__ __forceinline__ df2 two_sum2(float2 a, float2 b)
+{
+    const float2 s = add2(a, b);
+    const float2 bb = sub2(s, a);
+    return {s, add2(sub2(a, sub2(s, bb)), sub2(b, bb))};
+}
+
+__device__ __forceinline__ df2 df_add_f2(df2 a, float2 b)
+{
+    const df2 s = two_sum2(a.hi, b);
+    return fast_two_sum2(s.hi, add2(s.lo, a.lo));
+}
+
+__device__ __forceinline__ df2 df_add2(df2 a, df2 b)
+{
+    const df2 s = two_sum2(a.hi, b.hi);
+    return fast_two_sum2(s.hi, add2(s.lo, add2(a.lo, b.lo)));
+}
+
+__device__ __forceinline__ df2 df_mul2(df2 a, df32 b)
+{
+    const float2 bh = f2(b.hi), bl = f2(b.lo);
+    const float2 p = mul2(a.hi, bh);
+    float2 e = fma2(a.hi, bh, mul2(p, f2(-1.0f)));
+    e = fma2(a.hi, bl, fma2(a.lo, bh, e));
+    return fast_two_sum2(p, e);
+}
+
+// Three-input FP32 minimum and maximum (PTX min/max with three sources, sm_100+).
+__device__ __forceinline__ float min3f(float a, float b, float c)
+{
+    float d;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float max3f(float a, float b, float c)
+{
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// Generalised minmod of each lane (godunov-core's plm_gradient, restated) as the median of
+// min(x, y, z), max(x, y, z) and 0: the minimum when all three are positive,
+// the maximum when all are negative, else 0 — min(max(lo, 0), hi) for lo <= hi.
+__device__ __forceinline__ float2 plm_gradient2(float2 th, float2 a, float2 b, float2 c)
+{
+    const float2 x = mul2(th, sub2(b, a));
+    const float2 y = mul2(f2(0.5f), sub2(c, a));
+    const float2 z = mul2(th, sub2(c, b));
+    return make_float2(fminf(fmaxf(min3f(x.x, y.x, z.x), 0.0f), max3f(x.x, y.x, z.x)),
+                       fminf(fmaxf(min3f(x.y, y.y, z.y), 0.0f), max3f(x.y, y.y, z.y)));
+}
+
+// e^x - 1 of two small arguments (|x| <= 0.35): the Taylor series
+// x (1 + x/2 + x^2/6 + ... + x^7/8!) in Horner form; the first omitted term,
+// x^9/9!, is below 6e-10 |x| there.
+__device__ __forceinline__ float2 expm1_small2(float2 x)
+{
+    float2 p = f2(1.0f / 40320.0f);
+    p = fma2(p, x, f2(1.0f / 5040.0f));
+    p = fma2(p, x, f2(1.0f / 720.0f));
+    p = fma2(p, x, f2(1.0f / 120.0f));
+    p = fma2(p, x, f2(1.0f / 24.0f));
+    p = fma2(p, x, f2(1.0f / 6.0f));
+    p = fma2(p, x, f2(0.5f));
+    p = fma2(p, x, f2(1.0f));
+    return mul2(p, x);
+}
+
+// ---------------------------------------------------------------------------
+// Scalar FP32 pieces, written with explicit roundings (fmaf, __fmul_rn,
+// __fadd_rn: no contraction left to the compiler), so that every instantiation
+// of the kernel rounds them alike and the states depend neither on the tiling
+// nor on the batch.
+
+// cons -> prim without floors (hydro-iso2d / hydro-euler; physics.rs:696).
+template <int NF> __device__ __forceinline__ void prim_exact(const DevParamsF& P, const float* u, float* p)
+{
+    const float ir = __fdividef(1.0f, u[0]);
+    p[0] = u[0];
+    p[1] = __fmul_rn(u[1], ir);
+    p[2] = __fmul_rn(u[2], ir);
+    if constexpr (NF == 4) {
+        const float v2 = fmaf(p[1], p[1], __fmul_rn(p[2], p[2]));
+        p[3] = __fmul_rn(fmaf(__fmul_rn(-0.5f, u[0]), v2, u[3]), P.gm1);
+    }
+}
+
+// Hydrodynamics::max_signal_speed (physics.rs:521-526, 679-681).
+template <int NF> __device__ __forceinline__ float max_speed_exact(const DevParamsF& P, const float* u)
+{
+    float p[NF];
+    prim_exact<NF>(P, u, p);
+    const float v = fmaxf(fabsf(p[1]), fabsf(p[2]));
+    if constexpr (NF == 4) return __fadd_rn(v, sqrtf(__fmul_rn(__fmul_rn(P.gamma, p[3]), __fdividef(1.0f, p[0]))));
+    return v;
+}
+
+// Physics::sink_kernel (physics.rs:388-397): rate (1 - r^2 / s^2)^2 inside the sink radius s.
+__device__ __forceinline__ float sink_rate_exact(const DevParamsF& P, float dx, float dy)
+{
+    const float r2 = fmaf(dx, dx, __fmul_rn(dy, dy));
+    if (r2 < P.sink_r2) {
+        const float t = fmaf(-r2, P.inv_sink_r2, 1.0f);
+        return __fmul_rn(P.sink_rate, __fmul_rn(t, t));
+    }
+    return 0.0f;
+}
+
+// The torque-free sink velocity: the gas velocity relative to the body,
+// projected on the radial direction, plus the body's velocity (physics.rs:743-756).
+__device__ __forceinline__ void torque_free_exact(const DevParamsF& P, const PointMass<float>& b, float x, float y,
+                                                  float vx, float vy, float& vxc, float& vyc)
+{
+    const float vxb = P.one_body ? 0.0f : b.vx, vyb = P.one_body ? 0.0f : b.vy;
+    const float ddx = x - b.x, ddy = y - b.y;
+    const float r = sqrtf(fmaf(ddx, ddx, __fmul_rn(ddy, ddy)));
+    const float rx = __fdividef(ddx, r), ry = __fdividef(ddy, r);
+    const float dvdotr = fmaf(vx - vxb, rx, __fmul_rn(vy - vyb, ry));
+    vxc = fmaf(dvdotr, rx, vxb);
+    vyc = fmaf(dvdotr, ry, vyb);
+}
+
+// The sink items of one zone (the sink part of source_terms, physics.rs:
+// 528-582, 683-774): -rate u dt (impartial sinks) or -rate dt times the
+// torque-free state.
+template <int NF>
+__device__ __noinline__ void sink_items_exact(const DevParamsF& P, const Binary<float>& B, const float* u, float x,
+                                              float y, float dt, float* s1, float* s2)
+{
+    const float sr1 = __fmul_rn(sink_rate_exact(P, x - B.p1.x, y - B.p1.y), -dt);
+    const float sr2 = __fmul_rn(sink_rate_exact(P, x - B.p2.x, y - B.p2.y), -dt);
+    if (P.sink_model == 0) {
+#pragma unroll
+        for (int k = 0; k < NF; ++k) {
+            s1[k] = __fmul_rn(u[k], sr1);
+            s2[k] = __fmul_rn(u[k], sr2);
+        }
+        return;
+    }
+    float p[NF];
+    prim_exact<NF>(P, u, p);
+    float v1x, v1y, v2x, v2y;
+    torque_free_exact(P, B.p1, x, y, p[1], p[2], v1x, v1y);
+    torque_free_exact(P, B.p2, x, y, p[1], p[2], v2x, v2y);
+    const float sd = p[0];
+    float a1[NF], a2[NF];
+    a1[0] = a2[0] = sd;
+    a1[1] = __fmul_rn(sd, v1x); a1[2] = __fmul_rn(sd, v1y);
+    a2[1] = __fmul_rn(sd, v2x); a2[2] = __fmul_rn(sd, v2y);
+    if constexpr (NF == 4) {
+        const float e0 = __fmul_rn(__fdividef(p[3], p[0]), P.inv_gm1), hs = __fmul_rn(0.5f, sd);
+        a1[3] = fmaf(sd, e0, __fmul_rn(hs, fmaf(v1x, v1x, __fmul_rn(v1y, v1y))));
+        a2[3] = fmaf(sd, e0, __fmul_rn(hs, fmaf(v2x, v2x, __fmul_rn(v2y, v2y))));
+    }
+#pragma unroll
+    for (int k = 0; k < NF; ++k) {
+        s1[k] = __fmul_rn(a1[k], sr1);
+        s2[k] = __fmul_rn(a2[k], sr2);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Faces.
+//
+// Viscous stress, factored.  The face stress of stress_field (physics.rs:
+// 322-349) with the `nu` closure of scheme.rs:230-247 is
+//   tau_nn = (rho_l nu_l (s_nn,l + lambda bulk_l) + rho_r nu_r (s_nn,r + lambda bulk_r)) / 2
+// (and tau_t alike with s_xy and no bulk term).  nu_l = nu_r = nu for a
+// constant viscosity; for the alpha model nu_side = K(face) * cs2 with
+// K = alpha / Omega_2(face) / sqrt(gamma - 1), cs2 taken at the face from the
+// potential (isothermal, so nu_l = nu_r again) or from the cell's own
+// pressure (Euler).  Each cell therefore carries T_nn = c rho (s_nn + lambda
+// bulk) and T_xy = c rho s_xy with c = nu (constant), 1 (isothermal alpha) or
+// gamma p / rho (Euler alpha), and a face needs tau = K (T_l + T_r) / 2 with
+// K = 1 for the constant model.
+
+// 0.5 K of the alpha model at two faces (x, fy.x) and (x, fy.y), an isothermal
+// face's cs2 left out.  1 / a^3 is taken as rsqrt(a^2)^3: the reference's
+// a = |d| + 1e-12 dx (scheme.rs:244) differs from |d| below FP32 resolution
+// unless |d| is under about 1e-7 dx, and at |d| = 0 both give K = 0.
+__device__ __forceinline__ float2 alpha_half_k2(const float2* K, const Binary<float>& B, float x, float2 fy)
+{
+    const float dx1 = x - B.p1.x, dx2 = x - B.p2.x;
+    const float2 dy1 = sub2(fy, K[C_Y1]), dy2 = sub2(fy, K[C_Y2]);
+    const float2 d1 = fma2(dy1, dy1, f2(__fmul_rn(dx1, dx1))), d2 = fma2(dy2, dy2, f2(__fmul_rn(dx2, dx2)));
+    const float2 q1 = rsqrt2(d1), q2 = rsqrt2(d2);
+    const float2 w2 = fma2(K[C_M1], mul2(q1, mul2(q1, q1)), mul2(K[C_M2], mul2(q2, mul2(q2, q2))));
+    return mul2(K[C_ALPHA], rsqrt2(w2));
+}
+
+// Two faces normal to AXIS (intercell_flux, physics.rs:584-607, 776-803, with
+// hydro-iso2d's and hydro-euler's HLLE) from the states reconstructed on
+// either side.  cs2: the isothermal face sound speed; k: half the alpha
+// model's factor (1/2 for a constant viscosity); tn, tt: the sums of the two
+// cells' factored stresses; vxs, vys: the sums of their velocities (Euler).
+template <int NF, int AXIS>
+__device__ __forceinline__ void faces2(const float2* K, const float2* pl, const float2* pr, float2 cs2, float2 k,
+                                       float2 tn, float2 tt, float2 vxs, float2 vys, float2* F)
+{
+    const float2 vl = pl[1 + AXIS], vr = pr[1 + AXIS];
+    // conserved states and physical fluxes
+    float2 ul[NF], ur[NF], fl[NF], fr[NF], pgl, pgr, csl, csr;
+    ul[0] = pl[0];
+    ur[0] = pr[0];
+    ul[1] = mul2(pl[0], pl[1]); ul[2] = mul2(pl[0], pl[2]);
+    ur[1] = mul2(pr[0], pr[1]); ur[2] = mul2(pr[0], pr[2]);
+    if constexpr (NF == 3) {
+        pgl = mul2(pl[0], cs2);
+        pgr = mul2(pr[0], cs2);
+        csl = csr = sqrt2(cs2);
+    } else {
+        pgl = pl[3];
+        pgr = pr[3];
+        csl = sqrt2(mul2(mul2(K[C_GAMMA], pl[3]), rcp2(pl[0])));
+        csr = sqrt2(mul2(mul2(K[C_GAMMA], pr[3]), rcp2(pr[0])));
+        ul[3] = fma2(mul2(K[C_HALF], pl[0]), fma2(pl[1], pl[1], mul2(pl[2], pl[2])), mul2(pl[3], K[C_INV_GM1]));
+        ur[3] = fma2(mul2(K[C_HALF], pr[0]), fma2(pr[1], pr[1], mul2(pr[2], pr[2])), mul2(pr[3], K[C_INV_GM1]));
+        fl[3] = mul2(add2(ul[3], pl[3]), vl);
+        fr[3] = mul2(add2(ur[3], pr[3]), vr);
+    }
+    fl[0] = mul2(pl[0], vl);
+    fr[0] = mul2(pr[0], vr);
+    fl[1] = AXIS == 0 ? fma2(ul[1], vl, pgl) : mul2(ul[1], vl);
+    fr[1] = AXIS == 0 ? fma2(ur[1], vr, pgr) : mul2(ur[1], vr);
+    fl[2] = AXIS == 1 ? fma2(ul[2], vl, pgl) : mul2(ul[2], vl);
+    fr[2] = AXIS == 1 ? fma2(ur[2], vr, pgr) : mul2(ur[2], vr);
+    // outer wave speeds
+    const float2 alm = sub2(vl, csl), alp = add2(vl, csl), arm = sub2(vr, csr), arp = add2(vr, csr);
+    const float2 ap = make_float2(max3f(alp.x, arp.x, 0.0f), max3f(alp.y, arp.y, 0.0f));
+    const float2 am = make_float2(min3f(alm.x, arm.x, 0.0f), min3f(alm.y, arm.y, 0.0f));
+    const float2 inv = rcp2(sub2(ap, am));
+    const float2 nam = mul2(am, f2(-1.0f));
+    const float2 apam = mul2(ap, am);
+    // F = (fl ap - fr am - (ul - ur) ap am) / (ap - am)
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+        F[f] = mul2(fma2(sub2(ur[f], ul[f]), apam, fma2(fr[f], nam, mul2(fl[f], ap))), inv);
+    const float2 tau_n = mul2(k, tn), tau_t = mul2(k, tt);
+    const float2 tx = AXIS == 0 ? tau_n : tau_t, ty = AXIS == 0 ? tau_t : tau_n;
+    F[1] = sub2(F[1], tx);
+    F[2] = sub2(F[2], ty);
+    if constexpr (NF == 4) F[3] = sub2(F[3], mul2(K[C_HALF], fma2(tx, vxs, mul2(ty, vys))));
+}
+
+// Sum K values (a power of two, K <= 32) over the 32 lanes of a warp by
+// recursive halving: after the call lane l holds the warp total of value
+// item_of_lane(l, K); 2K - 1 shuffles in all.
+template <int K> __device__ __forceinline__ float warp_sum_items(float (&v)[K], int lane)
+{
+#pragma unroll
+    for (int half = K / 2, off = 16; half >= 1; half >>= 1, off >>= 1) {
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const float send = upper ? v[i] : v[i + half];
+            const float keep = upper ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+    }
+    float s = v[0];
+    for (int off = 16 / K; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    return s;
+}
+
+// Which value of warp_sum_items lane l ends up holding.
+template <int K> __device__ __forceinline__ int item_of_lane(int lane)
+{
+    int item = 0;
+    for (int half = K / 2, off = 16; half >= 1; half >>= 1, off >>= 1)
+        if (lane & off) item += half;
+    return item;
+}
+
+// The ledger word (item * NF + field) of a strip's ledger row m.
+template <int NF> __device__ __forceinline__ int ledger_word(int m)
+{
+    if constexpr (NF == 3) {
+        if (m < 4) return (GRAV1 + m / 2) * 3 + 1 + m % 2;
+        if (m < 7) return BUFFER * 3 + m - 4;
+        if (m < 13) return SINK1 * 3 + m - 7;
+        return FAKE_MASS * 3 + m - 13;
+    } else {
+        if (m < 6) return (GRAV1 + m / 3) * 4 + 1 + m % 3;
+        if (m < 10) return BUFFER * 4 + m - 6;
+        if (m == 10) return COOLING * 4 + 3;
+        return SINK1 * 4 + m - 11;
+    }
+}
+
+// A strip's ledger pieces of block row `brow`, by its warp: for every block
+// under the strip the sums over the columns inside it, the piece's slot in
+// the block's partials, and the fold of the block's pieces (in piece order)
+// by the block's last piece.  Out of line, so that it does not weigh on the
+// row loop's register allocation.
+template <int NF, int STORE>
+__device__ __noinline__ void flush_strip(const RunDev& rd, int strip, int ti, int brow, const float* led, bool sinks,
+                                         bool fake, int in_slot, int base_slot, int out_slot, int stage, double bf)
+{
+    using T = SWShape<NF, STORE>;
+    constexpr int NL = NITEMS * NF, K = NF == 3 ? 16 : 32;
+    const int lane = threadIdx.x & 31;
+    const int N = rd.N, bs = rd.bs;
+    const int j0 = strip * SW_COLS, w = min(SW_COLS, N - j0), c0 = 2 * lane - 2;
+    const int nc = chunks_in_block_row(brow, bs, N, rd.chunks), first_chunk = chunk_of_row(brow * bs, N, rd.chunks);
+    for (int b = j0 / bs; b <= (j0 + w - 1) / bs; ++b) {
+        const int lo = max(b * bs - j0, 0), hi = min(b * bs + bs - j0, w);
+        const bool inx = c0 >= lo && c0 < hi, iny = c0 + 1 >= lo && c0 + 1 < hi;
+        float v[K];
+#pragma unroll
+        for (int m = 0; m < K; ++m) {
+            const bool on = m < T::SINKS_AT || (m < (NF == 3 ? T::FAKE_AT : T::ITEMS) ? sinks : m < T::ITEMS && fake);
+            v[m] = 0.0f;
+            if (on) {
+                const float2 q = *(const float2*)(led + m * 64 + 2 * lane);
+                v[m] = (inx ? q.x : 0.0f) + (iny ? q.y : 0.0f);
+            }
+        }
+        const float s = warp_sum_items<K>(v, lane);
+        const int m = item_of_lane<K>(lane);
+        const int block = brow * rd.nb + b;
+        const int first_strip = b * bs / SW_COLS, ns = (b * bs + bs - 1) / SW_COLS - first_strip + 1;
+        const int piece = (strip - first_strip) * nc + ti - first_chunk, pieces = ns * nc;
+        double* part = rd.partial + (size_t)block * rd.tiles_per_block * NL;
+        if ((lane & (32 / K - 1)) == 0 && m < T::ITEMS) {
+            part[(size_t)piece * NL + ledger_word<NF>(m)] = (double)s;
+            __threadfence();   // visible before the counter below counts this piece
+        }
+        __syncwarp();
+        unsigned last = 0;
+        if (lane == 0) last = atomicAdd(rd.counter + block, 1u) == (unsigned)pieces - 1;
+        last = __shfl_sync(0xffffffffu, last, 0);
+        if (!last) continue;
+        __threadfence();
+        if (lane < NL) {
+            const double area = (double)rd.p.dx * rd.p.dx;
+            double sum = 0.0;
+#pragma unroll 16
+            for (int q = 0; q < pieces; ++q) sum += __ldcg(part + (size_t)q * NL + lane);
+            double v2 = __ldcg(rd.ledger[in_slot] + (size_t)block * NL + lane) + sum * area;
+            if (base_slot >= 0)
+                v2 = v2 * (-bf + 1.0) + __ldcg(rd.ledger[base_slot] + (size_t)block * NL + lane) * bf;
+            rd.ledger[out_slot][(size_t)block * NL + lane] = v2;
+            // the block's ds·dx·dy of this stage, for the orbital-element ledger
+            if (rd.stage_ds) rd.stage_ds[((size_t)stage * rd.nblocks + block) * NL + lane] = sum * area;
+        }
+        if (lane == 0) rd.counter[block] = 0u;
+    }
+}
+
+template <bool SINGLE>
+__device__ __forceinline__ const DevParamsF& params_for(const StageArgs& a, const DevParamsF& shared_copy)
+{
+    // a single-run launch reads its parameters from the kernel arguments
+    // (constant-bank operands), a batched one from shared memory
+    if constexpr (SINGLE) return a.pf1;
+    else return shared_copy;
+}
+
+// Asynchronous copy of BYTES bytes (4, 8 or 16, aligned to it) from global to shared memory.
+template <int BYTES> __device__ __forceinline__ void copy_async(void* dst, const void* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING> __device__ __forceinline__ void copy_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
+}
+
+// A staged pair at the stencil's precision, and whole.
+__device__ __forceinline__ float2 pair_of(const float* p) { return *(const float2*)p; }
+__device__ __forceinline__ float2 pair_of(const double* p)
+{
+    const double2 v = *(const double2*)p;
+    return make_float2((float)v.x, (float)v.y);
+}
+
+// ---------------------------------------------------------------------------
+// EVEN: the mesh has an even number of columns, so that a pair is one aligned word.
+template <int NF, int STORE, bool SINGLE, bool EVEN>
+__global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_constant__ StageArgs a)
+{
+    using T = SWShape<NF, STORE>;
+    using E = typename T::E;
+    const int lane = threadIdx.x;
+
+    int ri = 0;
+    const int g = blockIdx.x;
+    if constexpr (!SINGLE)
+        while (ri + 1 < a.nruns && g >= a.runs[ri + 1].tile_base) ++ri;
+    const RunDev& rd = a.runs[ri];
+    if (*(volatile unsigned long long*)a.err_key != ~0ull) return;   // an earlier stage failed: the advance is abandoned
+
+    __shared__ DevParamsF Psh;
+    const DevParamsF& P = params_for<SINGLE>(a, Psh);
+    __shared__ Binary<float> B;
+    __shared__ float2 K[C_COUNT];
+    if (lane < 10) ((float*)&B)[lane] = (float)rd.orbit[a.stage * 10 + lane];
+    if (!SINGLE && lane == 10) Psh = rd.pf;
+    extern __shared__ __align__(128) unsigned char smem_raw[];   // one declaration for every stage kernel
+    poison_dynamic_smem(smem_raw);
+    __syncwarp();
+    const float dt = (float)*rd.dt;
+    const float time = (float)rd.stage_time[a.stage];
+    if (lane == 0) {
+        K[C_THETA] = f2(P.plm);
+        K[C_HALF] = f2(0.5f);
+        K[C_NHALF] = f2(-0.5f);
+        K[C_INV_DX] = f2(P.inv_dx);
+        K[C_LAMBDA] = f2(P.lambda);
+        K[C_NU] = f2(P.nu);
+        K[C_INV_MACH2] = f2(P.inv_mach2);
+        K[C_M1] = f2(B.p1.m);
+        K[C_M2] = f2(B.p2.m);
+        K[C_NM1DT] = f2(__fmul_rn(-B.p1.m, dt));
+        K[C_NM2DT] = f2(__fmul_rn(-B.p2.m, dt));
+        K[C_Y1] = f2(B.p1.y);
+        K[C_Y2] = f2(B.p2.y);
+        K[C_SOFT2] = f2(P.soft2);
+        K[C_RADIUS] = f2(P.domain_radius);
+        K[C_BUF_SLOPE] = f2(-2.0f * P.inv_buffer_scale);
+        K[C_BUF_RATE] = f2(__fmul_rn(-2.0f * dt, P.half_rate_omega));
+        K[C_NDT_DX] = f2(__fmul_rn(-P.inv_dx, dt));
+        K[C_43] = f2(4.0f / 3.0f);
+        K[C_N23] = f2(-2.0f / 3.0f);
+        K[C_GAMMA] = f2(P.gamma);
+        K[C_GM1] = f2(P.gm1);
+        K[C_INV_GM1] = f2(P.inv_gm1);
+        K[C_COOL] = f2(__fmul_rn(-dt, P.inv_cool_beta));
+        K[C_ALPHA] = f2(__fmul_rn(__fmul_rn(0.5f, P.nu), P.inv_sqrt_gm));
+        K[C_ONE] = f2(1.0f);
+    }
+    __syncwarp();
+
+    const int N = rd.N, bs = rd.bs;
+    const size_t nn = (size_t)N * N;
+    // rows [i0, i0 + TH) of the strip from column j0: row chunk ti of C (chunk_start, runtime.cuh)
+    const int lt = g - rd.tile_base;
+    const int strip = lt % rd.tiles_j, ti = rd.chunk0 + lt / rd.tiles_j;
+    const int i0 = chunk_start(ti, N, rd.chunks), TH = chunk_start(ti + 1, N, rd.chunks) - i0;
+    const int j0 = strip * SW_COLS, w = min(SW_COLS, N - j0);
+    const int c0 = 2 * lane - 2;                            // this lane's columns c0, c0 + 1
+    const bool inx = c0 >= 0 && c0 < w, iny = EVEN ? inx : c0 >= 0 && c0 + 1 < w;
+    const bool has_base = a.base_slot >= 0;
+
+    const E* uin = (const E*)rd.slot[a.in_slot];
+    const E* ubase = has_base ? (const E*)rd.slot[a.base_slot] : nullptr;
+    const E* ubg = (const E*)rd.bg;
+
+    E* stencil = (E*)smem_raw;                              // [SW_SLOTS][NF][64]: this lane's pair at 2 lane
+    E* update = stencil + SW_SLOTS * T::STENCIL;            // [SW_USLOTS][NU][64]
+    float* led = (float*)(update + SW_USLOTS * T::UPDATE);  // [ITEMS][64]
+    E* my_stencil = stencil + 2 * lane;
+    E* my_update = update + 2 * lane;
+
+    // ---- row staging -------------------------------------------------------------
+    constexpr int PARTS = STORE == 1 ? 2 : 1;               // planes per field: hi and lo words
+    const int colx = ((j0 + c0) % N + N) % N, coly = colx + 1 == N ? 0 : colx + 1;   // this lane's columns in the mesh
+    auto copy_pair = [&](E* dst, const E* row) {
+        if constexpr (EVEN) copy_async<2 * sizeof(E)>(dst, row + colx);
+        else {
+            copy_async<sizeof(E)>(dst, row + colx);
+            copy_async<sizeof(E)>(dst + 1, row + coly);
+        }
+    };
+    // row rs of the stencil and row ru of the update, as one group
+    auto issue = [&](int rs, int ru) {
+        if (rs <= TH + 1) {
+            const size_t row = (size_t)wrap(wrap(i0 + rs, N), N) * N;   // (twice: a mesh may be one zone wide)
+            E* d = my_stencil + ((rs + 2) & (SW_SLOTS - 1)) * T::STENCIL;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) copy_pair(d + f * 64, uin + (size_t)(PARTS * f) * nn + row);
+        }
+        if (ru >= 0 && ru < TH) {
+            const size_t row = (size_t)(i0 + ru) * N;
+            E* d = my_update + (ru & 1) * T::UPDATE;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                if constexpr (STORE == 1) copy_pair(d + f * 64, uin + (size_t)(2 * f + 1) * nn + row);
+                copy_pair(d + ((STORE == 1 ? NF : 0) + f) * 64, ubg + (size_t)(PARTS * f) * nn + row);
+            }
+            if (has_base) {
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    copy_pair(d + (PARTS * NF + f) * 64, ubase + (size_t)(PARTS * f) * nn + row);
+                    if constexpr (STORE == 1) copy_pair(d + (3 * NF + f) * 64, ubase + (size_t)(2 * f + 1) * nn + row);
+                }
+            }
+        }
+        copy_commit();
+    };
+    issue(-2, -1);
+
+    const float theta = P.plm, pdt = P.pdt;
+    const df32 w1{a.w1f.hi, a.w1f.lo}, wb{a.bff.hi, a.bff.lo};
+    const bool half_avg = a.half_avg != 0;
+    const bool want_amax = a.amax_flag != 0, fake_on = NF == 3 && P.fake_rate != 0.0f;
+    // the T^4 law's slow-start factor exp(-2 pi / (t + dt)) of this stage (physics.rs:683-774)
+    const float slow = NF == 4 && P.cooling_slow_start ? __expf(-6.283185307f / (time + dt)) : 1.0f;
+    // positions: zone centres (y) of the pair, y of the pair's left faces
+    auto at = [](int k, int n) { return min(max(k, 0), n); };
+    const float2 yc2 = make_float2(rd.xcf[at(j0 + c0, N - 1)], rd.xcf[at(j0 + c0 + 1, N - 1)]);
+    const float2 yv2 = make_float2(rd.xvgf[at(j0 + c0, N)], rd.xvgf[at(j0 + c0 + 1, N)]);
+    const float near2 = (P.sink_r2 + P.soft2) * 1.0001f;    // the sinks' vote: softened distance, with a margin
+    // dy^2 + s^2 of a pair of y positions to a body
+    auto col_part = [&](float2 y, float2 by) {
+        const float2 d = sub2(y, by);
+        return fma2(d, d, K[C_SOFT2]);
+    };
+
+    float2 Pm1[NF], P0[NF];           // primitives of rows g - 1 and g
+    float2 xl[NF], xtn, xtt;          // row g - 1: state at its lower x faces, stresses
+    float2 fx[NF], dfy[NF];           // flux through row g - 1's upper x faces; its y fluxes' difference
+    constexpr int NACC = T::SINKS_AT;
+    float2 acc[NACC];                 // ledger items that are live everywhere, summed over rows
+#pragma unroll
+    for (int m = 0; m < NACC; ++m) acc[m] = f2(0.0f);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) Pm1[f] = P0[f] = xl[f] = fx[f] = dfy[f] = f2(0.0f);
+    xtn = xtt = f2(0.0f);
+    bool sinks_seen = false, fake_seen = false;
+    float amax = 0.0f;
+    int brow = i0 / bs, next_flush = bs - i0 % bs;          // row count at which block row `brow` ends
+    const float* xcr = rd.xcf + i0;                         // (the tables go on two entries beyond either end)
+    const float* xvr = rd.xvgf + i0;
+    float x_up = xcr[0], x_c = xcr[0], x_f = xvr[0];        // zone rows g - 1 and g, face g - 1/2
+    E* out = (E*)rd.slot[a.out_slot] + (size_t)i0 * N + j0 + c0;   // this pair of row g - 1
+
+    for (int n = -2; n <= TH + 1; ++n) {
+        issue(n + 1, n - 1);
+        const int gr = n - 1;
+        // positions of the next iteration's rows, loaded a row ahead
+        const float x_c_next = xcr[gr + 1], x_f_next = xvr[gr + 1];
+
+        // ---- row n -> primitives (try_block_primitive, scheme.rs:185-199) ------------
+        float2 pn[NF];
+        {
+            copy_wait<1>();   // the row's group, and that of the update below
+            const E* sb = my_stencil + ((n + 2) & (SW_SLOTS - 1)) * T::STENCIL;
+            float2 u[NF];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) u[f] = pair_of(sb + f * 64);
+            int ea = 0, eb = 0;
+            if constexpr (NF == 3) {
+                if (P.has_density_floor) {
+                    if (u[0].x < P.density_floor) { u[0].x = P.density_floor; u[1].x = u[2].x = 0.0f; }
+                    if (u[0].y < P.density_floor) { u[0].y = P.density_floor; u[1].y = u[2].y = 0.0f; }
+                }
+                const float2 ir = rcp2(u[0]);
+                pn[0] = u[0];
+                pn[1] = mul2(u[1], ir);
+                pn[2] = mul2(u[2], ir);
+                ea = u[0].x < 0.0f;
+                eb = u[0].y < 0.0f;
+            } else {
+                const float2 ir = rcp2(u[0]);
+                pn[0] = u[0];
+                pn[1] = mul2(u[1], ir);
+                pn[2] = mul2(u[2], ir);
+                pn[3] = mul2(sub2(u[3], mul2(mul2(K[C_HALF], u[0]), fma2(pn[1], pn[1], mul2(pn[2], pn[2])))), K[C_GM1]);
+                // the floors and checks of Euler::try_to_primitive (physics.rs:631-660)
+                if (P.has_density_floor) {
+                    if (pn[0].x < P.density_floor) {
+                        pn[0].x = P.density_floor;
+                        pn[1].x = pn[2].x = 0.0f;
+                        pn[3].x = P.density_floor_pow_gamma;
+                    }
+                    if (pn[0].y < P.density_floor) {
+                        pn[0].y = P.density_floor;
+                        pn[1].y = pn[2].y = 0.0f;
+                        pn[3].y = P.density_floor_pow_gamma;
+                    }
+                }
+                if (P.has_pressure_floor) {
+                    if (pn[3].x < P.pressure_floor && !(pn[0].x < 0.0f)) pn[3].x = P.pressure_floor;
+                    if (pn[3].y < P.pressure_floor && !(pn[0].y < 0.0f)) pn[3].y = P.pressure_floor;
+                }
+                ea = pn[0].x < 0.0f ? 1 : (pn[3].x <= 0.0f ? 2 : 0);
+                eb = pn[0].y < 0.0f ? 1 : (pn[3].y <= 0.0f ? 2 : 0);
+            }
+            if (__any_sync(0xffffffffu, ea || eb) && n >= 0 && n < TH) {
+                if (ea && inx) atomicMin(a.err_key, error_key(a.stage, ri, rd, i0 + n, j0 + c0, ea));
+                if (eb && iny) atomicMin(a.err_key, error_key(a.stage, ri, rd, i0 + n, j0 + c0 + 1, eb));
+            }
+        }
+
+        if (gr >= -1) {
+            // ---- slopes and stresses of row g (scheme.rs:216-254) ---------------------
+            float lv[NF], rv[NF];                           // columns c0 - 1 and c0 + 2
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                lv[f] = __shfl_up_sync(0xffffffffu, P0[f].y, 1);
+                rv[f] = __shfl_down_sync(0xffffffffu, P0[f].x, 1);
+                // the two outermost columns have no such neighbour: NaN in a
+                // read-set check build (tma.cuh), whose states must not change
+                if (lane == 0) lv[f] = poison_or(lv[f]);
+                if (lane == 31) rv[f] = poison_or(rv[f]);
+            }
+            float2 thx = K[C_THETA], thy = thx;
+            if (pdt > 0.0f) {   // (densities below 0 fail the advance before their slopes count)
+                thx = make_float2((Pm1[0].x < pdt || P0[0].x < pdt || pn[0].x < pdt) ? 0.0f : theta,
+                                  (Pm1[0].y < pdt || P0[0].y < pdt || pn[0].y < pdt) ? 0.0f : theta);
+                thy = make_float2((lv[0] < pdt || P0[0].x < pdt || P0[0].y < pdt) ? 0.0f : theta,
+                                  (P0[0].x < pdt || P0[0].y < pdt || rv[0] < pdt) ? 0.0f : theta);
+            }
+            float2 gx[NF], gy[NF];
+#pragma unroll
+            for (int f = 0; f < NF; ++f) {
+                gx[f] = plm_gradient2(thx, Pm1[f], P0[f], pn[f]);
+                gy[f] = plm_gradient2(thy, make_float2(lv[f], P0[f].x), P0[f], make_float2(P0[f].y, rv[f]));
+            }
+            const float2 da = mul2(gx[1], K[C_INV_DX]), db = mul2(gy[2], K[C_INV_DX]);
+            const float2 lb = mul2(K[C_LAMBDA], add2(da, db));
+            const float2 cv = P.visc == 0 ? mul2(K[C_NU], P0[0]) : (NF == 3 ? P0[0] : mul2(K[C_GAMMA], P0[NF - 1]));
+            const float2 txx = mul2(cv, fma2(K[C_43], da, fma2(K[C_N23], db, lb)));
+            const float2 tyy = mul2(cv, fma2(K[C_43], db, fma2(K[C_N23], da, lb)));
+            const float2 txy = mul2(cv, mul2(add2(gx[2], gy[1]), K[C_INV_DX]));
+
+            if (gr >= 0) {
+                // ---- y fluxes of row g at the pair's left faces -------------------------
+                float2 Fy[NF], dfy_new[NF];
+                {
+                    float2 pl[NF], pr[NF];
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        const float2 e = fma2(gy[f], K[C_HALF], P0[f]);
+                        pl[f] = make_float2(__shfl_up_sync(0xffffffffu, e.y, 1), e.x);
+                        pr[f] = fma2(gy[f], K[C_NHALF], P0[f]);
+                    }
+                    const float2 tn = add2(make_float2(__shfl_up_sync(0xffffffffu, tyy.y, 1), tyy.x), tyy);
+                    const float2 tt = add2(make_float2(__shfl_up_sync(0xffffffffu, txy.y, 1), txy.x), txy);
+                    float2 cs2 = f2(0.0f), k = K[C_HALF], vxs = f2(0.0f), vys = f2(0.0f);
+                    if constexpr (NF == 3) {
+                        // cs2 = -phi / M^2 (physics.rs:584-607), Plummer potential
+                        const float d1 = x_c - B.p1.x, d2 = x_c - B.p2.x;
+                        const float2 r1 = rsqrt2(add2(f2(__fmul_rn(d1, d1)), col_part(yv2, K[C_Y1])));
+                        const float2 r2 = rsqrt2(add2(f2(__fmul_rn(d2, d2)), col_part(yv2, K[C_Y2])));
+                        cs2 = mul2(fma2(K[C_M1], r1, mul2(K[C_M2], r2)), K[C_INV_MACH2]);
+                    } else {
+                        vxs = add2(make_float2(lv[1], P0[1].x), P0[1]);
+                        vys = add2(make_float2(lv[2], P0[2].x), P0[2]);
+                    }
+                    if (P.visc != 0) {
+                        k = alpha_half_k2(K, B, x_c, yv2);
+                        if constexpr (NF == 3) k = mul2(k, cs2);
+                    }
+                    faces2<NF, 1>(K, pl, pr, cs2, k, tn, tt, vxs, vys, Fy);
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        const float2 right = make_float2(Fy[f].y, __shfl_down_sync(0xffffffffu, Fy[f].x, 1));
+                        dfy_new[f] = sub2(right, Fy[f]);
+                    }
+                }
+                // ---- x fluxes between rows g - 1 and g ----------------------------------
+                float2 Fx[NF];
+                {
+                    float2 pr[NF];
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) pr[f] = fma2(gx[f], K[C_NHALF], P0[f]);
+                    float2 cs2 = f2(0.0f), k = K[C_HALF], vxs = f2(0.0f), vys = f2(0.0f);
+                    if constexpr (NF == 3) {
+                        const float d1 = x_f - B.p1.x, d2 = x_f - B.p2.x;
+                        const float2 r1 = rsqrt2(add2(f2(__fmul_rn(d1, d1)), col_part(yc2, K[C_Y1])));
+                        const float2 r2 = rsqrt2(add2(f2(__fmul_rn(d2, d2)), col_part(yc2, K[C_Y2])));
+                        cs2 = mul2(fma2(K[C_M1], r1, mul2(K[C_M2], r2)), K[C_INV_MACH2]);
+                    } else {
+                        vxs = add2(Pm1[1], P0[1]);
+                        vys = add2(Pm1[2], P0[2]);
+                    }
+                    if (P.visc != 0) {
+                        k = alpha_half_k2(K, B, x_f, yc2);
+                        if constexpr (NF == 3) k = mul2(k, cs2);
+                    }
+                    faces2<NF, 0>(K, xl, pr, cs2, k, add2(xtn, txx), add2(xtt, txy), vxs, vys, Fx);
+                }
+                // ---- update of row g - 1 (side effects masked in the first iteration) ------
+                {
+                    const int ru = gr - 1;
+                    const bool up_ok = ru >= 0;
+                    const E* sb = my_stencil + ((ru + 2) & (SW_SLOTS - 1)) * T::STENCIL;
+                    const E* q = my_update + (ru & 1) * T::UPDATE;
+                    const E* qg = q + (STORE == 1 ? NF * 64 : 0);                    // background
+                    const E* qb = qg + NF * 64;                                      // RK base
+                    float2 uc[NF], u0[NF];
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) {
+                        uc[f] = pair_of(sb + f * 64);
+                        u0[f] = pair_of(qg + f * 64);
+                    }
+                    // sources of the pair (Physics::source_terms, physics.rs:423-457;
+                    // Isothermal 528-582, Euler 683-774)
+                    float2 tot[NF], it[NACC];
+                    const float dx1 = x_up - B.p1.x, dx2 = x_up - B.p2.x;
+                    const float2 dy1 = sub2(yc2, K[C_Y1]), dy2 = sub2(yc2, K[C_Y2]);
+                    // Plummer accelerations (kepler-two-body, restated): -m d / (d^2 + s^2)^(3/2)
+                    const float2 t1 = fma2(dy1, dy1, f2(fmaf(dx1, dx1, P.soft2)));
+                    const float2 t2 = fma2(dy2, dy2, f2(fmaf(dx2, dx2, P.soft2)));
+                    const float2 r1 = rsqrt2(t1), r2 = rsqrt2(t2);
+                    const float2 r13 = mul2(r1, mul2(r1, r1)), r23 = mul2(r2, mul2(r2, r2));
+                    const float2 q1 = mul2(mul2(uc[0], K[C_NM1DT]), r13);
+                    const float2 q2 = mul2(mul2(uc[0], K[C_NM2DT]), r23);
+                    constexpr int G2 = NF - 1, BU = 2 * (NF - 1);
+                    it[0] = mul2(q1, f2(dx1));
+                    it[1] = mul2(q1, dy1);
+                    it[G2] = mul2(q2, f2(dx2));
+                    it[G2 + 1] = mul2(q2, dy2);
+                    // buffer: 0.5 rate (1 + tanh((r - R) / scale)) Omega_outer, 1 + tanh(y) = 2 / (1 + exp(-2y))
+                    const float2 rr2 = fma2(yc2, yc2, f2(__fmul_rn(x_up, x_up)));
+                    const float2 yb = mul2(sub2(sqrt2(rr2), K[C_RADIUS]), K[C_BUF_SLOPE]);
+                    const float2 den = add2(K[C_ONE], make_float2(__expf(yb.x), __expf(yb.y)));
+                    const float2 kb = mul2(K[C_BUF_RATE], rcp2(den));
+#pragma unroll
+                    for (int f = 0; f < NF; ++f) it[BU + f] = mul2(sub2(uc[f], u0[f]), kb);
+                    tot[0] = it[BU];
+                    tot[1] = add2(add2(it[0], it[G2]), it[BU + 1]);
+                    tot[2] = add2(add2(it[1], it[G2 + 1]), it[BU + 2]);
+                    if constexpr (NF == 4) {
+                        // primitive velocities and specific internal energy (no floors, physics.rs:696)
+                        const float2 ir = rcp2(uc[0]);
+                        const float2 vx = mul2(uc[1], ir), vy = mul2(uc[2], ir);
+                        const float2 v2 = fma2(vx, vx, mul2(vy, vy));
+                        const float2 e0 = mul2(sub2(uc[3], mul2(mul2(K[C_HALF], uc[0]), v2)), ir);
+                        // the work of gravity
+                        it[2] = fma2(it[0], vx, mul2(it[1], vy));
+                        it[5] = fma2(it[3], vx, mul2(it[4], vy));
+                        // Cooling of the specific internal energy, de = e_cooled - e0 formed directly
+                        // (e0 (exp(-c) - 1), e0 ((1 + x)^(-1/3) - 1) through expm1 and log1p): as a
+                        // difference of two near-equal energies it loses ~1e-7 / (c or x) of its value.
+                        // The item's mass and momentum are zero in FP32: in the reference they are
+                        // only the rounding of a prim -> cons round trip.
+                        float2 dec;
+                        if (P.cooling_kind == 1) {
+                            // beta-cooling (not in the reference): e -> e exp(-Omega dt / beta),
+                            // Omega^2 = sum m / (d^2 + s^2)^(3/2)
+                            const float2 om = sqrt2(fma2(K[C_M1], r13, mul2(K[C_M2], r23)));
+                            const float2 c = mul2(om, K[C_COOL]);
+                            if (__any_sync(0xffffffffu, fabsf(c.x) > 0.35f || fabsf(c.y) > 0.35f))
+                                dec = mul2(e0, make_float2(expm1f(c.x), expm1f(c.y)));
+                            else
+                                dec = mul2(e0, expm1_small2(c));
+                        } else {
+                            // T^4 law: e -> e (1 + 3 a e^3 dt)^(-1/3), a = coefficient / rho^n x slow start
+                            float d2[2];
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const float rho = s ? uc[0].y : uc[0].x, e = s ? e0.y : e0.x;
+                                float rho_n = 1.0f;
+                                for (int m = 0; m < P.density_index; ++m) rho_n = __fmul_rn(rho_n, rho);
+                                const float ac = __fmul_rn(__fdividef(P.cool_coef, rho_n), slow);
+                                const float z = __fmul_rn(__fmul_rn(__fmul_rn(3.0f, ac), __fmul_rn(__fmul_rn(e, e), e)), dt);
+                                d2[s] = __fmul_rn(e, expm1f(__fmul_rn(log1pf(z), -1.0f / 3.0f)));
+                            }
+                            dec = make_float2(d2[0], d2[1]);
+                        }
+                        if (P.has_mach_ceiling) {
+                            // e >= 2 e_kinetic / (gamma (gamma - 1) M^2)
+                            const float2 ek = mul2(f2(0.5f * P.k_mach_ceiling), v2);
+                            const float eca = e0.x + dec.x, ecb = e0.y + dec.y;
+                            const float ma = fmaxf(eca, ek.x), mb = fmaxf(ecb, ek.y);
+                            if (ma != eca) dec.x = ma - e0.x;
+                            if (mb != ecb) dec.y = mb - e0.y;
+                        }
+                        it[10] = mul2(uc[0], dec);
+                        tot[3] = add2(add2(add2(it[2], it[5]), it[BU + 3]), it[10]);
+                    }
+                    // sinks: only where a zone of the warp lies inside a sink radius
+                    const bool near = (inx && fminf(t1.x, t2.x) < near2) || (iny && fminf(t1.y, t2.y) < near2);
+                    if (__any_sync(0xffffffffu, near) && up_ok) {
+                        float* sl = led + T::SINKS_AT * 64 + 2 * lane;
+                        if (!sinks_seen) {
+#pragma unroll
+                            for (int m = 0; m < 2 * NF; ++m) *(float2*)(sl + m * 64) = f2(0.0f);
+                            sinks_seen = true;
+                        }
+#pragma unroll
+                        for (int side = 0; side < 2; ++side) {
+                            float us[NF], s1[NF], s2[NF];
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) us[f] = side ? uc[f].y : uc[f].x;
+                            sink_items_exact<NF>(P, B, us, x_up, side ? yc2.y : yc2.x, dt, s1, s2);
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) {
+                                const float sk = s1[f] + s2[f];
+                                if (side) tot[f].y += sk;
+                                else tot[f].x += sk;
+                                sl[f * 64 + side] += s1[f];
+                                sl[(NF + f) * 64 + side] += s2[f];
+                            }
+                        }
+                    }
+                    // fake mass: u0 rate dt unless Sigma < Sigma_0 threshold
+                    if (fake_on && up_ok) {
+                        float* sl = led + T::FAKE_AT * 64 + 2 * lane;
+                        const bool offa = uc[0].x < u0[0].x * P.fake_thr, offb = uc[0].y < u0[0].y * P.fake_thr;
+#pragma unroll
+                        for (int f = 0; f < 3; ++f) {
+                            const float2 fk = mul2(mul2(u0[f], f2(P.fake_rate)), f2(dt));
+                            const float2 on = make_float2(offa ? 0.0f : fk.x, offb ? 0.0f : fk.y);
+                            tot[f] = add2(tot[f], on);
+                            float2* s = (float2*)(sl + f * 64);
+                            *s = fake_seen ? add2(*s, on) : on;
+                        }
+                        fake_seen = true;
+                    }
+                    // flux divergence and the RK update (scheme.rs:290-305; state.rs:183-199)
+                    float2 uo[NF];
+                    if constexpr (STORE == 1) {
+                        df2 o[NF];
+#pragma unroll
+                        for (int f = 0; f < NF; ++f) {
+                            const float2 du = mul2(add2(sub2(Fx[f], fx[f]), dfy[f]), K[C_NDT_DX]);
+                            o[f] = df_add_f2(df2{uc[f], pair_of(q + f * 64)}, add2(du, tot[f]));
+                        }
+                        if (has_base) {
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) {
+                                const df2 b0{pair_of(qb + f * 64), pair_of(qb + (NF + f) * 64)};
+                                if (half_avg) {
+                                    const df2 sm = df_add2(o[f], b0);
+                                    o[f] = {mul2(sm.hi, K[C_HALF]), mul2(sm.lo, K[C_HALF])};
+                                } else {
+                                    const df2 x1 = df_mul2(o[f], w1), x2 = df_mul2(b0, wb);
+                                    o[f] = df_add2(x1, x2);
+                                }
+                            }
+                        }
+                        if (up_ok && inx) {
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) {
+                                E* oh = out + (size_t)(2 * f) * nn;
+                                E* ol = out + (size_t)(2 * f + 1) * nn;
+                                if constexpr (EVEN) {
+                                    *(float2*)oh = o[f].hi;
+                                    *(float2*)ol = o[f].lo;
+                                } else {
+                                    oh[0] = o[f].hi.x;
+                                    ol[0] = o[f].lo.x;
+                                    if (iny) { oh[1] = o[f].hi.y; ol[1] = o[f].lo.y; }
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int f = 0; f < NF; ++f) uo[f] = o[f].hi;
+                    } else {
+                        double2 o[NF];
+                        const double keep = -a.bf + 1.0;
+#pragma unroll
+                        for (int f = 0; f < NF; ++f) {
+                            const float2 du = mul2(add2(sub2(Fx[f], fx[f]), dfy[f]), K[C_NDT_DX]);
+                            const float2 inc = add2(du, tot[f]);
+                            o[f] = *(const double2*)(sb + f * 64);
+                            o[f].x += (double)inc.x;
+                            o[f].y += (double)inc.y;
+                            if (has_base) {
+                                const double2 b0 = *(const double2*)(qb + f * 64);
+                                o[f].x = o[f].x * keep + b0.x * a.bf;
+                                o[f].y = o[f].y * keep + b0.y * a.bf;
+                            }
+                            uo[f] = make_float2((float)o[f].x, (float)o[f].y);
+                        }
+                        if (up_ok && inx) {
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) {
+                                E* p = out + (size_t)f * nn;
+                                if constexpr (EVEN) *(double2*)p = o[f];
+                                else {
+                                    p[0] = o[f].x;
+                                    if (iny) p[1] = o[f].y;
+                                }
+                            }
+                        }
+                    }
+                    if (up_ok) {
+#pragma unroll
+                        for (int m = 0; m < NACC; ++m) acc[m] = add2(acc[m], it[m]);
+                        if (want_amax) {
+                            float ua[NF], ub[NF];
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) { ua[f] = uo[f].x; ub[f] = uo[f].y; }
+                            if (inx) amax = fmaxf(max_speed_exact<NF>(P, ua), amax);
+                            if (iny) amax = fmaxf(max_speed_exact<NF>(P, ub), amax);
+                        }
+                        if (ru + 1 == next_flush || ru + 1 == TH) {   // the end of a block row, or of the chunk
+#pragma unroll
+                            for (int m = 0; m < NACC; ++m) {
+                                *(float2*)(led + m * 64 + 2 * lane) = acc[m];
+                                acc[m] = f2(0.0f);
+                            }
+                            flush_strip<NF, STORE>(rd, strip, ti, brow, led, sinks_seen, fake_seen, a.in_slot,
+                                                   a.base_slot, a.out_slot, a.stage, a.bf);
+                            sinks_seen = fake_seen = false;
+                            ++brow;
+                            next_flush += bs;
+                        }
+                        out += N;
+                    }
+                }
+#pragma unroll
+                for (int f = 0; f < NF; ++f) { fx[f] = Fx[f]; dfy[f] = dfy_new[f]; }
+            }
+#pragma unroll
+            for (int f = 0; f < NF; ++f) xl[f] = fma2(gx[f], K[C_HALF], P0[f]);
+            xtn = txx;
+            xtt = txy;
+        }
+#pragma unroll
+        for (int f = 0; f < NF; ++f) { Pm1[f] = P0[f]; P0[f] = pn[f]; }
+        x_up = x_c;
+        x_c = x_c_next;
+        x_f = x_f_next;
+    }
+
+    if (want_amax) {
+        const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));   // amax >= 0: its bits are in order
+        if (lane == 0 && m) atomicMax(rd.amax, (unsigned long long)__double_as_longlong((double)__uint_as_float(m)));
+    }
+}
+
+}  // namespace b2d

@@ -49,7 +49,7 @@ typedef enum b2d_status {
     B2D_ERR_NEG_DENSITY    = 1,  /* HydroErrorType::NegativeDensity            */
     B2D_ERR_NEG_PRESSURE   = 2,  /* HydroErrorType::NegativePressure           */
     B2D_ERR_UNBOUND_ORBIT  = 3,  /* HydroErrorType::OrbitalEvolutionError      */
-    B2D_ERR_TIMEOUT        = 4,  /* a bounded device wait gave up               */
+    B2D_ERR_TIMEOUT        = 4,  /* not raised: no kernel waits on another's writes */
     B2D_ERR_CUDA           = 5,  /* CUDA runtime error (message via b2d_last_error) */
     B2D_ERR_INVALID        = 6,  /* bad argument                                */
     B2D_ERR_UNSUPPORTED    = 7   /* option combination not built                */
@@ -283,34 +283,31 @@ b2d_status b2d_initial_state(const b2d_config* cfg, const b2d_disk_model* model,
 /* ------------------------------------------------------------------------ */
 /* Tuning / introspection. */
 
-/* Tile shape of the stage kernel for a context: width in zones along j (a
- * multiple of 32 dividing block_size) and height along i (dividing
- * block_size).  The paired-column FP32 kernel (precision FP32_COMP,
- * isothermal) also takes 128-, 256- or 512-column tiles that span whole
- * blocks of 64 columns or more side by side.  The FP64 kernel cuts blocks into
- * sub-tiles of its own and takes any shape here.  0 keeps the current value. */
+/* Tile shape of a context: width in zones along j (a multiple of 32 dividing
+ * block_size; with compensated FP32 also 128, 256 or 512 columns spanning
+ * whole blocks of 64 columns or more side by side) and height along i
+ * (dividing block_size).  The FP32 kernel takes row chunks of the height; its
+ * column strips are 60 wide whatever the width.  The FP64 kernel cuts blocks
+ * into sub-tiles of its own, whatever the shape.  0 keeps the current value. */
 b2d_status b2d_set_tile(b2d_ctx* ctx, int32_t tile_w, int32_t tile_h);
 b2d_status b2d_get_tile(const b2d_ctx* ctx, int32_t* tile_w, int32_t* tile_h);
 
-/* Row chunks of the FP32 stage kernels (the paired-column kernel: FP32_COMP,
- * isothermal, tile width 64, 128, 256 or 512; the TMA-staged kernel: FP32 tiles
- * whose width is a multiple of 32, at most 128).  rows > 0: every column strip of tile
- * width is covered in ceil(N / rows) row chunks of near-equal height (at most
- * `rows`; 8 <= rows <= block_size), each of which may cross one block
- * boundary, so that the stage's CTAs can fill whole waves of the GPU; the
- * tile height then applies only to the other stage kernels.  0 (default):
- * block-aligned tiles of the tile height.  No reference counterpart: the
- * reference advances block by block (src/scheme.rs:323-349); results and
- * per-block ledgers do not depend on the tiling. */
+/* Row chunks of the FP32 stage kernel.  rows > 0: every column strip is covered
+ * in ceil(N / rows) row chunks of near-equal height (at most `rows`;
+ * 8 <= rows <= block_size), which may cross block boundaries, so that the
+ * stage's CTAs can fill whole waves of the GPU; the tile height then has no
+ * effect.  0 (default): block-aligned chunks of the tile height.  No reference
+ * counterpart: the reference advances block by block (src/scheme.rs:323-349);
+ * states do not depend on the tiling, per-block ledgers only by the order of
+ * their FP32 sums. */
 b2d_status b2d_set_strip_rows(b2d_ctx* ctx, int32_t rows);
 b2d_status b2d_get_strip_rows(const b2d_ctx* ctx, int32_t* rows);
 
-/* Tile autotuner (of the FP32 precisions; an FP64 context is timed once, as it
- * is): times every tile shape that divides the block size (width
- * 32..128; height 8..128), the paired FP32 kernel's tiles
- * that span blocks (128, 256 or 512 columns) and, where that kernel runs, the
- * strip rows that fill one, two or three whole waves of its resident CTAs, over `reps` advances of `fold` steps with CUDA events; keeps
- * the fastest (b2d_get_tile and b2d_get_strip_rows report it).  The
+/* Tile autotuner: for the FP32 kernel, times the tile heights that divide the
+ * block size (at most 128) and the strip rows that fill one, two or three
+ * whole waves of its resident CTAs, over `reps` advances of `fold` steps with
+ * CUDA events, and keeps the fastest (b2d_get_tile and b2d_get_strip_rows report
+ * it; the tile width stays).  An FP64 context is timed once, as it is.  The
  * context's state is unchanged. */
 b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int32_t* tile_w,
                         int32_t* tile_h, double* ms_per_stage);
