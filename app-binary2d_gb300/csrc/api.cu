@@ -138,7 +138,7 @@ __global__ void prologue_kernel(const RunDev* runs, int fold, int rk, int start,
 
 // State::max_signal_speed (state.rs:121-133) of one run's slot, in the
 // precision the stage kernels use for it at the end of an advance: FP64 for
-// the FP64 path, FP32 of the stored (high) words for the FP32 paths (FP64
+// the FP64 path, FP32 of the stored words for the FP32 paths (FP64
 // divisions and roots on a whole mesh are slow on this GPU).
 template <int NF, int STORE, class R>
 __global__ void max_speed_kernel(const RunDev* runs, int run, int slot)
@@ -150,12 +150,24 @@ __global__ void max_speed_kernel(const RunDev* runs, int run, int slot)
     const size_t z1 = rd.slab_hi > 0 ? (size_t)rd.slab_hi * rd.bs * rd.N : nn;
     R a = R(0);
     for (size_t z = z0 + blockIdx.x * (size_t)blockDim.x + threadIdx.x; z < z1; z += (size_t)gridDim.x * blockDim.x) {
-        R u[NF];
-        for (int f = 0; f < NF; ++f) {
-            if (STORE == 0) u[f] = (R)((const double*)rd.slot[slot])[f * nn + z];
-            else u[f] = (R)((const float*)rd.slot[slot])[(2 * f) * nn + z];
+        if constexpr (std::is_same<R, double>::value) {
+            double u[NF];
+            for (int f = 0; f < NF; ++f) u[f] = ((const double*)rd.slot[slot])[f * nn + z];
+            a = fmax(max_speed_f64<NF>(rd.p, u), a);
+        } else {
+            float hi[NF], lo[NF];
+            for (int f = 0; f < NF; ++f) {
+                if (STORE == 0) {
+                    const double v = ((const double*)rd.slot[slot])[f * nn + z];
+                    hi[f] = (float)v;
+                    lo[f] = (float)(v - (double)hi[f]);
+                } else {
+                    hi[f] = ((const float*)rd.slot[slot])[(2 * f) * nn + z];
+                    lo[f] = ((const float*)rd.slot[slot])[(2 * f + 1) * nn + z];
+                }
+            }
+            a = fmaxf(max_speed_f32<NF>(rd.pf, hi, lo), a);
         }
-        a = rmax(max_signal_speed<NF, R>(params_of<R>(rd), u), a);
     }
     __shared__ double red[256];
     red[threadIdx.x] = a;
@@ -259,9 +271,9 @@ struct RunHost {
     double* ledger[NSLOTS] = {};
     double* elements[NSLOTS] = {};
     double* partial = nullptr;
-    unsigned* counter = nullptr;
+    size_t partial_bytes = 0;
     double *xc = nullptr, *xv = nullptr;
-    float *xcf = nullptr, *xvgf = nullptr;
+    float2 *xcf = nullptr, *xvf = nullptr;
     double* buffer = nullptr;   // FP64: the buffer's rate of every zone
     double* stage_time = nullptr;
     double* orbit = nullptr;
@@ -295,6 +307,8 @@ struct b2d_ctx {
     std::vector<RunHost> runs;
     std::vector<RunDev> rdev_h;
     RunDev* rdev = nullptr;
+    int* d_bases = nullptr;           // [nruns] first CTA of each run
+    int stage_window = 1;             // stages whose ledger pieces fit their buffers
     // control arrays (device)
     double* d_dt = nullptr;           // [nruns]
     double* d_time = nullptr;         // [nruns][NSLOTS]
@@ -485,11 +499,11 @@ static void free_ctx(b2d_ctx* ctx)
         const size_t ri = &r - ctx->runs.data();
         if (ri < ctx->rdev_h.size())
             for (int s = 0; s < NSLOTS; ++s) cudaFree(ctx->rdev_h[ri].tracers[s]);
-        cudaFree(r.buffer); cudaFree(r.bg); cudaFree(r.partial); cudaFree(r.counter);
-        cudaFree(r.xc); cudaFree(r.xv); cudaFree(r.xcf); cudaFree(r.xvgf);
+        cudaFree(r.buffer); cudaFree(r.bg); cudaFree(r.partial);
+        cudaFree(r.xc); cudaFree(r.xv); cudaFree(r.xcf); cudaFree(r.xvf);
         cudaFree(r.stage_time); cudaFree(r.orbit); cudaFree(r.stage_ds); cudaFree(r.stage_de);
     }
-    cudaFree(ctx->rdev); cudaFree(ctx->d_dt); cudaFree(ctx->d_time); cudaFree(ctx->d_iter);
+    cudaFree(ctx->rdev); cudaFree(ctx->d_bases); cudaFree(ctx->d_dt); cudaFree(ctx->d_time); cudaFree(ctx->d_iter);
     cudaFree(ctx->d_amax); cudaFree(ctx->d_err_key); cudaFree(ctx->d_adv_count); cudaFree(ctx->d_staging);
     for (cudaEvent_t e : ctx->ev) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -504,7 +518,6 @@ static void free_ctx(b2d_ctx* ctx)
     delete ctx;
 }
 
-constexpr int TABLE_PAD = 4;     // entries of the FP32 position tables beyond either end
 constexpr int STRIP_COLS = 60;   // SW_COLS of the FP32 kernel (stagew.cuh)
 
 // Row chunks per column strip of a run: block-aligned tiles of height th, or,
@@ -521,6 +534,42 @@ static bool even_columns(const b2d_ctx* ctx)
     for (const RunHost& r : ctx->runs)
         if (r.N % 2) return false;
     return true;
+}
+
+// Buffers for the ledger pieces of as many stages as PIECE_BYTES hold (at
+// least one, at most an advance's capacity), and the run descriptors and first
+// CTAs on the device.  Graphs that hold the old descriptors go.
+static b2d_status alloc_pieces(b2d_ctx* ctx)
+{
+    constexpr size_t PIECE_BYTES = 64u << 20;
+    auto stage_bytes = [&](const RunDev& d) { return sizeof(double) * d.nblocks * d.tiles_per_block * NITEMS * ctx->nf; };
+    size_t total = 0;
+    std::vector<int> bases;
+    for (const RunDev& d : ctx->rdev_h) {
+        total += stage_bytes(d);
+        bases.push_back(d.tile_base);
+    }
+    ctx->stage_window = (int)std::min<size_t>(std::max<size_t>(PIECE_BYTES / total, 1), std::max(ctx->max_stages, 1));
+    for (int i = 0; i < ctx->nruns; ++i) {
+        RunHost& r = ctx->runs[i];
+        RunDev& d = ctx->rdev_h[i];
+        const size_t bytes = stage_bytes(d) * ctx->stage_window;
+        if (bytes > r.partial_bytes) {
+            CUDA_TRY(cudaFree(r.partial));
+            r.partial = nullptr;
+            r.partial_bytes = 0;
+            CUDA_TRY(cudaMalloc(&r.partial, bytes));
+            r.partial_bytes = bytes;
+        }
+        CUDA_TRY(cudaMemset(r.partial, 0, bytes));   // the words of items that are always zero are never written
+        d.partial = r.partial;
+        d.stage_window = ctx->stage_window;
+    }
+    CUDA_TRY(cudaMemcpy(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * ctx->nruns, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpy(ctx->d_bases, bases.data(), sizeof(int) * ctx->nruns, cudaMemcpyHostToDevice));
+    for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
+    ctx->graphs.clear();
+    return B2D_OK;
 }
 
 // Rebuild the tile bookkeeping for the current tile shape and push the run
@@ -554,18 +603,9 @@ static b2d_status sync_rundev(b2d_ctx* ctx)
             }
             d.tiles_per_block = rows * cols;
         }
-        CUDA_TRY(cudaFree(r.partial));
-        r.partial = nullptr;
-        const size_t partial_bytes = sizeof(double) * r.nblocks * d.tiles_per_block * NITEMS * ctx->nf;
-        CUDA_TRY(cudaMalloc(&r.partial, partial_bytes));
-        CUDA_TRY(cudaMemset(r.partial, 0, partial_bytes));   // the words of items that are always zero are never written
-        d.partial = r.partial;
     }
     ctx->total_tiles = base;
-    CUDA_TRY(cudaMemcpy(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * ctx->nruns, cudaMemcpyHostToDevice));
-    for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
-    ctx->graphs.clear();
-    return B2D_OK;
+    return alloc_pieces(ctx);
 }
 
 static b2d_status ensure_stage_capacity(b2d_ctx* ctx, int fold)
@@ -593,10 +633,7 @@ static b2d_status ensure_stage_capacity(b2d_ctx* ctx, int fold)
         ctx->rdev_h[i].stage_de = r.stage_de;
     }
     ctx->max_stages = cap;
-    CUDA_TRY(cudaMemcpy(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * ctx->nruns, cudaMemcpyHostToDevice));
-    for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
-    ctx->graphs.clear();
-    return B2D_OK;
+    return alloc_pieces(ctx);
 }
 
 extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t precision, b2d_status* status)
@@ -634,6 +671,7 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
     } while (0)
     CREATE_TRY(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     CREATE_TRY(cudaMalloc(&ctx->rdev, sizeof(RunDev) * nruns));
+    CREATE_TRY(cudaMalloc(&ctx->d_bases, sizeof(int) * nruns));
     CREATE_TRY(cudaMalloc(&ctx->d_dt, sizeof(double) * nruns));
     CREATE_TRY(cudaMalloc(&ctx->d_time, sizeof(double) * nruns * NSLOTS));
     CREATE_TRY(cudaMalloc(&ctx->d_iter, sizeof(long long) * nruns * NSLOTS));
@@ -671,37 +709,36 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
         }
         CREATE_TRY(cudaMalloc(&r.bg, r.state_bytes));
         CREATE_TRY(cudaMemset(r.bg, 0, r.state_bytes));
-        CREATE_TRY(cudaMalloc(&r.counter, sizeof(unsigned) * r.nblocks));
-        CREATE_TRY(cudaMemset(r.counter, 0, sizeof(unsigned) * r.nblocks));
         // geometry tables
         std::vector<double> xc(r.N), xv((size_t)r.nb * (r.bs + 1));
         for (int b = 0; b < r.nb; ++b) {
             host_cell_centers(&cfgs[i], b, xc.data() + (size_t)b * r.bs);
             host_block_vertices(&cfgs[i], b, xv.data() + (size_t)b * (r.bs + 1));
         }
-        std::vector<float> xcf(xc.begin(), xc.end()), xvf(xv.begin(), xv.end());
-        auto pad = [](std::vector<float>& v) {   // TABLE_PAD entries beyond either end, for row positions read ahead
-            v.insert(v.begin(), TABLE_PAD, v.front());
-            v.insert(v.end(), TABLE_PAD, v.back());
+        // centres, and faces by global index (face k of block k / bs, the last
+        // block's top face last), as FP32 high and low words
+        auto split = [](double v) {
+            const float hi = (float)v;
+            return make_float2(hi, (float)(v - (double)hi));
         };
-        // row faces by global index: face k of block k / bs, the last block's top face last
-        std::vector<float> xvgf((size_t)r.N + 1);
-        for (int k = 0; k < r.N; ++k) xvgf[k] = xvf[(size_t)(k / r.bs) * (r.bs + 1) + k % r.bs];
-        xvgf[r.N] = xvf[(size_t)(r.nb - 1) * (r.bs + 1) + r.bs];
-        pad(xcf);
-        pad(xvgf);
+        std::vector<float2> xcf, xvf;
+        for (int k = 0; k < r.N; ++k) {
+            xcf.push_back(split(xc[k]));
+            xvf.push_back(split(xv[(size_t)(k / r.bs) * (r.bs + 1) + k % r.bs]));
+        }
+        xvf.push_back(split(xv[(size_t)(r.nb - 1) * (r.bs + 1) + r.bs]));
         r.hxc = xc;
         CREATE_TRY(cudaMalloc(&r.xc, sizeof(double) * xc.size()));
         CREATE_TRY(cudaMalloc(&r.xv, sizeof(double) * xv.size()));
-        CREATE_TRY(cudaMalloc(&r.xcf, sizeof(float) * xcf.size()));
-        CREATE_TRY(cudaMalloc(&r.xvgf, sizeof(float) * xvgf.size()));
+        CREATE_TRY(cudaMalloc(&r.xcf, sizeof(float2) * xcf.size()));
+        CREATE_TRY(cudaMalloc(&r.xvf, sizeof(float2) * xvf.size()));
         CREATE_TRY(cudaMemcpy(r.xc, xc.data(), sizeof(double) * xc.size(), cudaMemcpyHostToDevice));
         CREATE_TRY(cudaMemcpy(r.xv, xv.data(), sizeof(double) * xv.size(), cudaMemcpyHostToDevice));
-        CREATE_TRY(cudaMemcpy(r.xcf, xcf.data(), sizeof(float) * xcf.size(), cudaMemcpyHostToDevice));
-        CREATE_TRY(cudaMemcpy(r.xvgf, xvgf.data(), sizeof(float) * xvgf.size(), cudaMemcpyHostToDevice));
+        CREATE_TRY(cudaMemcpy(r.xcf, xcf.data(), sizeof(float2) * xcf.size(), cudaMemcpyHostToDevice));
+        CREATE_TRY(cudaMemcpy(r.xvf, xvf.data(), sizeof(float2) * xvf.size(), cudaMemcpyHostToDevice));
 
         d.N = r.N; d.bs = r.bs; d.nb = r.nb; d.nblocks = r.nblocks;
-        d.xc = r.xc; d.xv = r.xv; d.xcf = r.xcf + TABLE_PAD; d.xvgf = r.xvgf + TABLE_PAD;
+        d.xc = r.xc; d.xv = r.xv; d.xcf = r.xcf; d.xvf = r.xvf;
         for (int s = 0; s < NSLOTS; ++s) {
             d.slot[s] = r.slot[s];
             d.ledger[s] = r.ledger[s];
@@ -718,7 +755,6 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
         d.bg = r.bg;
         d.time = ctx->d_time + (size_t)i * NSLOTS;
         d.iter = ctx->d_iter + (size_t)i * NSLOTS;
-        d.counter = r.counter;
         d.dt = ctx->d_dt + i;
         d.amax = ctx->d_amax + i;
         d.binary_q = cfgs[i].binary_mass_ratio;
@@ -1022,32 +1058,52 @@ static std::vector<StagePlan> plan_advance(int rk, int fold, int start, int* fin
     return plan;
 }
 
-// ItemizedChange<OrbitalElements> of every block over one advance
-// (compute_block_updated_solution, scheme.rs:307-314), after the stage
-// kernels, which only record each block's stage sums ds·dx·dy: the serial
-// FP64 perturbation stays out of their tails.  Two launches:
-//  * elements_de_kernel — one thread per (stage, block, gas item sink1, sink2,
-//    grav1, grav2): that item's perturbation (ItemizedChange::perturbation,
+// The ledgers of every block over one advance (compute_block_updated_solution,
+// scheme.rs:307-314), after the stage kernels, which only write their pieces
+// of each block's sums: folds and the serial FP64 perturbation stay out of
+// their tails.  Two kernels:
+//  * ledger_fold_kernel — one thread per (stage, block, item): the item's pieces,
+//    in order, to the block's stage sums ds·dx·dy, and for the gas items sink1,
+//    sink2, grav1, grav2 their perturbation (ItemizedChange::perturbation,
 //    state.rs:258-281).  An unbound perturbed orbit fails its stage with
 //    OrbitalEvolutionError, reported at position (0, 0) as in the reference.
 //    The reference converts every block's primitives before it updates any
 //    block, so within a stage a cons->prim failure anywhere wins: the key's
 //    block field is saturated and the failing block's index rides in the
 //    zone field; an earlier stage still wins through the stage field.
-//  * elements_sum_kernel — one thread per (block, element component): the
-//    stages in order, e_out = e_in + de averaged like the state
-//    (state.rs:191-197), in the slot schedule of plan_advance.
-__global__ void elements_de_kernel(const RunDev* runs, int nstages, unsigned long long* err_key)
+//    Launched once per stage_window stages: once per advance, but for meshes
+//    of very many pieces.
+//  * ledger_sum_kernel — one thread per (block, ledger word or element
+//    component): the stages in order, x_out = x_in + change averaged like the
+//    state (state.rs:191-197), in the slot schedule of plan_advance.
+template <int NF> __device__ __forceinline__ void fold_item(const RunDev& rd, int s, int block, int item, double* ds)
+{
+    constexpr int NL = NITEMS * NF;
+    const double* p = stage_pieces(rd, s, block, NL) + item * NF;
+    double v[NF] = {};
+#pragma unroll 8
+    for (int q = 0; q < rd.tiles_per_block; ++q)
+#pragma unroll
+        for (int f = 0; f < NF; ++f) v[f] += p[(size_t)q * NL + f];
+    const double area = rd.p.dx * rd.p.dx;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) ds[f] = v[f] * area;
+}
+
+__global__ void ledger_fold_kernel(const RunDev* runs, int first_stage, unsigned long long* err_key)
 {
     const int run = blockIdx.z;
     const RunDev& rd = runs[run];
-    const int s = blockIdx.y;
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;   // block * 4 + item
-    if (s >= nstages || id >= rd.nblocks * 4 || !rd.stage_ds || !rd.stage_de) return;
-    const int block = id >> 2, item = id & 3;
+    const int s = first_stage + blockIdx.y;
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;   // block * 8 + item
+    const int block = id >> 3, item = id & 7;
+    if (block >= rd.nblocks || item >= NITEMS) return;
     if (rd.slab_hi > 0 && (block / rd.nb < rd.slab_lo || block / rd.nb >= rd.slab_hi)) return;   // another slab's
     const int nf = rd.p.hydro == B2D_EULER ? 4 : 3;
-    const double* ds = rd.stage_ds + ((size_t)s * rd.nblocks + block) * NITEMS * nf + item * nf;
+    double* ds = rd.stage_ds + ((size_t)s * rd.nblocks + block) * NITEMS * nf + item * nf;
+    if (nf == 3) fold_item<3>(rd, s, block, item, ds);
+    else fold_item<4>(rd, s, block, item, ds);
+    if (item >= 4) return;
     const double* orbit = rd.orbit + 10 * s;
     double* de = rd.stage_de + (((size_t)s * rd.nblocks + block) * 4 + item) * 4;
     // pert1 (body 1: sink1, grav1) and pert2 (body 2: sink2, grav2), state.rs:261-269
@@ -1062,20 +1118,26 @@ __global__ void elements_de_kernel(const RunDev* runs, int nstages, unsigned lon
     }
 }
 
-__global__ void elements_sum_kernel(const RunDev* runs, int fold, int rk, int start)
+__global__ void ledger_sum_kernel(const RunDev* runs, int fold, int rk, int start)
 {
     const int run = blockIdx.y;
     const RunDev& rd = runs[run];
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;   // block * 28 + item * 4 + component
-    if (id >= rd.nblocks * NITEMS * 4 || !rd.stage_de || !rd.elements[start]) return;
-    const int block = id / (NITEMS * 4), k = id % (NITEMS * 4), item = k / 4;
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;   // ledger words [block][7 nf], then elements [block][7][4]
+    const int nl = NITEMS * (rd.p.hydro == B2D_EULER ? 4 : 3), words = rd.nblocks * nl;
+    if (id >= words + rd.nblocks * NITEMS * 4) return;
+    const bool elements = id >= words;
+    const int w = elements ? id - words : id;
+    const int block = w / (elements ? NITEMS * 4 : nl), k = w % (elements ? NITEMS * 4 : nl);
     if (rd.slab_hi > 0 && (block / rd.nb < rd.slab_lo || block / rd.nb >= rd.slab_hi)) return;
+    double* const* slots = elements ? rd.elements : rd.ledger;
+    // the change of each stage; only the gas items perturb the orbit
+    const double* change = elements ? (k < 16 ? rd.stage_de + (size_t)block * 16 + k : nullptr) : rd.stage_ds + (size_t)block * nl + k;
+    const size_t stride = (size_t)rd.nblocks * (elements ? 16 : nl);
     double e[NSLOTS];
-    e[start] = rd.elements[start][id];
+    e[start] = slots[start][w];
     int s = 0;
     auto stage = [&](int in, int base_slot, int out, double bf) {
-        const double de = item < 4 ? rd.stage_de[((size_t)s * rd.nblocks + block) * 16 + k] : 0.0;
-        double v = e[in] + de;
+        double v = e[in] + (change ? change[s * stride] : 0.0);
         if (base_slot >= 0) v = v * (-bf + 1.0) + e[base_slot] * bf;
         e[out] = v;
         ++s;
@@ -1103,7 +1165,7 @@ __global__ void elements_sum_kernel(const RunDev* runs, int fold, int rk, int st
             base = c;
         }
     }
-    rd.elements[base][id] = e[base];
+    slots[base][w] = e[base];
 }
 
 static int max_blocks(const b2d_ctx* ctx)
@@ -1124,7 +1186,9 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
 {
     StageArgs a;
     a.runs = ctx->rdev;
+    a.tile_bases = ctx->d_bases;
     a.nruns = ctx->nruns;
+    a.pf1 = ctx->rdev_h[0].pf;
     a.th = ctx->th;
     a.in_slot = sp.in;
     a.base_slot = sp.base;
@@ -1136,7 +1200,6 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
     a.w1f = split_df(-sp.bf + 1.0);
     a.bff = split_df(sp.bf);
     a.err_key = ctx->d_err_key;
-    a.pf1 = ctx->rdev_h[0].pf;
     cudaError_t e;
     if (ctx->precision == B2D_PREC_FP64)
         e = launch_stage_f64(ctx->nf, a, ctx->total_tiles, stage_f64_smem(ctx->nf, ctx->sub_h, ctx->sub_w), ctx->stream);
@@ -1284,16 +1347,25 @@ static b2d_status launch_tracers(b2d_ctx* ctx, const StagePlan& sp, bool count)
     return B2D_OK;
 }
 
-// The two per-advance orbital-element kernels (after the stage kernels).
-static b2d_status launch_elements(b2d_ctx* ctx, int fold, int start, int nstages, bool count)
+// Fold the ledger pieces once stage s has filled their buffers, or was the last of nstages.
+static b2d_status launch_fold(b2d_ctx* ctx, int s, int nstages, bool count)
 {
-    const dim3 dg((unsigned)((max_blocks(ctx) * 4 + 127) / 128), (unsigned)nstages, (unsigned)ctx->nruns);
-    elements_de_kernel<<<dg, 128, 0, ctx->stream>>>(ctx->rdev, nstages, ctx->d_err_key);
+    const int first = s / ctx->stage_window * ctx->stage_window;
+    if (s + 1 != nstages && s + 1 != first + ctx->stage_window) return B2D_OK;
+    const dim3 grid((unsigned)((max_blocks(ctx) * 8 + 127) / 128), (unsigned)(s + 1 - first), (unsigned)ctx->nruns);
+    ledger_fold_kernel<<<grid, 128, 0, ctx->stream>>>(ctx->rdev, first, ctx->d_err_key);
     CUDA_TRY(cudaGetLastError());
-    const dim3 sg((unsigned)((max_blocks(ctx) * NITEMS * 4 + 127) / 128), (unsigned)ctx->nruns);
-    elements_sum_kernel<<<sg, 128, 0, ctx->stream>>>(ctx->rdev, fold, ctx->rk, start);
+    if (count) ctx->launches++;
+    return B2D_OK;
+}
+
+// The ledgers' sums over an advance's stages, after the last fold.
+static b2d_status launch_ledgers(b2d_ctx* ctx, int fold, int start, bool count)
+{
+    const dim3 grid((unsigned)((max_blocks(ctx) * NITEMS * (4 + ctx->nf) + 127) / 128), (unsigned)ctx->nruns);
+    ledger_sum_kernel<<<grid, 128, 0, ctx->stream>>>(ctx->rdev, fold, ctx->rk, start);
     CUDA_TRY(cudaGetLastError());
-    if (count) ctx->launches += 2;
+    if (count) ctx->launches++;
     return B2D_OK;
 }
 
@@ -1320,8 +1392,10 @@ static b2d_status enqueue_advance(b2d_ctx* ctx, int fold, int start, int* final_
         if (count) ctx->launches++;
         st = launch_tracers(ctx, plan[s], count);
         if (st != B2D_OK) return st;
+        st = launch_fold(ctx, (int)s, (int)plan.size(), count);
+        if (st != B2D_OK) return st;
     }
-    return launch_elements(ctx, fold, start, (int)plan.size(), count);
+    return launch_ledgers(ctx, fold, start, count);
 }
 
 extern "C" b2d_status b2d_set_tracers(b2d_ctx* ctx, int32_t run, int64_t n, const double* xy)
@@ -1583,7 +1657,8 @@ extern "C" int64_t b2d_launches_per_advance(const b2d_ctx* ctx, int32_t fold)
     if (!ctx) return 0;
     int with_tracers = 0;
     for (const RunDev& d : ctx->rdev_h) with_tracers += d.ntracers > 0 ? 1 : 0;
-    return 3 + (int64_t)fold * ctx->rk * (1 + with_tracers);
+    const int64_t stages = (int64_t)fold * ctx->rk, window = std::min<int64_t>(ctx->stage_window, stages);
+    return 2 + (stages + window - 1) / window + stages * (1 + with_tracers);
 }
 
 extern "C" b2d_status b2d_set_instrument(b2d_ctx* ctx, int32_t enable)
@@ -1841,6 +1916,8 @@ extern "C" b2d_status b2d_slab_stage(b2d_ctx* ctx)
     ctx->launches++;
     st = launch_tracers(ctx, ctx->slab_plan[s], true);
     if (st != B2D_OK) return st;
+    st = launch_fold(ctx, s, (int)ctx->slab_plan.size(), true);
+    if (st != B2D_OK) return st;
     ctx->slab_next++;
     return B2D_OK;
 }
@@ -1849,7 +1926,7 @@ extern "C" b2d_status b2d_slab_end(b2d_ctx* ctx, double* dt_out, b2d_error* err_
 {
     if (!ctx || ctx->slab_next != (int)ctx->slab_plan.size() || ctx->slab_plan.empty())
         return fail(B2D_ERR_INVALID, "the slab advance has stages left to run");
-    b2d_status st = launch_elements(ctx, ctx->slab_fold, ctx->slab_start, (int)ctx->slab_plan.size(), true);
+    b2d_status st = launch_ledgers(ctx, ctx->slab_fold, ctx->slab_start, true);
     ctx->slab_next = -1;
     if (st != B2D_OK) return st;
     return finish_advance(ctx, ctx->slab_final, dt_out, err_out);
@@ -1934,6 +2011,25 @@ __global__ void noalloc_setup_kernel(RunDev* rd, double time, double dt)
     }
 }
 
+// The stage's ledger: pieces folded, added and averaged as compute_block_updated_solution
+// and weighted_average do (scheme.rs:307-313, state.rs:196).
+__global__ void noalloc_ledger_kernel(const RunDev* run, int base_slot, double bf)
+{
+    const RunDev& rd = *run;
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;   // block * 7 + item
+    if (id >= rd.nblocks * NITEMS) return;
+    const int nf = rd.p.hydro == B2D_EULER ? 4 : 3;
+    double ds[4];
+    if (nf == 3) fold_item<3>(rd, 0, id / NITEMS, id % NITEMS, ds);
+    else fold_item<4>(rd, 0, id / NITEMS, id % NITEMS, ds);
+    for (int f = 0; f < nf; ++f) {
+        const size_t w = (size_t)id * nf + f;
+        double v = rd.ledger[0][w] + ds[f];
+        if (base_slot >= 0) v = v * (-bf + 1.0) + rd.ledger[base_slot][w] * bf;
+        rd.ledger[2][w] = v;
+    }
+}
+
 extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_in, const double* d_background,
                                         const double* d_base, double* d_out, const double* d_ledger_in,
                                         const double* d_ledger_base, double* d_ledger_out, double time, double dt,
@@ -1986,7 +2082,6 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     long long* iters = (long long*)(orbit + 16);           // 4 (unused by the stage)
     unsigned long long* amax = (unsigned long long*)(orbit + 20);
     unsigned long long* err_key = amax + 1;
-    unsigned* counter = (unsigned*)(base + off_cnt);
     double* partial = (double*)(base + off_part);
 
     std::vector<double> xc(N), xv((size_t)nb * (bs + 1));
@@ -2011,7 +2106,7 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     rd.ledger[0] = (double*)d_ledger_in; rd.ledger[1] = (double*)d_ledger_base;
     rd.ledger[2] = d_ledger_out; rd.ledger[3] = d_ledger_out;
     rd.time = times; rd.iter = iters;
-    rd.partial = partial; rd.counter = counter;
+    rd.partial = partial; rd.stage_window = 1;
     rd.dt = d_dt; rd.stage_time = stime; rd.orbit = orbit; rd.amax = amax;
     rd.binary_q = cfg->binary_mass_ratio; rd.binary_e = cfg->binary_eccentricity;
     rd.p = make_params<double>(*cfg);
@@ -2021,7 +2116,6 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     CUDA_TRY(cudaMemcpyAsync(d_run, &rd, sizeof rd, cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_xc, xc.data(), sizeof(double) * xc.size(), cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_xv, xv.data(), sizeof(double) * xv.size(), cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemsetAsync(counter, 0, sizeof(unsigned) * nblocks, stream));
     CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(unsigned long long), stream));
     CUDA_TRY(cudaMemsetAsync(err_key, 0xff, sizeof(unsigned long long), stream));
     noalloc_setup_kernel<<<1, 32, 0, stream>>>(d_run, time, dt);
@@ -2029,7 +2123,9 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
 
     StageArgs a;
     a.runs = d_run;
+    a.tile_bases = nullptr;
     a.nruns = 1;
+    a.pf1 = rd.pf;
     a.th = sub_h;
     a.in_slot = 0;
     a.base_slot = d_base ? 1 : -1;
@@ -2043,6 +2139,8 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     a.err_key = err_key;
     cudaError_t e = launch_stage_f64(nf, a, rd.ntiles, stage_f64_smem(nf, sub_h, sub_w), stream);
     if (e != cudaSuccess) return fail(B2D_ERR_CUDA, std::string("stage kernel launch: ") + cudaGetErrorString(e));
+    noalloc_ledger_kernel<<<(nblocks * NITEMS + 127) / 128, 128, 0, stream>>>(d_run, a.base_slot, a.bf);
+    CUDA_TRY(cudaGetLastError());
     if (d_max_speed) CUDA_TRY(cudaMemcpyAsync(d_max_speed, amax, sizeof(double), cudaMemcpyDeviceToDevice, stream));
 
     unsigned long long key = ~0ull;

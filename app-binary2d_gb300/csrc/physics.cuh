@@ -1,5 +1,5 @@
 // physics.cuh — physics parameters in device form, and the per-zone formulas
-// that several kernels share, templated on the stencil arithmetic R.
+// that several kernels share.
 //
 // R = double: the parity path.  Every expression is evaluated in the order
 // of the reference's Rust source (this translation unit is compiled with
@@ -52,39 +52,41 @@ using DevParamsF = DevParamsT<float>;
 template <class R> struct PointMass { R m, x, y, vx, vy; };
 template <class R> struct Binary { PointMass<R> p1, p2; };
 
-template <class R> __device__ __forceinline__ R rmax(R a, R b) { return fmax(a, b); }
-template <> __device__ __forceinline__ float rmax<float>(float a, float b) { return fmaxf(a, b); }
-template <class R> __device__ __forceinline__ R rabs(R a) { return fabs(a); }
-template <> __device__ __forceinline__ float rabs<float>(float a) { return fabsf(a); }
-template <class R> __device__ __forceinline__ R rsqrt_(R a) { return sqrt(a); }
-template <> __device__ __forceinline__ float rsqrt_<float>(float a) { return sqrtf(a); }
-
 // ---------------------------------------------------------------------------
-// Conserved -> primitive (hydro-iso2d / hydro-euler, restated).
-template <int NF, class R> __device__ __forceinline__ void cons_to_prim_raw(const DevParamsT<R>& P, const R* u, R* p)
+// Hydrodynamics::max_signal_speed (physics.rs:521-526, 679-681).
+template <int NF> __device__ __forceinline__ double max_speed_f64(const DevParams& P, const double* u)
 {
-    p[0] = u[0];
-    if constexpr (std::is_same<R, double>::value) {
-        p[1] = u[1] / u[0];
-        p[2] = u[2] / u[0];
-        if constexpr (NF == 4) p[3] = (u[3] - 0.5 * u[0] * (p[1] * p[1] + p[2] * p[2])) * P.gm1;
-    } else {
-        float ir = __fdividef(1.0f, u[0]);
-        p[1] = u[1] * ir;
-        p[2] = u[2] * ir;
-        if constexpr (NF == 4) p[3] = (u[3] - 0.5f * u[0] * (p[1] * p[1] + p[2] * p[2])) * P.gm1;
+    const double vx = u[1] / u[0], vy = u[2] / u[0];
+    const double v = fmax(fabs(vx), fabs(vy));
+    if constexpr (NF == 4) {
+        const double p = (u[3] - 0.5 * u[0] * (vx * vx + vy * vy)) * P.gm1;
+        return v + sqrt(P.gamma * p / u[0]);
     }
+    return v;
 }
 
-// Hydrodynamics::max_signal_speed (physics.rs:521-526 iso; 679-681 euler).
-template <int NF, class R> __device__ __forceinline__ R max_signal_speed(const DevParamsT<R>& P, const R* u)
+// The same in FP32, from a zone's words as double-floats hi + lo, every
+// rounding written out: the kernels that call it are compiled with different
+// flags and have to agree.  At Mach 30 the internal energy is 1/400 of the
+// total: as a difference of FP32 words it is off by 2.5e-5, so it is formed
+// from both words and the kinetic energy's remainders.
+template <int NF> __device__ __forceinline__ float max_speed_f32(const DevParamsF& P, const float* hi, const float* lo)
 {
-    R p[NF];
-    cons_to_prim_raw<NF, R>(P, u, p);
-    R v = rmax(rabs(p[1]), rabs(p[2]));
+    const float v = fmaxf(fabsf(__fdiv_rn(hi[1], hi[0])), fabsf(__fdiv_rn(hi[2], hi[0])));
     if constexpr (NF == 4) {
-        R cs = rsqrt_(R(P.gamma) * p[3] / p[0]);
-        return v + cs;
+        // m^2 = a + b, a rounded
+        const float a1 = __fmul_rn(hi[1], hi[1]), a2 = __fmul_rn(hi[2], hi[2]);
+        const float b1 = __fmaf_rn(__fmul_rn(2.0f, hi[1]), lo[1], __fmaf_rn(hi[1], hi[1], -a1));
+        const float b2 = __fmaf_rn(__fmul_rn(2.0f, hi[2]), lo[2], __fmaf_rn(hi[2], hi[2], -a2));
+        const float big = fmaxf(a1, a2), small = fminf(a1, a2);
+        const float a = __fadd_rn(big, small);
+        const float b = __fadd_rn(__fadd_rn(small, -__fadd_rn(a, -big)), __fadd_rn(b1, b2));
+        // k + r = (a + b) / (2 rho)
+        const float ir = __frcp_rn(hi[0]), ha = __fmul_rn(0.5f, a);
+        const float k = __fmul_rn(ha, ir);
+        const float r = __fmul_rn(__fmaf_rn(-k, lo[0], __fmaf_rn(0.5f, b, __fmaf_rn(-k, hi[0], ha))), ir);
+        const float e = __fadd_rn(__fadd_rn(hi[3], -k), __fadd_rn(lo[3], -r));
+        return __fadd_rn(v, __fsqrt_rn(__fmul_rn(__fmul_rn(P.gamma, __fmul_rn(e, P.gm1)), ir)));
     }
     return v;
 }

@@ -1,6 +1,8 @@
 // runtime.cuh — device-side descriptors shared by the kernels and the C ABI.
 #pragma once
 
+#include <vector_types.h>
+
 #include "../../include/b2d.h"
 #include "physics.cuh"
 
@@ -26,15 +28,15 @@ struct RunDev {
     const double* buffer;    // FP64 kernel: [N][N] buffer rate (nullptr: computed where it is used)
     const double* xc;        // [N] cell centres by global index (block formula, mesh.rs:49-54)
     const double* xv;        // [nb][bs+1] block vertices (mesh.rs:42-47)
-    const float* xcf;        // FP32 centres; like xvgf, 4 entries longer than the mesh at either end
-    const float* xvgf;       // [N+1] row faces by global index, FP32 (a block's first vertex at its lower boundary)
+    const float2* xcf;       // [N] the centres as FP32 high and low words
+    const float2* xvf;       // [N+1] faces by global index (a block's first vertex at its lower boundary), likewise
     void* slot[NSLOTS];      // conserved state per slot (STORE layout)
     const void* bg;          // BlockData::initial_conserved (STORE layout)
     double* ledger[NSLOTS];  // [nblocks][7][nf] per slot
     double* time;            // [NSLOTS]
     long long* iter;         // [NSLOTS]
-    double* partial;         // [nblocks][tiles_per_block][7 nf] ledger pieces of the tiles over each block
-    unsigned* counter;       // [nblocks]
+    double* partial;         // [stage_window][nblocks][tiles_per_block][7 nf] ledger pieces of the tiles over each block
+    int stage_window;        // stages whose pieces are kept before they are folded
     double* dt;              // [1]
     double* stage_time;      // [max_stages]
     double* orbit;           // [max_stages][10]: m, x, y, vx, vy of body 1 then body 2
@@ -52,6 +54,7 @@ struct RunDev {
 
 struct StageArgs {
     const RunDev* runs;
+    const int* tile_bases;   // [nruns] first CTA of each run
     int nruns;
     int th;
     int in_slot, base_slot, out_slot;
@@ -60,8 +63,8 @@ struct StageArgs {
     double bf;               // weight of the RK base state (br of godunov-core)
     int half_avg;            // bf is 1/2
     b2d::df32w w1f, bff;     // 1 - bf and bf as double-float
-    DevParamsF pf1;          // FP32 parameters of a single-run context, read as kernel arguments
     unsigned long long* err_key;  // failure key, ~0 when no zone failed
+    DevParamsF pf1;          // FP32 parameters of a single-run context, read as kernel arguments
 };
 
 // Row chunks of a column strip.  A run's N rows split into C chunks; chunk c
@@ -82,8 +85,23 @@ __host__ __device__ inline int chunks_in_block_row(int b, int bs, int N, int C)
     return chunk_of_row((b + 1) * bs - 1, N, C) - chunk_of_row(b * bs, N, C) + 1;
 }
 
-template <class R> __host__ __device__ inline const DevParamsT<R>& params_of(const RunDev& rd);
-template <> __host__ __device__ inline const DevParamsT<double>& params_of<double>(const RunDev& rd) { return rd.p; }
-template <> __host__ __device__ inline const DevParamsT<float>& params_of<float>(const RunDev& rd) { return rd.pf; }
+// The ledger pieces of a block in a stage.
+__host__ __device__ inline double* stage_pieces(const RunDev& rd, int stage, int block, int words)
+{
+    return rd.partial + ((size_t)(stage % rd.stage_window) * rd.nblocks + block) * rd.tiles_per_block * words;
+}
+
+#ifdef __CUDACC__
+// The run that CTA g belongs to: the last one whose first CTA is not beyond it
+// (256 runs at most; the whole warp searches, so that a batch of many runs
+// costs one load's latency).
+__device__ __forceinline__ int find_run(const StageArgs& a, int g)
+{
+    int n = 0;
+    for (int k = threadIdx.x & 31; k - (int)(threadIdx.x & 31) < a.nruns; k += 32)
+        n += __popc(__ballot_sync(0xffffffffu, k < a.nruns && a.tile_bases[min(k, a.nruns - 1)] <= g));
+    return n - 1;
+}
+#endif
 
 }  // namespace b2d

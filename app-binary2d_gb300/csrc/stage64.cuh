@@ -4,7 +4,7 @@
 // every run of a context: cons→prim (try_block_primitive, scheme.rs:185-199),
 // PLM slopes and HLLE + viscous fluxes (scheme.rs:216-268), flux divergence +
 // sources + RK average (scheme.rs:290-305, state.rs:183-199), the per-block
-// source ledger (scheme.rs:288-313) and, on the last stage of an advance, the
+// source ledger's pieces (scheme.rs:288-313) and, on the last stage of an advance, the
 // max signal speed of the next dt (state.rs:121-133).
 //
 // What bounds it.  GB300 executes two FP64 lanes per clock and SM: one FP64
@@ -197,7 +197,8 @@ __device__ __forceinline__ void side64(const double* p, double pg, const Divisor
 }
 
 // ---------------------------------------------------------------------------
-template <int NF> __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(StageArgs a)
+template <int NF>
+__global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_constant__ StageArgs a)
 {
     constexpr int NL = NITEMS * NF;
     constexpr int NREC = 2 * NF + 4;   // slopes along x and y, then T or the shear: xx, yy, xy, bulk
@@ -206,24 +207,22 @@ template <int NF> __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kern
     constexpr int NT = S64_THREADS, NW = NT / 32;
 
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    int ri = 0;
     const int g = blockIdx.x;
-    while (ri + 1 < a.nruns && g >= a.runs[ri + 1].tile_base) ++ri;
+    const int ri = a.nruns == 1 ? 0 : find_run(a, g);
     const RunDev& rd = a.runs[ri];
-    if (g - rd.tile_base >= rd.ntiles) return;
 
     __shared__ DevParams P;
     __shared__ double orb[10];
-    __shared__ int failed, is_last;
+    __shared__ int failed;
     __shared__ double led[NW][NL];
     __shared__ double wmax[NW];
+    for (int i = t; i < NW * NL; i += NT) led[i / NL][i % NL] = 0.0;
+    if (t == 0) P = rd.p;
     // an earlier stage failed: the advance is abandoned (the caller keeps its state)
     if (t == 0) failed = (*(volatile unsigned long long*)a.err_key != ~0ull);
     __syncthreads();
     if (failed) return;
-    if (t == 0) P = rd.p;
     if (t < 10) orb[t] = rd.orbit[a.stage * 10 + t];
-    for (int i = t; i < NW * NL; i += NT) led[i / NL][i % NL] = 0.0;
     extern __shared__ __align__(128) unsigned char smem_raw[];   // one declaration for every stage kernel
     poison_dynamic_smem(smem_raw);
     __syncthreads();
@@ -744,36 +743,14 @@ template <int NF> __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kern
     if (t < NL) {
         double v = 0.0;
         for (int w = 0; w < NW; ++w) v += led[w][t];
-        rd.partial[((size_t)block * rd.tiles_per_block + piece) * NL + t] = v;
-        __threadfence();   // visible before the counter below counts this piece
+        // folded, in piece order, after the stages (b2d_advance's ledger kernels)
+        stage_pieces(rd, a.stage, block, NL)[(size_t)piece * NL + t] = v;
     }
     if (a.amax_flag && t == 0) {
         double m = 0.0;
         for (int w = 0; w < NW; ++w) m = fmax(m, wmax[w]);
         if (m > 0.0) atomicMax(rd.amax, (unsigned long long)__double_as_longlong(m));
     }
-    __syncthreads();
-
-    // The last CTA of a block to finish folds the pieces into the block's
-    // ledger: integrated_source_terms + ds·dx·dy (scheme.rs:307-313), averaged
-    // like the conserved state (state.rs:196).
-    if (t == 0) is_last = atomicAdd(rd.counter + block, 1u) == (unsigned)rd.tiles_per_block - 1;
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    if (t < NL) {
-        const double area = P.dx * P.dx;
-        double v = 0.0;
-        for (int q = 0; q < rd.tiles_per_block; ++q)
-            v += __ldcg(rd.partial + ((size_t)block * rd.tiles_per_block + q) * NL + t);
-        const double ds = v * area;
-        v = __ldcg(rd.ledger[a.in_slot] + (size_t)block * NL + t) + ds;
-        if (a.base_slot >= 0) v = v * keep + __ldcg(rd.ledger[a.base_slot] + (size_t)block * NL + t) * a.bf;
-        rd.ledger[a.out_slot][(size_t)block * NL + t] = v;
-        // the block's ds·dx·dy of this stage, for the orbital-element ledger
-        if (rd.stage_ds) rd.stage_ds[((size_t)a.stage * rd.nblocks + block) * NL + t] = ds;
-    }
-    if (t == 0) rd.counter[block] = 0u;
 }
 
 }  // namespace b2d

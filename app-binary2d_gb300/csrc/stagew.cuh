@@ -5,7 +5,7 @@
 // every run of a context, on the FP64 state or on the compensated FP32 state:
 // cons→prim (scheme.rs:185-199), PLM slopes and HLLE + viscous fluxes
 // (scheme.rs:216-268), flux divergence + sources + RK average
-// (scheme.rs:290-305, state.rs:183-199), the per-block source ledger
+// (scheme.rs:290-305, state.rs:183-199), the per-block source ledger's pieces
 // (scheme.rs:288-313) and, on the last stage of an advance, the max signal
 // speed of the next dt (state.rs:121-133).
 //
@@ -34,17 +34,22 @@
 //    g = n - 1, its upper x faces and its y faces, and updates row g - 1.
 //  * Ledger.  The items that are live everywhere are summed per column in
 //    registers; a block's part is reduced over the warp at the last row of
-//    each block row and at the chunk's end, one piece per strip and chunk,
-//    and the last piece of a block folds them in order.
+//    each block row and at the chunk's end, one piece per strip and chunk.  The
+//    pieces of all stages are folded, in order, after the last of them: a fence,
+//    a counter and a fold in the stage's tail cost it about 5 us.
 //
-// What bounds it: instruction issue (681 warp instructions per row of 60
-// columns and isothermal first stage, about 390 of them arithmetic; issue 52 %
-// busy at 12 warps per SM), not memory (about 2.7 of 6.7 TB/s).  Measured per
-// stage against the kernels it took the place of: isothermal 2048^2 0.127 ->
-// 0.109 ms (a CTA of 10 warps marching in step over 512 columns), 384^2 33 -> 22
-// us, the 64-run sweep 1.05 -> 0.69 ms, Euler 4096^2 0.65 -> 0.55 ms, 768^2 48
-// -> 42 us, blocks of 50^2 (RK3, alpha viscosity) 163 -> 25 us (one thread per
-// column of a block), FP64 state 1024^2 106 -> 94 us.
+// What bounds it: instruction issue (about 660 warp instructions per row of
+// 60 columns and isothermal first stage, 390 of them arithmetic; issue 59 %
+// busy at 12 warps per SM), not memory (3.4 of 6.7 TB/s).  Measured per stage, as
+// this file began and now, against the kernels that it took the place of:
+// isothermal 2048^2 0.127 -> 0.109 -> 0.084 ms (a CTA of 10 warps marching in
+// step over 512 columns), 384^2 33 -> 22 -> 14.8 us, the 64-run sweep 1.05 ->
+// 0.69 -> 0.57 ms, Euler 4096^2 0.65 -> 0.55 -> 0.49 ms, 768^2 48 -> 42 -> 34 us,
+// blocks of 50^2 (RK3, alpha viscosity) 163 -> 25 -> 14.5 us (one thread per
+// column of a block), FP64 state 1024^2 106 -> 94 -> 82 us.  Tried and slower:
+// the row loop unrolled twice (104 against 98 us at 2048^2: spills), the run's
+// descriptor as a kernel argument (99 against 92), programmatic dependent
+// launch (768^2: 47 against 40 us).
 #pragma once
 
 #include "stage.cuh"
@@ -60,17 +65,24 @@ constexpr int SW_USLOTS = 2;             // update rows: one in use, one ahead
 template <int NF, int STORE> struct SWShape {
     using E = typename std::conditional<STORE == 1, float, double>::type;
     static constexpr int NU = (STORE == 1 ? 4 : 2) * NF;  // update planes: (lo,) bg, base hi (, base lo)
-    static constexpr int ITEMS = NF == 3 ? 16 : 19;       // ledger rows: everywhere, sinks, fake mass
+    static constexpr int ITEMS = NF == 3 ? 16 : 19;       // ledger items: live everywhere, sinks, fake mass
     static constexpr int SINKS_AT = NF == 3 ? 7 : 11, FAKE_AT = 13;
     static constexpr int STENCIL = NF * 64;               // elements of a staged row
     static constexpr int UPDATE = NU * 64;
-    static constexpr int BYTES = (SW_SLOTS * STENCIL + SW_USLOTS * UPDATE) * (int)sizeof(E) + ITEMS * 64 * 4;
+    static constexpr int BYTES = (SW_SLOTS * STENCIL + SW_USLOTS * UPDATE) * (int)sizeof(E) + (ITEMS - SINKS_AT) * 64 * 4;
+    static_assert(SINKS_AT * 64 * 4 <= UPDATE * (int)sizeof(E), "a consumed update row takes the other items' sums");
 };
 
-// Constants as pairs.
+// Constants as pairs, with what can be folded into them: the limiter works on
+// twice the slopes, the stress on (slope / dx) times c, the sound speed on
+// masses over Mach^2, the buffer on powers of two.
 enum {
-    C_THETA, C_HALF, C_NHALF, C_INV_DX, C_LAMBDA, C_NU, C_INV_MACH2, C_M1, C_M2, C_NM1DT, C_NM2DT, C_Y1, C_Y2, C_SOFT2,
-    C_RADIUS, C_BUF_SLOPE, C_BUF_RATE, C_NDT_DX, C_43, C_N23, C_GAMMA, C_GM1, C_INV_GM1, C_COOL, C_ALPHA, C_ONE, C_COUNT
+    C_THETA2,                // 2 theta
+    C_QUARTER, C_NQUARTER, C_HALF, C_ONE,
+    C_TN, C_TT, C_VISC,      // 4/3 + lambda, -2/3 + lambda; c / (2 dx) of the cell's stress
+    C_CM1, C_CM2,            // m / Mach^2
+    C_M1, C_M2, C_NM1DT, C_NM2DT, C_SOFT2,
+    C_BUF_SLOPE, C_BUF_OFFSET, C_BUF_RATE, C_NDT_DX, C_GAMMA, C_GM1, C_INV_GM1, C_COOL, C_ALPHA, C_COUNT
 };
 
 // ---------------------------------------------------------------------------
@@ -136,16 +148,22 @@ __device__ __forceinline__ float max3f(float a, float b, float c)
     return d;
 }
 
-// Generalised minmod of each lane (godunov-core's plm_gradient, restated) as the median of
-// min(x, y, z), max(x, y, z) and 0: the minimum when all three are positive,
-// the maximum when all are negative, else 0 — min(max(lo, 0), hi) for lo <= hi.
+// Twice the generalised minmod of each lane (godunov-core's plm_gradient,
+// restated), th = 2 theta: the median of min(x, y, z), max(x, y, z) and 0 — the
+// minimum when all three are positive, the maximum when all are negative, else
+// 0: min(max(lo, 0), hi) for lo <= hi.
 __device__ __forceinline__ float2 plm_gradient2(float2 th, float2 a, float2 b, float2 c)
 {
-    const float2 x = mul2(th, sub2(b, a));
-    const float2 y = mul2(f2(0.5f), sub2(c, a));
-    const float2 z = mul2(th, sub2(c, b));
+    const float2 x = mul2(th, sub2(b, a)), y = sub2(c, a), z = mul2(th, sub2(c, b));
     return make_float2(fminf(fmaxf(min3f(x.x, y.x, z.x), 0.0f), max3f(x.x, y.x, z.x)),
                        fminf(fmaxf(min3f(x.y, y.y, z.y), 0.0f), max3f(x.y, y.y, z.y)));
+}
+
+__device__ __forceinline__ float exp2_fast(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
 }
 
 // e^x - 1 of two small arguments (|x| <= 0.35): the Taylor series
@@ -183,16 +201,6 @@ template <int NF> __device__ __forceinline__ void prim_exact(const DevParamsF& P
     }
 }
 
-// Hydrodynamics::max_signal_speed (physics.rs:521-526, 679-681).
-template <int NF> __device__ __forceinline__ float max_speed_exact(const DevParamsF& P, const float* u)
-{
-    float p[NF];
-    prim_exact<NF>(P, u, p);
-    const float v = fmaxf(fabsf(p[1]), fabsf(p[2]));
-    if constexpr (NF == 4) return __fadd_rn(v, sqrtf(__fmul_rn(__fmul_rn(P.gamma, p[3]), __fdividef(1.0f, p[0]))));
-    return v;
-}
-
 // Physics::sink_kernel (physics.rs:388-397): rate (1 - r^2 / s^2)^2 inside the sink radius s.
 __device__ __forceinline__ float sink_rate_exact(const DevParamsF& P, float dx, float dy)
 {
@@ -206,11 +214,10 @@ __device__ __forceinline__ float sink_rate_exact(const DevParamsF& P, float dx, 
 
 // The torque-free sink velocity: the gas velocity relative to the body,
 // projected on the radial direction, plus the body's velocity (physics.rs:743-756).
-__device__ __forceinline__ void torque_free_exact(const DevParamsF& P, const PointMass<float>& b, float x, float y,
+__device__ __forceinline__ void torque_free_exact(const DevParamsF& P, const PointMass<float>& b, float ddx, float ddy,
                                                   float vx, float vy, float& vxc, float& vyc)
 {
     const float vxb = P.one_body ? 0.0f : b.vx, vyb = P.one_body ? 0.0f : b.vy;
-    const float ddx = x - b.x, ddy = y - b.y;
     const float r = sqrtf(fmaf(ddx, ddx, __fmul_rn(ddy, ddy)));
     const float rx = __fdividef(ddx, r), ry = __fdividef(ddy, r);
     const float dvdotr = fmaf(vx - vxb, rx, __fmul_rn(vy - vyb, ry));
@@ -220,13 +227,13 @@ __device__ __forceinline__ void torque_free_exact(const DevParamsF& P, const Poi
 
 // The sink items of one zone (the sink part of source_terms, physics.rs:
 // 528-582, 683-774): -rate u dt (impartial sinks) or -rate dt times the
-// torque-free state.
+// torque-free state, at (dx1, dy1) from body 1 and (dx2, dy2) from body 2.
 template <int NF>
-__device__ __noinline__ void sink_items_exact(const DevParamsF& P, const Binary<float>& B, const float* u, float x,
-                                              float y, float dt, float* s1, float* s2)
+__device__ __noinline__ void sink_items_exact(const DevParamsF& P, const Binary<float>& B, const float* u, float dx1,
+                                              float dy1, float dx2, float dy2, float dt, float* s1, float* s2)
 {
-    const float sr1 = __fmul_rn(sink_rate_exact(P, x - B.p1.x, y - B.p1.y), -dt);
-    const float sr2 = __fmul_rn(sink_rate_exact(P, x - B.p2.x, y - B.p2.y), -dt);
+    const float sr1 = __fmul_rn(sink_rate_exact(P, dx1, dy1), -dt);
+    const float sr2 = __fmul_rn(sink_rate_exact(P, dx2, dy2), -dt);
     if (P.sink_model == 0) {
 #pragma unroll
         for (int k = 0; k < NF; ++k) {
@@ -238,8 +245,8 @@ __device__ __noinline__ void sink_items_exact(const DevParamsF& P, const Binary<
     float p[NF];
     prim_exact<NF>(P, u, p);
     float v1x, v1y, v2x, v2y;
-    torque_free_exact(P, B.p1, x, y, p[1], p[2], v1x, v1y);
-    torque_free_exact(P, B.p2, x, y, p[1], p[2], v2x, v2y);
+    torque_free_exact(P, B.p1, dx1, dy1, p[1], p[2], v1x, v1y);
+    torque_free_exact(P, B.p2, dx2, dy2, p[1], p[2], v2x, v2y);
     const float sd = p[0];
     float a1[NF], a2[NF];
     a1[0] = a2[0] = sd;
@@ -272,16 +279,13 @@ __device__ __noinline__ void sink_items_exact(const DevParamsF& P, const Binary<
 // gamma p / rho (Euler alpha), and a face needs tau = K (T_l + T_r) / 2 with
 // K = 1 for the constant model.
 
-// 0.5 K of the alpha model at two faces (x, fy.x) and (x, fy.y), an isothermal
-// face's cs2 left out.  1 / a^3 is taken as rsqrt(a^2)^3: the reference's
+// 0.5 K of the alpha model at two faces at these distances from the bodies, an
+// isothermal face's cs2 left out.  1 / a^3 is taken as rsqrt(a^2)^3: the reference's
 // a = |d| + 1e-12 dx (scheme.rs:244) differs from |d| below FP32 resolution
 // unless |d| is under about 1e-7 dx, and at |d| = 0 both give K = 0.
-__device__ __forceinline__ float2 alpha_half_k2(const float2* K, const Binary<float>& B, float x, float2 fy)
+__device__ __forceinline__ float2 alpha_half_k2(const float2* K, float2 dx1, float2 dx2, float2 dy1, float2 dy2)
 {
-    const float dx1 = x - B.p1.x, dx2 = x - B.p2.x;
-    const float2 dy1 = sub2(fy, K[C_Y1]), dy2 = sub2(fy, K[C_Y2]);
-    const float2 d1 = fma2(dy1, dy1, f2(__fmul_rn(dx1, dx1))), d2 = fma2(dy2, dy2, f2(__fmul_rn(dx2, dx2)));
-    const float2 q1 = rsqrt2(d1), q2 = rsqrt2(d2);
+    const float2 q1 = rsqrt2(fma2(dy1, dy1, mul2(dx1, dx1))), q2 = rsqrt2(fma2(dy2, dy2, mul2(dx2, dx2)));
     const float2 w2 = fma2(K[C_M1], mul2(q1, mul2(q1, q1)), mul2(K[C_M2], mul2(q2, mul2(q2, q2))));
     return mul2(K[C_ALPHA], rsqrt2(w2));
 }
@@ -311,8 +315,8 @@ __device__ __forceinline__ void faces2(const float2* K, const float2* pl, const 
         pgr = pr[3];
         csl = sqrt2(mul2(mul2(K[C_GAMMA], pl[3]), rcp2(pl[0])));
         csr = sqrt2(mul2(mul2(K[C_GAMMA], pr[3]), rcp2(pr[0])));
-        ul[3] = fma2(mul2(K[C_HALF], pl[0]), fma2(pl[1], pl[1], mul2(pl[2], pl[2])), mul2(pl[3], K[C_INV_GM1]));
-        ur[3] = fma2(mul2(K[C_HALF], pr[0]), fma2(pr[1], pr[1], mul2(pr[2], pr[2])), mul2(pr[3], K[C_INV_GM1]));
+        ul[3] = fma2(K[C_HALF], fma2(ul[1], pl[1], mul2(ul[2], pl[2])), mul2(pl[3], K[C_INV_GM1]));
+        ur[3] = fma2(K[C_HALF], fma2(ur[1], pr[1], mul2(ur[2], pr[2])), mul2(pr[3], K[C_INV_GM1]));
         fl[3] = mul2(add2(ul[3], pl[3]), vl);
         fr[3] = mul2(add2(ur[3], pr[3]), vr);
     }
@@ -327,12 +331,10 @@ __device__ __forceinline__ void faces2(const float2* K, const float2* pl, const 
     const float2 ap = make_float2(max3f(alp.x, arp.x, 0.0f), max3f(alp.y, arp.y, 0.0f));
     const float2 am = make_float2(min3f(alm.x, arm.x, 0.0f), min3f(alm.y, arm.y, 0.0f));
     const float2 inv = rcp2(sub2(ap, am));
-    const float2 nam = mul2(am, f2(-1.0f));
-    const float2 apam = mul2(ap, am);
-    // F = (fl ap - fr am - (ul - ur) ap am) / (ap - am)
+    // F = (fl ap - fr am + (ur - ul) ap am) / (ap - am), with wl + wr = 1
+    const float2 wl = mul2(ap, inv), wr = sub2(K[C_ONE], wl), wd = mul2(am, wl);
 #pragma unroll
-    for (int f = 0; f < NF; ++f)
-        F[f] = mul2(fma2(sub2(ur[f], ul[f]), apam, fma2(fr[f], nam, mul2(fl[f], ap))), inv);
+    for (int f = 0; f < NF; ++f) F[f] = fma2(sub2(ur[f], ul[f]), wd, fma2(fr[f], wr, mul2(fl[f], wl)));
     const float2 tau_n = mul2(k, tn), tau_t = mul2(k, tt);
     const float2 tx = AXIS == 0 ? tau_n : tau_t, ty = AXIS == 0 ? tau_t : tau_n;
     F[1] = sub2(F[1], tx);
@@ -386,13 +388,12 @@ template <int NF> __device__ __forceinline__ int ledger_word(int m)
 }
 
 // A strip's ledger pieces of block row `brow`, by its warp: for every block
-// under the strip the sums over the columns inside it, the piece's slot in
-// the block's partials, and the fold of the block's pieces (in piece order)
-// by the block's last piece.  Out of line, so that it does not weigh on the
-// row loop's register allocation.
+// under the strip the sums over the columns inside it, in the piece's slot of
+// the block's.  Out of line, so that it does not weigh on the row loop's
+// register allocation.
 template <int NF, int STORE>
-__device__ __noinline__ void flush_strip(const RunDev& rd, int strip, int ti, int brow, const float* led, bool sinks,
-                                         bool fake, int in_slot, int base_slot, int out_slot, int stage, double bf)
+__device__ __noinline__ void flush_strip(const RunDev& rd, int stage, int strip, int ti, int brow, const float* sums,
+                                         const float* led, bool sinks, bool fake)
 {
     using T = SWShape<NF, STORE>;
     constexpr int NL = NITEMS * NF, K = NF == 3 ? 16 : 32;
@@ -409,39 +410,15 @@ __device__ __noinline__ void flush_strip(const RunDev& rd, int strip, int ti, in
             const bool on = m < T::SINKS_AT || (m < (NF == 3 ? T::FAKE_AT : T::ITEMS) ? sinks : m < T::ITEMS && fake);
             v[m] = 0.0f;
             if (on) {
-                const float2 q = *(const float2*)(led + m * 64 + 2 * lane);
+                const float2 q = *(const float2*)((m < T::SINKS_AT ? sums + m * 64 : led + (m - T::SINKS_AT) * 64) + 2 * lane);
                 v[m] = (inx ? q.x : 0.0f) + (iny ? q.y : 0.0f);
             }
         }
         const float s = warp_sum_items<K>(v, lane);
         const int m = item_of_lane<K>(lane);
-        const int block = brow * rd.nb + b;
-        const int first_strip = b * bs / SW_COLS, ns = (b * bs + bs - 1) / SW_COLS - first_strip + 1;
-        const int piece = (strip - first_strip) * nc + ti - first_chunk, pieces = ns * nc;
-        double* part = rd.partial + (size_t)block * rd.tiles_per_block * NL;
-        if ((lane & (32 / K - 1)) == 0 && m < T::ITEMS) {
-            part[(size_t)piece * NL + ledger_word<NF>(m)] = (double)s;
-            __threadfence();   // visible before the counter below counts this piece
-        }
-        __syncwarp();
-        unsigned last = 0;
-        if (lane == 0) last = atomicAdd(rd.counter + block, 1u) == (unsigned)pieces - 1;
-        last = __shfl_sync(0xffffffffu, last, 0);
-        if (!last) continue;
-        __threadfence();
-        if (lane < NL) {
-            const double area = (double)rd.p.dx * rd.p.dx;
-            double sum = 0.0;
-#pragma unroll 16
-            for (int q = 0; q < pieces; ++q) sum += __ldcg(part + (size_t)q * NL + lane);
-            double v2 = __ldcg(rd.ledger[in_slot] + (size_t)block * NL + lane) + sum * area;
-            if (base_slot >= 0)
-                v2 = v2 * (-bf + 1.0) + __ldcg(rd.ledger[base_slot] + (size_t)block * NL + lane) * bf;
-            rd.ledger[out_slot][(size_t)block * NL + lane] = v2;
-            // the block's ds·dx·dy of this stage, for the orbital-element ledger
-            if (rd.stage_ds) rd.stage_ds[((size_t)stage * rd.nblocks + block) * NL + lane] = sum * area;
-        }
-        if (lane == 0) rd.counter[block] = 0u;
+        const int piece = (strip - b * bs / SW_COLS) * nc + ti - first_chunk;
+        if ((lane & (32 / K - 1)) == 0 && m < T::ITEMS)
+            stage_pieces(rd, stage, brow * rd.nb + b, NL)[(size_t)piece * NL + ledger_word<NF>(m)] = (double)s;
     }
 }
 
@@ -482,51 +459,54 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
     using E = typename T::E;
     const int lane = threadIdx.x;
 
-    int ri = 0;
     const int g = blockIdx.x;
-    if constexpr (!SINGLE)
-        while (ri + 1 < a.nruns && g >= a.runs[ri + 1].tile_base) ++ri;
+    const int ri = SINGLE ? 0 : find_run(a, g);
     const RunDev& rd = a.runs[ri];
-    if (*(volatile unsigned long long*)a.err_key != ~0ull) return;   // an earlier stage failed: the advance is abandoned
 
     __shared__ DevParamsF Psh;
     const DevParamsF& P = params_for<SINGLE>(a, Psh);
     __shared__ Binary<float> B;
     __shared__ float2 K[C_COUNT];
-    if (lane < 10) ((float*)&B)[lane] = (float)rd.orbit[a.stage * 10 + lane];
     if (!SINGLE && lane == 10) Psh = rd.pf;
     extern __shared__ __align__(128) unsigned char smem_raw[];   // one declaration for every stage kernel
     poison_dynamic_smem(smem_raw);
+    __shared__ float B_lo[10];
+    if (lane < 10) {
+        const double o = rd.orbit[a.stage * 10 + lane];
+        const float hi = (float)o;
+        ((float*)&B)[lane] = hi;
+        B_lo[lane] = (float)(o - (double)hi);
+    }
+    if (*(volatile unsigned long long*)a.err_key != ~0ull) return;   // an earlier stage failed: the advance is abandoned
     __syncwarp();
     const float dt = (float)*rd.dt;
     const float time = (float)rd.stage_time[a.stage];
     if (lane == 0) {
-        K[C_THETA] = f2(P.plm);
+        const float visc = P.visc == 0 ? P.nu : (NF == 3 ? 1.0f : P.gamma), log2e = 1.4426950408889634f;
+        K[C_THETA2] = f2(2.0f * P.plm);
+        K[C_QUARTER] = f2(0.25f);
+        K[C_NQUARTER] = f2(-0.25f);
         K[C_HALF] = f2(0.5f);
-        K[C_NHALF] = f2(-0.5f);
-        K[C_INV_DX] = f2(P.inv_dx);
-        K[C_LAMBDA] = f2(P.lambda);
-        K[C_NU] = f2(P.nu);
-        K[C_INV_MACH2] = f2(P.inv_mach2);
+        K[C_ONE] = f2(1.0f);
+        K[C_TN] = f2(4.0f / 3.0f + P.lambda);
+        K[C_TT] = f2(-2.0f / 3.0f + P.lambda);
+        K[C_VISC] = f2(__fmul_rn(__fmul_rn(0.5f, visc), P.inv_dx));
+        K[C_CM1] = f2(__fmul_rn(B.p1.m, P.inv_mach2));
+        K[C_CM2] = f2(__fmul_rn(B.p2.m, P.inv_mach2));
         K[C_M1] = f2(B.p1.m);
         K[C_M2] = f2(B.p2.m);
         K[C_NM1DT] = f2(__fmul_rn(-B.p1.m, dt));
         K[C_NM2DT] = f2(__fmul_rn(-B.p2.m, dt));
-        K[C_Y1] = f2(B.p1.y);
-        K[C_Y2] = f2(B.p2.y);
         K[C_SOFT2] = f2(P.soft2);
-        K[C_RADIUS] = f2(P.domain_radius);
-        K[C_BUF_SLOPE] = f2(-2.0f * P.inv_buffer_scale);
+        K[C_BUF_SLOPE] = f2(__fmul_rn(-2.0f * P.inv_buffer_scale, log2e));
+        K[C_BUF_OFFSET] = f2(__fmul_rn(__fmul_rn(2.0f * P.inv_buffer_scale, log2e), P.domain_radius));
         K[C_BUF_RATE] = f2(__fmul_rn(-2.0f * dt, P.half_rate_omega));
         K[C_NDT_DX] = f2(__fmul_rn(-P.inv_dx, dt));
-        K[C_43] = f2(4.0f / 3.0f);
-        K[C_N23] = f2(-2.0f / 3.0f);
         K[C_GAMMA] = f2(P.gamma);
         K[C_GM1] = f2(P.gm1);
         K[C_INV_GM1] = f2(P.inv_gm1);
         K[C_COOL] = f2(__fmul_rn(-dt, P.inv_cool_beta));
         K[C_ALPHA] = f2(__fmul_rn(__fmul_rn(0.5f, P.nu), P.inv_sqrt_gm));
-        K[C_ONE] = f2(1.0f);
     }
     __syncwarp();
 
@@ -547,7 +527,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
 
     E* stencil = (E*)smem_raw;                              // [SW_SLOTS][NF][64]: this lane's pair at 2 lane
     E* update = stencil + SW_SLOTS * T::STENCIL;            // [SW_USLOTS][NU][64]
-    float* led = (float*)(update + SW_USLOTS * T::UPDATE);  // [ITEMS][64]
+    float* led = (float*)(update + SW_USLOTS * T::UPDATE);  // [ITEMS - SINKS_AT][64]
     E* my_stencil = stencil + 2 * lane;
     E* my_update = update + 2 * lane;
 
@@ -562,15 +542,20 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
         }
     };
     // row rs of the stencil and row ru of the update, as one group
+    int gi = wrap(wrap(i0 - 2, N), N);                      // mesh row of rs (a mesh may be one zone wide)
+    size_t row_s = (size_t)gi * N, row_u = (size_t)i0 * N;
     auto issue = [&](int rs, int ru) {
         if (rs <= TH + 1) {
-            const size_t row = (size_t)wrap(wrap(i0 + rs, N), N) * N;   // (twice: a mesh may be one zone wide)
+            const size_t row = row_s;
+            row_s += N;
+            if (++gi == N) { gi = 0; row_s = 0; }
             E* d = my_stencil + ((rs + 2) & (SW_SLOTS - 1)) * T::STENCIL;
 #pragma unroll
             for (int f = 0; f < NF; ++f) copy_pair(d + f * 64, uin + (size_t)(PARTS * f) * nn + row);
         }
         if (ru >= 0 && ru < TH) {
-            const size_t row = (size_t)(i0 + ru) * N;
+            const size_t row = row_u;
+            row_u += N;
             E* d = my_update + (ru & 1) * T::UPDATE;
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
@@ -589,46 +574,84 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
     };
     issue(-2, -1);
 
-    const float theta = P.plm, pdt = P.pdt;
+    const float theta2 = 2.0f * P.plm, pdt = P.pdt;
     const df32 w1{a.w1f.hi, a.w1f.lo}, wb{a.bff.hi, a.bff.lo};
     const bool half_avg = a.half_avg != 0;
     const bool want_amax = a.amax_flag != 0, fake_on = NF == 3 && P.fake_rate != 0.0f;
     // the T^4 law's slow-start factor exp(-2 pi / (t + dt)) of this stage (physics.rs:683-774)
     const float slow = NF == 4 && P.cooling_slow_start ? __expf(-6.283185307f / (time + dt)) : 1.0f;
-    // positions: zone centres (y) of the pair, y of the pair's left faces
+    // Distances to the bodies, from positions as double-floats (close to a body the difference of
+    // FP32 positions is off by 1e-6), as tables: per lane along y, in shared memory since registers
+    // are scarce, and per row along x, 31 rows at a time (loads in the row loop would be waited for
+    // in every row).
     auto at = [](int k, int n) { return min(max(k, 0), n); };
-    const float2 yc2 = make_float2(rd.xcf[at(j0 + c0, N - 1)], rd.xcf[at(j0 + c0 + 1, N - 1)]);
-    const float2 yv2 = make_float2(rd.xvgf[at(j0 + c0, N)], rd.xvgf[at(j0 + c0 + 1, N)]);
+    auto from = [](float2 x, float hi, float lo) { return __fadd_rn(__fadd_rn(x.x, -hi), __fadd_rn(x.y, -lo)); };
+    __shared__ float2 dyc1[32], dyc2[32], dyv1[32], dyv2[32], sYc[32];   // of the pair's centres and left faces
+    {
+        const float2 ya = rd.xcf[at(j0 + c0, N - 1)], yb = rd.xcf[at(j0 + c0 + 1, N - 1)];
+        const float2 va = rd.xvf[at(j0 + c0, N)], vb = rd.xvf[at(j0 + c0 + 1, N)];
+        sYc[lane] = make_float2(ya.x, yb.x);
+        dyc1[lane] = make_float2(from(ya, B.p1.y, B_lo[2]), from(yb, B.p1.y, B_lo[2]));
+        dyc2[lane] = make_float2(from(ya, B.p2.y, B_lo[7]), from(yb, B.p2.y, B_lo[7]));
+        dyv1[lane] = make_float2(from(va, B.p1.y, B_lo[2]), from(vb, B.p1.y, B_lo[2]));
+        dyv2[lane] = make_float2(from(va, B.p2.y, B_lo[7]), from(vb, B.p2.y, B_lo[7]));
+    }
+    __shared__ float2 rows[5][32];                          // dx1, dx2 and x^2 of zone rows, dx1, dx2 of the faces above
+    enum { R_C1, R_C2, R_XX, R_F1, R_F2 };
+    auto fill_rows = [&](int first) {
+        const float2 xa = rd.xcf[at(i0 + first + lane, N - 1)], fa = rd.xvf[at(i0 + first + lane, N)];
+        __syncwarp();
+        rows[R_C1][lane] = f2(from(xa, B.p1.x, B_lo[1]));
+        rows[R_C2][lane] = f2(from(xa, B.p2.x, B_lo[6]));
+        rows[R_XX][lane] = f2(__fmul_rn(xa.x, xa.x));
+        rows[R_F1][lane] = f2(from(fa, B.p1.x, B_lo[1]));
+        rows[R_F2][lane] = f2(from(fa, B.p2.x, B_lo[6]));
+        __syncwarp();
+    };
     const float near2 = (P.sink_r2 + P.soft2) * 1.0001f;    // the sinks' vote: softened distance, with a margin
-    // dy^2 + s^2 of a pair of y positions to a body
-    auto col_part = [&](float2 y, float2 by) {
-        const float2 d = sub2(y, by);
-        return fma2(d, d, K[C_SOFT2]);
+    // dy^2 + s^2 of the pair's left faces and of its centres to either body (isothermal)
+    constexpr int NPART = NF == 3 ? 4 : 1;
+    __shared__ float2 part[NPART][32];
+    if constexpr (NF == 3) {
+        auto col_part = [&](float2 d) { return fma2(d, d, K[C_SOFT2]); };
+        part[0][lane] = col_part(dyv1[lane]);
+        part[1][lane] = col_part(dyv2[lane]);
+        part[2][lane] = col_part(dyc1[lane]);
+        part[3][lane] = col_part(dyc2[lane]);
+    }
+    // cs2 = -phi / M^2 (physics.rs:584-607) with the Plummer potential, of two faces dx1, dx2 from the bodies along x
+    auto sound2 = [&](float2 dx1, float2 dx2, int which) {
+        const float2 r1 = rsqrt2(fma2(dx1, dx1, part[which % NPART][lane]));
+        const float2 r2 = rsqrt2(fma2(dx2, dx2, part[(which + 1) % NPART][lane]));
+        return fma2(K[C_CM1], r1, mul2(K[C_CM2], r2));
     };
 
     float2 Pm1[NF], P0[NF];           // primitives of rows g - 1 and g
     float2 xl[NF], xtn, xtt;          // row g - 1: state at its lower x faces, stresses
-    float2 fx[NF], dfy[NF];           // flux through row g - 1's upper x faces; its y fluxes' difference
+    float2 div[NF];                   // row g - 1's y fluxes' difference less the flux through its upper x faces
     constexpr int NACC = T::SINKS_AT;
     float2 acc[NACC];                 // ledger items that are live everywhere, summed over rows
 #pragma unroll
     for (int m = 0; m < NACC; ++m) acc[m] = f2(0.0f);
 #pragma unroll
-    for (int f = 0; f < NF; ++f) Pm1[f] = P0[f] = xl[f] = fx[f] = dfy[f] = f2(0.0f);
+    for (int f = 0; f < NF; ++f) Pm1[f] = P0[f] = xl[f] = div[f] = f2(0.0f);
     xtn = xtt = f2(0.0f);
     bool sinks_seen = false, fake_seen = false;
     float amax = 0.0f;
     int brow = i0 / bs, next_flush = bs - i0 % bs;          // row count at which block row `brow` ends
-    const float* xcr = rd.xcf + i0;                         // (the tables go on two entries beyond either end)
-    const float* xvr = rd.xvgf + i0;
-    float x_up = xcr[0], x_c = xcr[0], x_f = xvr[0];        // zone rows g - 1 and g, face g - 1/2
-    E* out = (E*)rd.slot[a.out_slot] + (size_t)i0 * N + j0 + c0;   // this pair of row g - 1
+    E* out = (E*)rd.slot[a.out_slot];
+    __builtin_assume(__isGlobal(out));
+    out += (size_t)i0 * N + j0 + c0;                        // this pair of row g - 1
 
+    int next_fill = 0;
     for (int n = -2; n <= TH + 1; ++n) {
         issue(n + 1, n - 1);
         const int gr = n - 1;
-        // positions of the next iteration's rows, loaded a row ahead
-        const float x_c_next = xcr[gr + 1], x_f_next = xvr[gr + 1];
+        if (gr == next_fill) {   // the table holds rows gr - 1 to gr + 30
+            fill_rows(gr - 1);
+            next_fill += 31;
+        }
+        const int rt = gr - (next_fill - 32);               // row g's place in it
 
         // ---- row n -> primitives (try_block_primitive, scheme.rs:185-199) ------------
         float2 pn[NF];
@@ -694,59 +717,53 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                 if (lane == 0) lv[f] = poison_or(lv[f]);
                 if (lane == 31) rv[f] = poison_or(rv[f]);
             }
-            float2 thx = K[C_THETA], thy = thx;
+            float2 thx = K[C_THETA2], thy = thx;
             if (pdt > 0.0f) {   // (densities below 0 fail the advance before their slopes count)
-                thx = make_float2((Pm1[0].x < pdt || P0[0].x < pdt || pn[0].x < pdt) ? 0.0f : theta,
-                                  (Pm1[0].y < pdt || P0[0].y < pdt || pn[0].y < pdt) ? 0.0f : theta);
-                thy = make_float2((lv[0] < pdt || P0[0].x < pdt || P0[0].y < pdt) ? 0.0f : theta,
-                                  (P0[0].x < pdt || P0[0].y < pdt || rv[0] < pdt) ? 0.0f : theta);
+                thx = make_float2((Pm1[0].x < pdt || P0[0].x < pdt || pn[0].x < pdt) ? 0.0f : theta2,
+                                  (Pm1[0].y < pdt || P0[0].y < pdt || pn[0].y < pdt) ? 0.0f : theta2);
+                thy = make_float2((lv[0] < pdt || P0[0].x < pdt || P0[0].y < pdt) ? 0.0f : theta2,
+                                  (P0[0].x < pdt || P0[0].y < pdt || rv[0] < pdt) ? 0.0f : theta2);
             }
-            float2 gx[NF], gy[NF];
+            float2 gx[NF], gy[NF];                          // twice the slopes
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
                 gx[f] = plm_gradient2(thx, Pm1[f], P0[f], pn[f]);
                 gy[f] = plm_gradient2(thy, make_float2(lv[f], P0[f].x), P0[f], make_float2(P0[f].y, rv[f]));
             }
-            const float2 da = mul2(gx[1], K[C_INV_DX]), db = mul2(gy[2], K[C_INV_DX]);
-            const float2 lb = mul2(K[C_LAMBDA], add2(da, db));
-            const float2 cv = P.visc == 0 ? mul2(K[C_NU], P0[0]) : (NF == 3 ? P0[0] : mul2(K[C_GAMMA], P0[NF - 1]));
-            const float2 txx = mul2(cv, fma2(K[C_43], da, fma2(K[C_N23], db, lb)));
-            const float2 tyy = mul2(cv, fma2(K[C_43], db, fma2(K[C_N23], da, lb)));
-            const float2 txy = mul2(cv, mul2(add2(gx[2], gy[1]), K[C_INV_DX]));
+            const float2 cv = mul2(K[C_VISC], P0[NF == 4 && P.visc != 0 ? NF - 1 : 0]);
+            const float2 txx = mul2(cv, fma2(K[C_TN], gx[1], mul2(K[C_TT], gy[2])));
+            const float2 tyy = mul2(cv, fma2(K[C_TN], gy[2], mul2(K[C_TT], gx[1])));
+            const float2 txy = mul2(cv, add2(gx[2], gy[1]));
 
             if (gr >= 0) {
                 // ---- y fluxes of row g at the pair's left faces -------------------------
-                float2 Fy[NF], dfy_new[NF];
+                float2 Fy[NF], dfy[NF];
                 {
                     float2 pl[NF], pr[NF];
 #pragma unroll
                     for (int f = 0; f < NF; ++f) {
-                        const float2 e = fma2(gy[f], K[C_HALF], P0[f]);
+                        const float2 e = fma2(gy[f], K[C_QUARTER], P0[f]);
                         pl[f] = make_float2(__shfl_up_sync(0xffffffffu, e.y, 1), e.x);
-                        pr[f] = fma2(gy[f], K[C_NHALF], P0[f]);
+                        pr[f] = fma2(gy[f], K[C_NQUARTER], P0[f]);
                     }
                     const float2 tn = add2(make_float2(__shfl_up_sync(0xffffffffu, tyy.y, 1), tyy.x), tyy);
                     const float2 tt = add2(make_float2(__shfl_up_sync(0xffffffffu, txy.y, 1), txy.x), txy);
                     float2 cs2 = f2(0.0f), k = K[C_HALF], vxs = f2(0.0f), vys = f2(0.0f);
-                    if constexpr (NF == 3) {
-                        // cs2 = -phi / M^2 (physics.rs:584-607), Plummer potential
-                        const float d1 = x_c - B.p1.x, d2 = x_c - B.p2.x;
-                        const float2 r1 = rsqrt2(add2(f2(__fmul_rn(d1, d1)), col_part(yv2, K[C_Y1])));
-                        const float2 r2 = rsqrt2(add2(f2(__fmul_rn(d2, d2)), col_part(yv2, K[C_Y2])));
-                        cs2 = mul2(fma2(K[C_M1], r1, mul2(K[C_M2], r2)), K[C_INV_MACH2]);
-                    } else {
+                    const float2 dx1 = rows[R_C1][rt], dx2 = rows[R_C2][rt];
+                    if constexpr (NF == 3) cs2 = sound2(dx1, dx2, 0);
+                    else {
                         vxs = add2(make_float2(lv[1], P0[1].x), P0[1]);
                         vys = add2(make_float2(lv[2], P0[2].x), P0[2]);
                     }
                     if (P.visc != 0) {
-                        k = alpha_half_k2(K, B, x_c, yv2);
+                        k = alpha_half_k2(K, dx1, dx2, dyv1[lane], dyv2[lane]);
                         if constexpr (NF == 3) k = mul2(k, cs2);
                     }
                     faces2<NF, 1>(K, pl, pr, cs2, k, tn, tt, vxs, vys, Fy);
 #pragma unroll
                     for (int f = 0; f < NF; ++f) {
                         const float2 right = make_float2(Fy[f].y, __shfl_down_sync(0xffffffffu, Fy[f].x, 1));
-                        dfy_new[f] = sub2(right, Fy[f]);
+                        dfy[f] = sub2(right, Fy[f]);
                     }
                 }
                 // ---- x fluxes between rows g - 1 and g ----------------------------------
@@ -754,19 +771,16 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                 {
                     float2 pr[NF];
 #pragma unroll
-                    for (int f = 0; f < NF; ++f) pr[f] = fma2(gx[f], K[C_NHALF], P0[f]);
+                    for (int f = 0; f < NF; ++f) pr[f] = fma2(gx[f], K[C_NQUARTER], P0[f]);
                     float2 cs2 = f2(0.0f), k = K[C_HALF], vxs = f2(0.0f), vys = f2(0.0f);
-                    if constexpr (NF == 3) {
-                        const float d1 = x_f - B.p1.x, d2 = x_f - B.p2.x;
-                        const float2 r1 = rsqrt2(add2(f2(__fmul_rn(d1, d1)), col_part(yc2, K[C_Y1])));
-                        const float2 r2 = rsqrt2(add2(f2(__fmul_rn(d2, d2)), col_part(yc2, K[C_Y2])));
-                        cs2 = mul2(fma2(K[C_M1], r1, mul2(K[C_M2], r2)), K[C_INV_MACH2]);
-                    } else {
+                    const float2 dx1 = rows[R_F1][rt], dx2 = rows[R_F2][rt];
+                    if constexpr (NF == 3) cs2 = sound2(dx1, dx2, 2);
+                    else {
                         vxs = add2(Pm1[1], P0[1]);
                         vys = add2(Pm1[2], P0[2]);
                     }
                     if (P.visc != 0) {
-                        k = alpha_half_k2(K, B, x_f, yc2);
+                        k = alpha_half_k2(K, dx1, dx2, dyc1[lane], dyc2[lane]);
                         if constexpr (NF == 3) k = mul2(k, cs2);
                     }
                     faces2<NF, 0>(K, xl, pr, cs2, k, add2(xtn, txx), add2(xtt, txy), vxs, vys, Fx);
@@ -788,24 +802,24 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                     // sources of the pair (Physics::source_terms, physics.rs:423-457;
                     // Isothermal 528-582, Euler 683-774)
                     float2 tot[NF], it[NACC];
-                    const float dx1 = x_up - B.p1.x, dx2 = x_up - B.p2.x;
-                    const float2 dy1 = sub2(yc2, K[C_Y1]), dy2 = sub2(yc2, K[C_Y2]);
+                    const float2 dx1 = rows[R_C1][rt - 1], dx2 = rows[R_C2][rt - 1];
+                    const float2 dy1 = dyc1[lane], dy2 = dyc2[lane];
                     // Plummer accelerations (kepler-two-body, restated): -m d / (d^2 + s^2)^(3/2)
-                    const float2 t1 = fma2(dy1, dy1, f2(fmaf(dx1, dx1, P.soft2)));
-                    const float2 t2 = fma2(dy2, dy2, f2(fmaf(dx2, dx2, P.soft2)));
+                    const float2 t1 = fma2(dx1, dx1, NF == 3 ? part[2 % NPART][lane] : fma2(dy1, dy1, K[C_SOFT2]));
+                    const float2 t2 = fma2(dx2, dx2, NF == 3 ? part[3 % NPART][lane] : fma2(dy2, dy2, K[C_SOFT2]));
                     const float2 r1 = rsqrt2(t1), r2 = rsqrt2(t2);
                     const float2 r13 = mul2(r1, mul2(r1, r1)), r23 = mul2(r2, mul2(r2, r2));
                     const float2 q1 = mul2(mul2(uc[0], K[C_NM1DT]), r13);
                     const float2 q2 = mul2(mul2(uc[0], K[C_NM2DT]), r23);
                     constexpr int G2 = NF - 1, BU = 2 * (NF - 1);
-                    it[0] = mul2(q1, f2(dx1));
+                    it[0] = mul2(q1, dx1);
                     it[1] = mul2(q1, dy1);
-                    it[G2] = mul2(q2, f2(dx2));
+                    it[G2] = mul2(q2, dx2);
                     it[G2 + 1] = mul2(q2, dy2);
-                    // buffer: 0.5 rate (1 + tanh((r - R) / scale)) Omega_outer, 1 + tanh(y) = 2 / (1 + exp(-2y))
-                    const float2 rr2 = fma2(yc2, yc2, f2(__fmul_rn(x_up, x_up)));
-                    const float2 yb = mul2(sub2(sqrt2(rr2), K[C_RADIUS]), K[C_BUF_SLOPE]);
-                    const float2 den = add2(K[C_ONE], make_float2(__expf(yb.x), __expf(yb.y)));
+                    // buffer: 0.5 rate (1 + tanh(y)) Omega_outer, y = (r - R) / scale, 1 + tanh(y) = 2 / (1 + exp(-2y))
+                    const float2 yc2 = sYc[lane], rr2 = fma2(yc2, yc2, rows[R_XX][rt - 1]);
+                    const float2 yb = fma2(sqrt2(rr2), K[C_BUF_SLOPE], K[C_BUF_OFFSET]);
+                    const float2 den = add2(K[C_ONE], make_float2(exp2_fast(yb.x), exp2_fast(yb.y)));
                     const float2 kb = mul2(K[C_BUF_RATE], rcp2(den));
 #pragma unroll
                     for (int f = 0; f < NF; ++f) it[BU + f] = mul2(sub2(uc[f], u0[f]), kb);
@@ -862,9 +876,9 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                         tot[3] = add2(add2(add2(it[2], it[5]), it[BU + 3]), it[10]);
                     }
                     // sinks: only where a zone of the warp lies inside a sink radius
-                    const bool near = (inx && fminf(t1.x, t2.x) < near2) || (iny && fminf(t1.y, t2.y) < near2);
+                    const bool near = inx && fminf(min3f(t1.x, t2.x, t1.y), t2.y) < near2;
                     if (__any_sync(0xffffffffu, near) && up_ok) {
-                        float* sl = led + T::SINKS_AT * 64 + 2 * lane;
+                        float* sl = led + 2 * lane;
                         if (!sinks_seen) {
 #pragma unroll
                             for (int m = 0; m < 2 * NF; ++m) *(float2*)(sl + m * 64) = f2(0.0f);
@@ -875,7 +889,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                             float us[NF], s1[NF], s2[NF];
 #pragma unroll
                             for (int f = 0; f < NF; ++f) us[f] = side ? uc[f].y : uc[f].x;
-                            sink_items_exact<NF>(P, B, us, x_up, side ? yc2.y : yc2.x, dt, s1, s2);
+                            sink_items_exact<NF>(P, B, us, dx1.x, side ? dy1.y : dy1.x, dx2.x, side ? dy2.y : dy2.x, dt, s1, s2);
 #pragma unroll
                             for (int f = 0; f < NF; ++f) {
                                 const float sk = s1[f] + s2[f];
@@ -888,7 +902,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                     }
                     // fake mass: u0 rate dt unless Sigma < Sigma_0 threshold
                     if (fake_on && up_ok) {
-                        float* sl = led + T::FAKE_AT * 64 + 2 * lane;
+                        float* sl = led + (T::FAKE_AT - T::SINKS_AT) * 64 + 2 * lane;
                         const bool offa = uc[0].x < u0[0].x * P.fake_thr, offb = uc[0].y < u0[0].y * P.fake_thr;
 #pragma unroll
                         for (int f = 0; f < 3; ++f) {
@@ -901,12 +915,12 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                         fake_seen = true;
                     }
                     // flux divergence and the RK update (scheme.rs:290-305; state.rs:183-199)
-                    float2 uo[NF];
+                    float2 uo[NF], ulo[NF];                             // the result's high and low words
                     if constexpr (STORE == 1) {
                         df2 o[NF];
 #pragma unroll
                         for (int f = 0; f < NF; ++f) {
-                            const float2 du = mul2(add2(sub2(Fx[f], fx[f]), dfy[f]), K[C_NDT_DX]);
+                            const float2 du = mul2(add2(Fx[f], div[f]), K[C_NDT_DX]);
                             o[f] = df_add_f2(df2{uc[f], pair_of(q + f * 64)}, add2(du, tot[f]));
                         }
                         if (has_base) {
@@ -938,13 +952,13 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                             }
                         }
 #pragma unroll
-                        for (int f = 0; f < NF; ++f) uo[f] = o[f].hi;
+                        for (int f = 0; f < NF; ++f) { uo[f] = o[f].hi; ulo[f] = o[f].lo; }
                     } else {
                         double2 o[NF];
                         const double keep = -a.bf + 1.0;
 #pragma unroll
                         for (int f = 0; f < NF; ++f) {
-                            const float2 du = mul2(add2(sub2(Fx[f], fx[f]), dfy[f]), K[C_NDT_DX]);
+                            const float2 du = mul2(add2(Fx[f], div[f]), K[C_NDT_DX]);
                             const float2 inc = add2(du, tot[f]);
                             o[f] = *(const double2*)(sb + f * 64);
                             o[f].x += (double)inc.x;
@@ -954,7 +968,10 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                                 o[f].x = o[f].x * keep + b0.x * a.bf;
                                 o[f].y = o[f].y * keep + b0.y * a.bf;
                             }
-                            uo[f] = make_float2((float)o[f].x, (float)o[f].y);
+                            if (want_amax) {
+                                uo[f] = make_float2((float)o[f].x, (float)o[f].y);
+                                ulo[f] = make_float2((float)(o[f].x - (double)uo[f].x), (float)(o[f].y - (double)uo[f].y));
+                            }
                         }
                         if (up_ok && inx) {
 #pragma unroll
@@ -972,20 +989,20 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
 #pragma unroll
                         for (int m = 0; m < NACC; ++m) acc[m] = add2(acc[m], it[m]);
                         if (want_amax) {
-                            float ua[NF], ub[NF];
+                            float ua[NF], ub[NF], la[NF], lb[NF];
 #pragma unroll
-                            for (int f = 0; f < NF; ++f) { ua[f] = uo[f].x; ub[f] = uo[f].y; }
-                            if (inx) amax = fmaxf(max_speed_exact<NF>(P, ua), amax);
-                            if (iny) amax = fmaxf(max_speed_exact<NF>(P, ub), amax);
+                            for (int f = 0; f < NF; ++f) { ua[f] = uo[f].x; ub[f] = uo[f].y; la[f] = ulo[f].x; lb[f] = ulo[f].y; }
+                            if (inx) amax = fmaxf(max_speed_f32<NF>(P, ua, la), amax);
+                            if (iny) amax = fmaxf(max_speed_f32<NF>(P, ub, lb), amax);
                         }
                         if (ru + 1 == next_flush || ru + 1 == TH) {   // the end of a block row, or of the chunk
+                            float* sums = (float*)(update + (ru & 1) * T::UPDATE);   // this row's, which is done with
 #pragma unroll
                             for (int m = 0; m < NACC; ++m) {
-                                *(float2*)(led + m * 64 + 2 * lane) = acc[m];
+                                *(float2*)(sums + m * 64 + 2 * lane) = acc[m];
                                 acc[m] = f2(0.0f);
                             }
-                            flush_strip<NF, STORE>(rd, strip, ti, brow, led, sinks_seen, fake_seen, a.in_slot,
-                                                   a.base_slot, a.out_slot, a.stage, a.bf);
+                            flush_strip<NF, STORE>(rd, a.stage, strip, ti, brow, sums, led, sinks_seen, fake_seen);
                             sinks_seen = fake_seen = false;
                             ++brow;
                             next_flush += bs;
@@ -994,18 +1011,15 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                     }
                 }
 #pragma unroll
-                for (int f = 0; f < NF; ++f) { fx[f] = Fx[f]; dfy[f] = dfy_new[f]; }
+                for (int f = 0; f < NF; ++f) div[f] = sub2(dfy[f], Fx[f]);
             }
 #pragma unroll
-            for (int f = 0; f < NF; ++f) xl[f] = fma2(gx[f], K[C_HALF], P0[f]);
+            for (int f = 0; f < NF; ++f) xl[f] = fma2(gx[f], K[C_QUARTER], P0[f]);
             xtn = txx;
             xtt = txy;
         }
 #pragma unroll
         for (int f = 0; f < NF; ++f) { Pm1[f] = P0[f]; P0[f] = pn[f]; }
-        x_up = x_c;
-        x_c = x_c_next;
-        x_f = x_f_next;
     }
 
     if (want_amax) {
