@@ -16,6 +16,7 @@
 
 #include "elements.cuh"
 #include "runtime.cuh"
+#include "split.cuh"
 
 namespace b2d {
 cudaError_t launch_stage_f64(int nf, const StageArgs& a, int grid, size_t smem, cudaStream_t s);
@@ -759,6 +760,8 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
         d.amax = ctx->d_amax + i;
         d.binary_q = cfgs[i].binary_mass_ratio;
         d.binary_e = cfgs[i].binary_eccentricity;
+        d.tracer_radius = split(cfgs[i].domain_radius);
+        d.tracer_inv_dx = split(r.N / (2.0 * cfgs[i].domain_radius));
         d.p = make_params<double>(cfgs[i]);
         d.pf = make_params<float>(cfgs[i]);
         ctx->staging_bytes = std::max(ctx->staging_bytes, nn * ctx->nf * sizeof(double));
@@ -1216,60 +1219,110 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
 // input, bilinear between the four surrounding cell centres of the uniform
 // mesh, advanced by the same RK stages and weighted averages as the state and
 // wrapped into the periodic domain [-R, R)^2.  Positions are FP64.
-// Gas velocity of one cell.  R = double is the FP64 parity arithmetic; the
-// FP32 paths interpolate in FP32 (the FP64 divisions would dominate on this
-// GPU) and keep the positions in FP64.
-template <class R, int STORE>
-__device__ __forceinline__ void tracer_cell_velocity(const RunDev& rd, int slot, int i, int j, R& vx, R& vy)
+//
+// tracer_kernel<0> is the FP64 parity arithmetic; tracer_kernel<1> and <2>
+// serve the FP32 paths (FP64 state, compensated state).  What bounds them is
+// the gathers and the positions' traffic (a position 16 bytes read, its base
+// read, its result written; 12 state words around each tracer), so FP64 work,
+// at two lanes per clock and SM, is kept out: cell and offset come from the
+// position as a double-float, the displacement and the base's average too,
+// and what is left are the additions to the FP64 positions, two per
+// coordinate at most, and an integer compare for the periodic wrap.  Measured
+// at 8192^2 with 1e7 tracers: a launch takes 146 us (179 with a base),
+// about 600 when these steps were FP64 conversions and quotients.
+template <int STORE> __device__ __forceinline__ float2 tracer_velocity_f32(const RunDev& rd, int slot, size_t idx)
 {
-    const size_t nn = (size_t)rd.N * rd.N, idx = (size_t)i * rd.N + j;
-    R u[3];
+    const size_t nn = (size_t)rd.N * rd.N;
+    float u[3];
     for (int f = 0; f < 3; ++f) {
-        if (STORE == 0) u[f] = (R)((const double*)rd.slot[slot])[f * nn + idx];
-        else u[f] = (R)((const float*)rd.slot[slot])[(2 * f) * nn + idx];
+        if (STORE == 1) u[f] = narrow(((const double*)rd.slot[slot])[f * nn + idx]);
+        else u[f] = ((const float*)rd.slot[slot])[(2 * f) * nn + idx];
     }
-    if constexpr (std::is_same<R, double>::value) {
-        vx = u[1] / u[0];
-        vy = u[2] / u[0];
-    } else {
-        const float ir = __fdividef(1.0f, u[0]);
-        vx = u[1] * ir;
-        vy = u[2] * ir;
-    }
+    const float ir = __fdividef(1.0f, u[0]);
+    return make_float2(u[1] * ir, u[2] * ir);
 }
 
-template <class T, int STORE>
-__global__ void tracer_kernel(const RunDev* runs, int run, int in_slot, int base_slot, int out_slot, double bf)
+// The cell centre below coordinate v (as hi + lo) and the offset from it in
+// cells: (v + R) / dx - 1/2 = i + a.
+__device__ __forceinline__ void tracer_cell(float hi, float lo, float2 R, float2 inv_dx, int& i, float& a)
+{
+    // s + e = v + R
+    const float s = __fadd_rn(hi, R.x), bb = __fadd_rn(s, -hi);
+    const float e = __fadd_rn(__fadd_rn(__fadd_rn(hi, -__fadd_rn(s, -bb)), __fadd_rn(R.x, -bb)), __fadd_rn(lo, R.y));
+    const float p = __fmul_rn(s, inv_dx.x);
+    const float q = __fmaf_rn(e, inv_dx.x, __fmaf_rn(s, inv_dx.y, __fmaf_rn(s, inv_dx.x, -p)));
+    const float g = __fadd_rn(p, -0.5f), fl = floorf(g);
+    i = (int)fl;
+    a = __fadd_rn(__fadd_rn(g, -fl), q);
+    // p's rounding can put a position on the wrong side of a cell's edge
+    if (a < 0.0f) { --i; a += 1.0f; } else if (a >= 1.0f) { ++i; a -= 1.0f; }
+}
+
+static __device__ __noinline__ double tracer_wrap(double xo, double R)
+{
+    if (xo >= R) xo -= 2.0 * R;
+    if (xo < -R) xo += 2.0 * R;
+    return xo;
+}
+
+// x + (hi + lo), or with a base xb + w (x + (hi + lo) - xb) on the base's
+// periodic image, wrapped into [-R, R).
+__device__ __forceinline__ double tracer_move(double x, float xh, float xl, float d, bool has_base, double xb, float2 w,
+                                              double R, float Rf)
+{
+    double xo;
+    if (!has_base) xo = x + widen(d);
+    else {
+        float bh, bl;
+        split_double(xb, bh, bl);
+        // h + l = x - xb + d
+        float dd = __fadd_rn(xh, -bh);
+        const float ee = __fadd_rn(dd, -xh);
+        float l = __fadd_rn(__fadd_rn(__fadd_rn(xh, -__fadd_rn(dd, -ee)), -__fadd_rn(bh, ee)), __fadd_rn(xl, -bl));
+        if (dd > Rf) dd = __fadd_rn(dd, -2.0f * Rf);
+        else if (dd < -Rf) dd = __fadd_rn(dd, 2.0f * Rf);
+        const float h = __fadd_rn(dd, d), bb = __fadd_rn(h, -dd);
+        l = __fadd_rn(l, __fadd_rn(__fadd_rn(dd, -__fadd_rn(h, -bb)), __fadd_rn(d, -bb)));
+        // times w
+        const float p = __fmul_rn(h, w.x);
+        const float q = __fmaf_rn(l, w.x, __fmaf_rn(h, w.y, __fmaf_rn(h, w.x, -p)));
+        xo = (xb + widen(p)) + widen(q);
+    }
+    const unsigned long long m = (unsigned long long)__double_as_longlong(xo) & 0x7fffffffffffffffull;
+    return m >= (unsigned long long)__double_as_longlong(R) ? tracer_wrap(xo, R) : xo;
+}
+
+// MODE 0: FP64 arithmetic on the FP64 state; 1, 2: FP32 arithmetic on the FP64, compensated state.
+// bf: the base's weight; w: 1 - bf as FP32 high and low words.
+template <int MODE>
+__global__ void __launch_bounds__(256) tracer_kernel(const RunDev* runs, int run, int in_slot, int base_slot, int out_slot,
+                                                     double bf, float2 w)
 {
     const RunDev& rd = runs[run];
     const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (k >= rd.ntracers) return;
     const double R = rd.p.domain_radius, dx = rd.p.dx, dt = *rd.dt;
     const int N = rd.N;
-    const double x = rd.tracers[in_slot][2 * k], y = rd.tracers[in_slot][2 * k + 1];
-    const double L = 2.0 * R;
-    T ax, ay;
+    const double2 at = ((const double2*)rd.tracers[in_slot])[k];
+    double2 base = make_double2(0.0, 0.0);
+    if (base_slot >= 0) base = ((const double2*)rd.tracers[base_slot])[k];
     int i0, j0;
-    if constexpr (std::is_same<T, double>::value) {
+    double gx = 0.0, gy = 0.0;
+    float ax = 0.0f, ay = 0.0f, xh = 0.0f, xl = 0.0f, yh = 0.0f, yl = 0.0f;
+    if constexpr (MODE == 0) {
         // the oracle's arithmetic
-        const double gx = (x + R) / dx - 0.5, gy = (y + R) / dx - 0.5;
+        gx = (at.x + R) / dx - 0.5;
+        gy = (at.y + R) / dx - 0.5;
         const double fi = floor(gx), fj = floor(gy);
-        ax = gx - fi;
-        ay = gy - fj;
+        gx = gx - fi;
+        gy = gy - fj;
         i0 = (int)fi;
         j0 = (int)fj;
     } else {
-        // FP64 is slow on this GPU: the cell from an FP32 estimate, the offset in
-        // it exactly from FP64 (one fused step), then FP32 for the rest
-        const double xr = x + R, yr = y + R;
-        const float idx_f = (float)rd.p.inv_dx;
-        i0 = (int)floorf((float)xr * idx_f - 0.5f);
-        j0 = (int)floorf((float)yr * idx_f - 0.5f);
-        ax = (float)fma(-((double)i0 + 0.5), dx, xr) * idx_f;
-        ay = (float)fma(-((double)j0 + 0.5), dx, yr) * idx_f;
-        // the FP32 estimate can be one cell off within its rounding of a boundary
-        if (ax < 0.0f) { --i0; ax += 1.0f; } else if (ax >= 1.0f) { ++i0; ax -= 1.0f; }
-        if (ay < 0.0f) { --j0; ay += 1.0f; } else if (ay >= 1.0f) { ++j0; ay -= 1.0f; }
+        split_double(at.x, xh, xl);
+        split_double(at.y, yh, yl);
+        tracer_cell(xh, xl, rd.tracer_radius, rd.tracer_inv_dx, i0, ax);
+        tracer_cell(yh, yl, rd.tracer_radius, rd.tracer_inv_dx, j0, ay);
     }
     // positions are kept in [-R, R), so the cell index is in [-1, N - 1]: one
     // conditional wrap, then a clamp that keeps any other input in bounds
@@ -1278,69 +1331,66 @@ __global__ void tracer_kernel(const RunDev* runs, int run, int in_slot, int base
     i0 = min(max(i0, 0), N - 1);
     j0 = min(max(j0, 0), N - 1);
     const int i1 = i0 + 1 == N ? 0 : i0 + 1, j1 = j0 + 1 == N ? 0 : j0 + 1;
-    T v00x, v00y, v10x, v10y, v01x, v01y, v11x, v11y;
-    tracer_cell_velocity<T, STORE>(rd, in_slot, i0, j0, v00x, v00y);
-    tracer_cell_velocity<T, STORE>(rd, in_slot, i1, j0, v10x, v10y);
-    tracer_cell_velocity<T, STORE>(rd, in_slot, i0, j1, v01x, v01y);
-    tracer_cell_velocity<T, STORE>(rd, in_slot, i1, j1, v11x, v11y);
-    const T one = T(1);
-    const T w00 = (one - ax) * (one - ay), w10 = ax * (one - ay), w01 = (one - ax) * ay, w11 = ax * ay;
-    const T vx = w00 * v00x + w10 * v10x + w01 * v01x + w11 * v11x;
-    const T vy = w00 * v00y + w10 * v10y + w01 * v01y + w11 * v11y;
+    const size_t c00 = (size_t)i0 * N + j0, c01 = (size_t)i0 * N + j1, c10 = (size_t)i1 * N + j0, c11 = (size_t)i1 * N + j1;
     double xo, yo;
-    if constexpr (std::is_same<T, double>::value) {
-        xo = x + dt * vx;
-        yo = y + dt * vy;
+    if constexpr (MODE == 0) {
+        const size_t nn = (size_t)N * N;
+        const double* u = (const double*)rd.slot[in_slot];
+        auto vel = [&](size_t c, double& vx, double& vy) {
+            vx = u[nn + c] / u[c];
+            vy = u[2 * nn + c] / u[c];
+        };
+        double v00x, v00y, v10x, v10y, v01x, v01y, v11x, v11y;
+        vel(c00, v00x, v00y);
+        vel(c10, v10x, v10y);
+        vel(c01, v01x, v01y);
+        vel(c11, v11x, v11y);
+        const double w00 = (1.0 - gx) * (1.0 - gy), w10 = gx * (1.0 - gy), w01 = (1.0 - gx) * gy, w11 = gx * gy;
+        const double L = 2.0 * R;
+        xo = at.x + dt * (w00 * v00x + w10 * v10x + w01 * v01x + w11 * v11x);
+        yo = at.y + dt * (w00 * v00y + w10 * v10y + w01 * v01y + w11 * v11y);
         if (base_slot >= 0) {
             // average with the base position on the same periodic image
-            const double xb = rd.tracers[base_slot][2 * k], yb = rd.tracers[base_slot][2 * k + 1];
-            if (xo - xb > R) xo -= L;
-            else if (xo - xb < -R) xo += L;
-            if (yo - yb > R) yo -= L;
-            else if (yo - yb < -R) yo += L;
-            xo = xo * (-bf + 1.0) + xb * bf;
-            yo = yo * (-bf + 1.0) + yb * bf;
+            if (xo - base.x > R) xo -= L;
+            else if (xo - base.x < -R) xo += L;
+            if (yo - base.y > R) yo -= L;
+            else if (yo - base.y < -R) yo += L;
+            xo = xo * (-bf + 1.0) + base.x * bf;
+            yo = yo * (-bf + 1.0) + base.y * bf;
         }
+        if (xo >= R) xo -= L;
+        if (xo < -R) xo += L;
+        if (yo >= R) yo -= L;
+        if (yo < -R) yo += L;
     } else {
-        // the stage's displacement in FP32, accumulated in FP64
-        const float dtf = (float)dt;
-        xo = x + (double)(dtf * vx);
-        yo = y + (double)(dtf * vy);
-        if (base_slot >= 0) {
-            // base + (new - base) (1 - bf), on the base's periodic image
-            const double xb = rd.tracers[base_slot][2 * k], yb = rd.tracers[base_slot][2 * k + 1];
-            double ddx = xo - xb, ddy = yo - yb;
-            const float Rf = (float)R;
-            if ((float)ddx > Rf) ddx -= L;
-            else if ((float)ddx < -Rf) ddx += L;
-            if ((float)ddy > Rf) ddy -= L;
-            else if ((float)ddy < -Rf) ddy += L;
-            const double w1 = -bf + 1.0;
-            xo = fma(ddx, w1, xb);
-            yo = fma(ddy, w1, yb);
-        }
+        const float2 v00 = tracer_velocity_f32<MODE>(rd, in_slot, c00), v10 = tracer_velocity_f32<MODE>(rd, in_slot, c10);
+        const float2 v01 = tracer_velocity_f32<MODE>(rd, in_slot, c01), v11 = tracer_velocity_f32<MODE>(rd, in_slot, c11);
+        const float bx = 1.0f - ax, by = 1.0f - ay;
+        const float w00 = bx * by, w10 = ax * by, w01 = bx * ay, w11 = ax * ay;
+        const float vx = w00 * v00.x + w10 * v10.x + w01 * v01.x + w11 * v11.x;
+        const float vy = w00 * v00.y + w10 * v10.y + w01 * v01.y + w11 * v11.y;
+        const float dtf = narrow(dt), Rf = rd.tracer_radius.x;
+        xo = tracer_move(at.x, xh, xl, dtf * vx, base_slot >= 0, base.x, w, R, Rf);
+        yo = tracer_move(at.y, yh, yl, dtf * vy, base_slot >= 0, base.y, w, R, Rf);
     }
-    if (xo >= R) xo -= L;
-    if (xo < -R) xo += L;
-    if (yo >= R) yo -= L;
-    if (yo < -R) yo += L;
-    rd.tracers[out_slot][2 * k] = xo;
-    rd.tracers[out_slot][2 * k + 1] = yo;
+    ((double2*)rd.tracers[out_slot])[k] = make_double2(xo, yo);
 }
 
 static b2d_status launch_tracers(b2d_ctx* ctx, const StagePlan& sp, bool count)
 {
+    const df32w keep = split_df(-sp.bf + 1.0);
+    const float2 w = make_float2(keep.hi, keep.lo);   // the new position's weight
     for (int r = 0; r < ctx->nruns; ++r) {
         const long long n = ctx->rdev_h[r].ntracers;
         if (n <= 0) continue;
         const int threads = 256;
         const unsigned grid = (unsigned)((n + threads - 1) / threads);
         if (ctx->precision == B2D_PREC_FP64)
-            tracer_kernel<double, 0><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf);
+            tracer_kernel<0><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w);
         else if (ctx->precision == B2D_PREC_FP32_STATE64)
-            tracer_kernel<float, 0><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf);
+            tracer_kernel<1><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w);
         else
-            tracer_kernel<float, 1><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf);
+            tracer_kernel<2><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w);
         CUDA_TRY(cudaGetLastError());
         if (count) ctx->launches++;
     }

@@ -48,6 +48,7 @@ struct RunDev {
     double el0[4];               // unperturbed elements (a, M, q, e), physics.rs:411-417
     long long ntracers;          // massless tracer particles of this run (0: none)
     double* tracers[NSLOTS];     // [ntracers][2] positions (x, y) per state slot
+    float2 tracer_radius, tracer_inv_dx;   // domain radius and 1 / dx as FP32 high and low words
     DevParams p;     // FP64 kernels
     DevParamsF pf;   // FP32 kernels
 };
