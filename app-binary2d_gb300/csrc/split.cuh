@@ -15,6 +15,7 @@ namespace b2d {
 // of the test that decides whether they are wanted.
 static __device__ __noinline__ float narrow_any(double v) { return (float)v; }
 static __device__ __noinline__ double widen_any(float v) { return (double)v; }
+static __device__ __noinline__ double halve_any(double v) { return 0.5 * v; }
 static __device__ __noinline__ float2 split_any(double v)
 {
     const float hi = (float)v;
@@ -61,6 +62,14 @@ __device__ __forceinline__ float narrow_bits(double v)
 }
 
 __device__ __forceinline__ float narrow(double v) { return split_range(v) ? narrow_bits(v) : narrow_any(v); }
+
+// v / 2: one off the exponent.
+__device__ __forceinline__ double halve(double v)
+{
+    const unsigned h = (unsigned)__double2hiint(v);
+    if ((h & 0x7fffffffu) - 0x00200000u >= 0x7fd00000u) return halve_any(v);   // zero, next to subnormal, infinite, NaN
+    return __hiloint2double((int)(h - 0x00100000u), __double2loint(v));
+}
 
 // Exact for zero, normal and (flushed to zero) subnormal v.
 __device__ __forceinline__ double widen(float v)

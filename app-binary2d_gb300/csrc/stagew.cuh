@@ -46,12 +46,15 @@
 // step over 512 columns), 384^2 33 -> 22 -> 14.8 us, the 64-run sweep 1.05 ->
 // 0.69 -> 0.57 ms, Euler 4096^2 0.65 -> 0.55 -> 0.49 ms, 768^2 48 -> 42 -> 34 us,
 // blocks of 50^2 (RK3, alpha viscosity) 163 -> 25 -> 14.5 us (one thread per
-// column of a block), FP64 state 1024^2 106 -> 94 -> 82 us.  Tried and slower:
+// column of a block), FP64 state 1024^2 106 -> 94 -> 47 us (the last of it by forming FP32 pairs of
+// the FP64 words, and widening increments, with integer instructions: with the
+// FP64 pipe's conversions for either or both 50 to 70 us).  Tried and slower:
 // the row loop unrolled twice (104 against 98 us at 2048^2: spills), the run's
 // descriptor as a kernel argument (99 against 92), programmatic dependent
 // launch (768^2: 47 against 40 us).
 #pragma once
 
+#include "split.cuh"
 #include "stage.cuh"
 
 namespace b2d {
@@ -442,12 +445,30 @@ template <int PENDING> __device__ __forceinline__ void copy_wait()
     asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
 }
 
-// A staged pair at the stencil's precision, and whole.
+// A staged pair, and the pairs of all fields at the stencil's precision (an
+// FP64 state's by integer operations: the FP64 pipe converts two lanes a clock).
 __device__ __forceinline__ float2 pair_of(const float* p) { return *(const float2*)p; }
-__device__ __forceinline__ float2 pair_of(const double* p)
+template <int NF> __device__ __forceinline__ void pairs_of(const float* p, float2* u)
 {
-    const double2 v = *(const double2*)p;
-    return make_float2((float)v.x, (float)v.y);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) u[f] = pair_of(p + f * 64);
+}
+template <int NF> __device__ __forceinline__ void pairs_of(const double* p, float2* u)
+{
+    double2 v[NF];
+    bool ok = true;
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        v[f] = *(const double2*)(p + f * 64);
+        ok = ok && split_range(v[f].x) && split_range(v[f].y);
+    }
+    if (ok) {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) u[f] = make_float2(narrow_bits(v[f].x), narrow_bits(v[f].y));
+    } else {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) u[f] = make_float2(narrow(v[f].x), narrow(v[f].y));
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -659,8 +680,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
             copy_wait<1>();   // the row's group, and that of the update below
             const E* sb = my_stencil + ((n + 2) & (SW_SLOTS - 1)) * T::STENCIL;
             float2 u[NF];
-#pragma unroll
-            for (int f = 0; f < NF; ++f) u[f] = pair_of(sb + f * 64);
+            pairs_of<NF>(sb, u);
             int ea = 0, eb = 0;
             if constexpr (NF == 3) {
                 if (P.has_density_floor) {
@@ -794,11 +814,8 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                     const E* qg = q + (STORE == 1 ? NF * 64 : 0);                    // background
                     const E* qb = qg + NF * 64;                                      // RK base
                     float2 uc[NF], u0[NF];
-#pragma unroll
-                    for (int f = 0; f < NF; ++f) {
-                        uc[f] = pair_of(sb + f * 64);
-                        u0[f] = pair_of(qg + f * 64);
-                    }
+                    pairs_of<NF>(sb, uc);
+                    pairs_of<NF>(qg, u0);
                     // sources of the pair (Physics::source_terms, physics.rs:423-457;
                     // Isothermal 528-582, Euler 683-774)
                     float2 tot[NF], it[NACC];
@@ -955,22 +972,28 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                         for (int f = 0; f < NF; ++f) { uo[f] = o[f].hi; ulo[f] = o[f].lo; }
                     } else {
                         double2 o[NF];
-                        const double keep = -a.bf + 1.0;
 #pragma unroll
                         for (int f = 0; f < NF; ++f) {
                             const float2 du = mul2(add2(Fx[f], div[f]), K[C_NDT_DX]);
                             const float2 inc = add2(du, tot[f]);
                             o[f] = *(const double2*)(sb + f * 64);
-                            o[f].x += (double)inc.x;
-                            o[f].y += (double)inc.y;
-                            if (has_base) {
+                            o[f].x += widen(inc.x);
+                            o[f].y += widen(inc.y);
+                        }
+                        if (has_base) {
+                            const double keep = -a.bf + 1.0;
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) {
                                 const double2 b0 = *(const double2*)(qb + f * 64);
-                                o[f].x = o[f].x * keep + b0.x * a.bf;
-                                o[f].y = o[f].y * keep + b0.y * a.bf;
+                                if (half_avg) o[f] = make_double2(halve(o[f].x + b0.x), halve(o[f].y + b0.y));
+                                else o[f] = make_double2(o[f].x * keep + b0.x * a.bf, o[f].y * keep + b0.y * a.bf);
                             }
-                            if (want_amax) {
-                                uo[f] = make_float2((float)o[f].x, (float)o[f].y);
-                                ulo[f] = make_float2((float)(o[f].x - (double)uo[f].x), (float)(o[f].y - (double)uo[f].y));
+                        }
+                        if (want_amax) {
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) {
+                                split_double(o[f].x, uo[f].x, ulo[f].x);
+                                split_double(o[f].y, uo[f].y, ulo[f].y);
                             }
                         }
                         if (up_ok && inx) {
