@@ -22,10 +22,10 @@ namespace b2d {
 cudaError_t launch_stage_f64(int nf, const StageArgs& a, int grid, size_t smem, cudaStream_t s);
 cudaError_t launch_buffer_rate(const RunDev* runs, int run, int N, double* out, cudaStream_t s);
 size_t stage_f64_smem(int nf, int th, int tw);
-cudaError_t launch_stage_f32_iso(int store, bool even, const StageArgs& a, int grid, cudaStream_t s);
-cudaError_t launch_stage_f32_euler(int store, bool even, const StageArgs& a, int grid, cudaStream_t s);
-int resident_f32_iso(int store, bool even, int nruns);
-int resident_f32_euler(int store, bool even, int nruns);
+cudaError_t launch_stage_f32_iso(int store, int divisor, const StageArgs& a, int grid, cudaStream_t s);
+cudaError_t launch_stage_f32_euler(int store, int divisor, const StageArgs& a, int grid, cudaStream_t s);
+int resident_f32_iso(int store, int divisor, int nruns);
+int resident_f32_euler(int store, int divisor, int nruns);
 void host_block_vertices(const b2d_config* c, int b, double* xv);
 void host_cell_centers(const b2d_config* c, int b, double* xc);
 }  // namespace b2d
@@ -534,12 +534,14 @@ static int row_chunks(const b2d_ctx* ctx, const RunHost& r)
     return r.N / ctx->th;
 }
 
-// Every run has an even number of columns: the FP32 kernel stages pairs of them as one word.
-static bool even_columns(const b2d_ctx* ctx)
+// 4, 2 or 1: the largest of them that divides the sides of all runs (how many
+// columns the FP32 kernel can copy as one aligned word).
+static int side_divisor(const b2d_ctx* ctx)
 {
+    int d = 4;
     for (const RunHost& r : ctx->runs)
-        if (r.N % 2) return false;
-    return true;
+        while (r.N % d) d /= 2;
+    return d;
 }
 
 // Buffers for the ledger pieces of as many stages as PIECE_BYTES hold (at
@@ -1238,7 +1240,7 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
     if (ctx->precision == B2D_PREC_FP64)
         e = launch_stage_f64(ctx->nf, a, ctx->total_tiles, stage_f64_smem(ctx->nf, ctx->sub_h, ctx->sub_w), ctx->stream);
     else
-        e = (ctx->nf == 3 ? launch_stage_f32_iso : launch_stage_f32_euler)(store_of(ctx), even_columns(ctx), a,
+        e = (ctx->nf == 3 ? launch_stage_f32_iso : launch_stage_f32_euler)(store_of(ctx), side_divisor(ctx), a,
                                                                            ctx->total_tiles, ctx->stream);
     if (e != cudaSuccess) return fail(B2D_ERR_CUDA, std::string("stage kernel launch: ") + cudaGetErrorString(e));
     return B2D_OK;
@@ -1832,7 +1834,7 @@ static long long resident_ctas(const b2d_ctx* ctx)
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    return (long long)sms * (ctx->nf == 3 ? resident_f32_iso : resident_f32_euler)(store_of(ctx), even_columns(ctx), ctx->nruns);
+    return (long long)sms * (ctx->nf == 3 ? resident_f32_iso : resident_f32_euler)(store_of(ctx), side_divisor(ctx), ctx->nruns);
 }
 
 // CTAs of a launch with row chunks of at most `rows` rows.

@@ -19,17 +19,20 @@
 //  * Packed arithmetic.  Every per-column quantity is a float2 and the
 //    arithmetic runs as Blackwell's packed FADD2 / FMUL2 / FFMA2; min / max,
 //    compares, selects and the special-function unit stay per column.
-//  * Row staging.  Every lane copies its own two columns of the rows ahead into
-//    a ring in shared memory by asynchronous copies (8 bytes, or 16 of an FP64
-//    state; a mesh of odd side takes single words), one group per row: the
-//    stage input a row ahead of its use, and what the update reads besides (low
-//    words, background, RK base).  Lanes read back only what they copied
-//    themselves, so nothing waits but the lane.  The periodic edge is a matter
-//    of a lane's column.  (Bulk copies (TMA) cost more here: a warp's row is 15
-//    planes of 240 bytes, each an instruction of its own with uniform
-//    addresses, 180 of 970 instructions a row.)
+//  * Row staging.  Asynchronous copies bring the rows ahead into a ring in
+//    shared memory, one group per row: the stage input a row ahead of its use,
+//    and what the update reads besides (low words, background, RK base).  Where
+//    four columns are an aligned 16 bytes (an FP32 state whose sides are
+//    multiples of 4; any pair of an FP64 state) the copies go past the L1: with
+//    8-byte copies through it every row in flight holds three lines per plane,
+//    more than the L1 has beside the rings (Euler 4096^2 474 us a stage with
+//    28 KB of L1 left, 392 with 60 KB, 375 past it).  Other sides copy pairs or
+//    single words.  (Bulk copies (TMA) cost more here: a warp's row is 15 planes
+//    of 240 bytes, each an instruction of its own with uniform addresses, 180 of
+//    970 instructions a row.)
 //  * Constants that packed instructions take are kept twice, as a pair, in
-//    shared memory: one load instead of two moves per use.
+//    shared memory: one load instead of two moves per use.  All shared memory is
+//    one block behind one address.
 //  * Pipeline.  Iteration n converts row n, forms slopes and stresses of row
 //    g = n - 1, its upper x faces and its y faces, and updates row g - 1.
 //  * Ledger.  The items that are live everywhere are summed per column in
@@ -38,20 +41,27 @@
 //    pieces of all stages are folded, in order, after the last of them: a fence,
 //    a counter and a fold in the stage's tail cost it about 5 us.
 //
-// What bounds it: instruction issue (about 660 warp instructions per row of
-// 60 columns and isothermal first stage, 390 of them arithmetic; issue 59 %
-// busy at 12 warps per SM), not memory (3.4 of 6.7 TB/s).  Measured per stage, as
-// this file began and now, against the kernels that it took the place of:
-// isothermal 2048^2 0.127 -> 0.109 -> 0.084 ms (a CTA of 10 warps marching in
-// step over 512 columns), 384^2 33 -> 22 -> 14.8 us, the 64-run sweep 1.05 ->
-// 0.69 -> 0.57 ms, Euler 4096^2 0.65 -> 0.55 -> 0.49 ms, 768^2 48 -> 42 -> 34 us,
-// blocks of 50^2 (RK3, alpha viscosity) 163 -> 25 -> 14.5 us (one thread per
-// column of a block), FP64 state 1024^2 106 -> 94 -> 47 us (the last of it by forming FP32 pairs of
-// the FP64 words, and widening increments, with integer instructions: with the
-// FP64 pipe's conversions for either or both 50 to 70 us).  Tried and slower:
-// the row loop unrolled twice (104 against 98 us at 2048^2: spills), the run's
-// descriptor as a kernel argument (99 against 92), programmatic dependent
-// launch (768^2: 47 against 40 us).
+// What bounds it: instruction issue (680 warp instructions per row of 60
+// columns and isothermal first stage, guard rows and set-up included, 290 of
+// them packed or special-function arithmetic and min / max; a warp in flight
+// waits 4.4 cycles per instruction and a scheduler has three), not memory (4.0
+// of 6.7 TB/s).  Measured per stage, with the kernels that it took the place of,
+// as this file began, and now:
+//   isothermal 2048^2          127 -> 109 -> 73 us (10 warps a CTA in step over 512 columns)
+//   isothermal 384^2            33 -> 22 -> 13 us
+//   the sweep of 64 runs      1050 -> 690 -> 520 us
+//   Euler 4096^2               650 -> 550 -> 364 us
+//   Euler 768^2                 48 -> 42 -> 29.5 us
+//   blocks of 50^2, RK3, alpha 163 -> 25 -> 13.4 us (a thread per column of a block)
+//   FP64 state 1024^2          106 -> 94 -> 40 us
+// Of this, forming FP32 pairs of FP64 words and widening increments with integer
+// instructions gave the FP64 state 47 us where the FP64 pipe's conversions take 50
+// to 70.  Tried and slower: the row loop unrolled twice (104 against 98 us at
+// 2048^2: spills); the run's descriptor as a kernel argument (99 against 92);
+// programmatic dependent launch (768^2: 47 against 40 us); 16 warps per SM with
+// 128 registers (85 against 78 us: more instructions, and four warps share what
+// three nearly fill); pairs carried from row to row as 64-bit values (76 against
+// 73 us: more moves).
 #pragma once
 
 #include "split.cuh"
@@ -60,32 +70,54 @@
 namespace b2d {
 
 constexpr int SW_COLS = 60;              // columns of a strip
-constexpr int SW_CTAS = 12;              // one-warp CTAs per SM: 168 registers a thread
 constexpr int SW_SLOTS = 4;              // stencil ring: rows n - 2 (for its update) to n + 1
 constexpr int SW_USLOTS = 2;             // update rows: one in use, one ahead
 
+// Constants as pairs, with what can be folded into them: the limiter works on
+// slopes over theta, the stress on (slope / dx) times c, the sound speed on
+// masses over Mach^2, the buffer on powers of two.
+enum {
+    C_ITHETA2,               // 1 / (2 theta), and 0 for theta = 0
+    C_EDGE, C_NEDGE,         // theta / 2: half a slope
+    C_NHALF, C_HALF, C_ONE,
+    C_TN, C_TT, C_VISC,      // 4/3 + lambda, -2/3 + lambda; theta c / dx of the cell's stress
+    C_CM1, C_CM2,            // m / Mach^2
+    C_M1, C_M2, C_NM1DT, C_NM2DT, C_SOFT2,
+    C_BUF_SLOPE, C_BUF_OFFSET, C_BUF_RATE, C_NDT_DX, C_GAMMA, C_GM1, C_INV_GM1, C_COOL, C_ALPHA, C_COUNT
+};
+
+// How a warp copies its rows: a word, a pair of columns or four columns at a
+// time, by what divides the mesh's side (four columns of FP32 words, two of FP64).
+enum { COPY_WORDS, COPY_PAIRS, COPY_QUADS };
+
 // Shared memory of one warp.
-template <int NF, int STORE> struct SWShape {
+template <int NF, int STORE, int COPY> struct SWShape {
     using E = typename std::conditional<STORE == 1, float, double>::type;
     static constexpr int NU = (STORE == 1 ? 4 : 2) * NF;  // update planes: (lo,) bg, base hi (, base lo)
     static constexpr int ITEMS = NF == 3 ? 16 : 19;       // ledger items: live everywhere, sinks, fake mass
     static constexpr int SINKS_AT = NF == 3 ? 7 : 11, FAKE_AT = 13;
-    static constexpr int STENCIL = NF * 64;               // elements of a staged row
-    static constexpr int UPDATE = NU * 64;
-    static constexpr int BYTES = (SW_SLOTS * STENCIL + SW_USLOTS * UPDATE) * (int)sizeof(E) + (ITEMS - SINKS_AT) * 64 * 4;
-    static_assert(SINKS_AT * 64 * 4 <= UPDATE * (int)sizeof(E), "a consumed update row takes the other items' sums");
-};
-
-// Constants as pairs, with what can be folded into them: the limiter works on
-// twice the slopes, the stress on (slope / dx) times c, the sound speed on
-// masses over Mach^2, the buffer on powers of two.
-enum {
-    C_THETA2,                // 2 theta
-    C_QUARTER, C_NQUARTER, C_HALF, C_ONE,
-    C_TN, C_TT, C_VISC,      // 4/3 + lambda, -2/3 + lambda; c / (2 dx) of the cell's stress
-    C_CM1, C_CM2,            // m / Mach^2
-    C_M1, C_M2, C_NM1DT, C_NM2DT, C_SOFT2,
-    C_BUF_SLOPE, C_BUF_OFFSET, C_BUF_RATE, C_NDT_DX, C_GAMMA, C_GM1, C_INV_GM1, C_COOL, C_ALPHA, C_COUNT
+    // a staged plane's row: columns -2 to 61 of the strip (quads: -4 to 63), and of the
+    // update's planes too (quads: 0 to 59)
+    static constexpr int S_PITCH = COPY == COPY_QUADS ? 68 : 64, S_FIRST = COPY == COPY_QUADS ? 2 : 0;
+    static constexpr int U_PITCH = COPY == COPY_QUADS ? 60 : 64, U_FIRST = COPY == COPY_QUADS ? -2 : 0;
+    static constexpr int PARTIALS = NF == 3 ? 4 : 1;
+    // The warp's tables.  They lie with the rings in one block, whose address is held in a register:
+    // the compiler forms the address of every shared array of its own anew wherever it is used.
+    struct Tables {
+        float2 K[C_COUNT];
+        float2 dyc1[32], dyc2[32], dyv1[32], dyv2[32], yc[32];   // of the pair's centres and left faces
+        float2 rows[5][32];                                 // dx1, dx2 and x^2 of zone rows, dx1, dx2 of the faces above
+        float2 part[PARTIALS][32];                          // dy^2 + s^2 of faces and centres to either body (isothermal)
+        Binary<float> B;
+        float B_lo[10];
+        DevParamsF P;                                       // a batched launch's parameters
+    };
+    static constexpr int TABLES = ((int)sizeof(Tables) + 127) / 128 * 128;
+    static constexpr int STENCIL = NF * S_PITCH;          // elements of a staged row
+    static constexpr int UPDATE = NU * U_PITCH;
+    static constexpr int BYTES = TABLES + (SW_SLOTS * STENCIL + SW_USLOTS * UPDATE + (COPY == COPY_QUADS ? 4 : 0)) * (int)sizeof(E);
+    static constexpr int CTAS = 12;   // per SM
+    static_assert(SINKS_AT * 64 * 4 <= UPDATE * (int)sizeof(E), "a consumed update row takes the items' sums");
 };
 
 // ---------------------------------------------------------------------------
@@ -94,9 +126,23 @@ __device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-// a - b as b * (-1) + a: one rounding, the same value as a subtraction
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(__fdividef(1.0f, a.x), __fdividef(1.0f, a.y)); }
+// (no intrinsic for it; as b * (-1) + a it takes the constant's two registers)
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    union U { float2 f; unsigned long long u; } x, y, d;
+    x.f = a;
+    y.f = b;
+    asm("sub.rn.ftz.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(x.u), "l"(y.u));
+    return d.f;
+}
+// 1 / a: __fdividef(1, a) gives the same values and tests for |a| > 2^126 besides
+__device__ __forceinline__ float rcp(float a)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+    return y;
+}
+__device__ __forceinline__ float2 rcp2(float2 a) { return make_float2(rcp(a.x), rcp(a.y)); }
 __device__ __forceinline__ float2 sqrt2(float2 a) { return make_float2(sqrtf(a.x), sqrtf(a.y)); }
 __device__ __forceinline__ float2 rsqrt2(float2 a) { return make_float2(rsqrtf(a.x), rsqrtf(a.y)); }
 
@@ -114,12 +160,6 @@ __device__ __forceinline__ df2 two_sum2(float2 a, float2 b)
     const float2 s = add2(a, b);
     const float2 bb = sub2(s, a);
     return {s, add2(sub2(a, sub2(s, bb)), sub2(b, bb))};
-}
-
-__device__ __forceinline__ df2 df_add_f2(df2 a, float2 b)
-{
-    const df2 s = two_sum2(a.hi, b);
-    return fast_two_sum2(s.hi, add2(s.lo, a.lo));
 }
 
 __device__ __forceinline__ df2 df_add2(df2 a, df2 b)
@@ -151,21 +191,26 @@ __device__ __forceinline__ float max3f(float a, float b, float c)
     return d;
 }
 
-// Twice the generalised minmod of each lane (godunov-core's plm_gradient,
-// restated), th = 2 theta: the median of min(x, y, z), max(x, y, z) and 0 — the
-// minimum when all three are positive, the maximum when all are negative, else
-// 0: min(max(lo, 0), hi) for lo <= hi.
-__device__ __forceinline__ float2 plm_gradient2(float2 th, float2 a, float2 b, float2 c)
+// The generalised minmod of differences a and b and of y = (a + b) / (2 theta)
+// (godunov-core's plm_gradient, restated; over theta): the median of min(a, y, b),
+// max(a, y, b) and 0 — the minimum when all three are positive, the maximum when
+// all are negative, else 0: min(max(lo, 0), hi) for lo <= hi.
+__device__ __forceinline__ float minmod3(float a, float y, float b)
 {
-    const float2 x = mul2(th, sub2(b, a)), y = sub2(c, a), z = mul2(th, sub2(c, b));
-    return make_float2(fminf(fmaxf(min3f(x.x, y.x, z.x), 0.0f), max3f(x.x, y.x, z.x)),
-                       fminf(fmaxf(min3f(x.y, y.y, z.y), 0.0f), max3f(x.y, y.y, z.y)));
+    return fminf(fmaxf(min3f(a, y, b), 0.0f), max3f(a, y, b));
 }
 
 __device__ __forceinline__ float exp2_fast(float x)
 {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__device__ __forceinline__ float log2_fast(float x)
+{
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -282,11 +327,11 @@ __device__ __noinline__ void sink_items_exact(const DevParamsF& P, const Binary<
 // gamma p / rho (Euler alpha), and a face needs tau = K (T_l + T_r) / 2 with
 // K = 1 for the constant model.
 
-// 0.5 K of the alpha model at two faces at these distances from the bodies, an
+// -0.5 K of the alpha model at two faces at these distances from the bodies, an
 // isothermal face's cs2 left out.  1 / a^3 is taken as rsqrt(a^2)^3: the reference's
 // a = |d| + 1e-12 dx (scheme.rs:244) differs from |d| below FP32 resolution
 // unless |d| is under about 1e-7 dx, and at |d| = 0 both give K = 0.
-__device__ __forceinline__ float2 alpha_half_k2(const float2* K, float2 dx1, float2 dx2, float2 dy1, float2 dy2)
+__device__ __forceinline__ float2 alpha_nhalf_k2(const float2* K, float2 dx1, float2 dx2, float2 dy1, float2 dy2)
 {
     const float2 q1 = rsqrt2(fma2(dy1, dy1, mul2(dx1, dx1))), q2 = rsqrt2(fma2(dy2, dy2, mul2(dx2, dx2)));
     const float2 w2 = fma2(K[C_M1], mul2(q1, mul2(q1, q1)), mul2(K[C_M2], mul2(q2, mul2(q2, q2))));
@@ -295,54 +340,55 @@ __device__ __forceinline__ float2 alpha_half_k2(const float2* K, float2 dx1, flo
 
 // Two faces normal to AXIS (intercell_flux, physics.rs:584-607, 776-803, with
 // hydro-iso2d's and hydro-euler's HLLE) from the states reconstructed on
-// either side.  cs2: the isothermal face sound speed; k: half the alpha
-// model's factor (1/2 for a constant viscosity); tn, tt: the sums of the two
+// either side.  cs2: the isothermal face sound speed; k: minus half the alpha
+// model's factor (-1/2 for a constant viscosity); tn, tt: the sums of the two
 // cells' factored stresses; vxs, vys: the sums of their velocities (Euler).
+//
+// With wl + wr = 1, wl = a+ / (a+ - a-) and wd = a- wl the HLLE flux is
+//   F = fl wl + fr wr + (ur - ul) wd,
+// and f = u v + pressure terms, so that the states enter through two products,
+//   F = ul A + ur B + pressure terms, A = vl wl - wd, B = vr wr + wd:
+// 13 packed operations of an isothermal face pair where forming the conserved
+// states and the fluxes on either side takes 22.
 template <int NF, int AXIS>
 __device__ __forceinline__ void faces2(const float2* K, const float2* pl, const float2* pr, float2 cs2, float2 k,
                                        float2 tn, float2 tt, float2 vxs, float2 vys, float2* F)
 {
-    const float2 vl = pl[1 + AXIS], vr = pr[1 + AXIS];
-    // conserved states and physical fluxes
-    float2 ul[NF], ur[NF], fl[NF], fr[NF], pgl, pgr, csl, csr;
-    ul[0] = pl[0];
-    ur[0] = pr[0];
-    ul[1] = mul2(pl[0], pl[1]); ul[2] = mul2(pl[0], pl[2]);
-    ur[1] = mul2(pr[0], pr[1]); ur[2] = mul2(pr[0], pr[2]);
-    if constexpr (NF == 3) {
-        pgl = mul2(pl[0], cs2);
-        pgr = mul2(pr[0], cs2);
-        csl = csr = sqrt2(cs2);
-    } else {
-        pgl = pl[3];
-        pgr = pr[3];
+    constexpr int VN = 1 + AXIS, VT = 2 - AXIS;
+    const float2 vl = pl[VN], vr = pr[VN];
+    float2 csl, csr;
+    if constexpr (NF == 3) csl = csr = sqrt2(cs2);
+    else {
         csl = sqrt2(mul2(mul2(K[C_GAMMA], pl[3]), rcp2(pl[0])));
         csr = sqrt2(mul2(mul2(K[C_GAMMA], pr[3]), rcp2(pr[0])));
-        ul[3] = fma2(K[C_HALF], fma2(ul[1], pl[1], mul2(ul[2], pl[2])), mul2(pl[3], K[C_INV_GM1]));
-        ur[3] = fma2(K[C_HALF], fma2(ur[1], pr[1], mul2(ur[2], pr[2])), mul2(pr[3], K[C_INV_GM1]));
-        fl[3] = mul2(add2(ul[3], pl[3]), vl);
-        fr[3] = mul2(add2(ur[3], pr[3]), vr);
     }
-    fl[0] = mul2(pl[0], vl);
-    fr[0] = mul2(pr[0], vr);
-    fl[1] = AXIS == 0 ? fma2(ul[1], vl, pgl) : mul2(ul[1], vl);
-    fr[1] = AXIS == 0 ? fma2(ur[1], vr, pgr) : mul2(ur[1], vr);
-    fl[2] = AXIS == 1 ? fma2(ul[2], vl, pgl) : mul2(ul[2], vl);
-    fr[2] = AXIS == 1 ? fma2(ur[2], vr, pgr) : mul2(ur[2], vr);
     // outer wave speeds
     const float2 alm = sub2(vl, csl), alp = add2(vl, csl), arm = sub2(vr, csr), arp = add2(vr, csr);
     const float2 ap = make_float2(max3f(alp.x, arp.x, 0.0f), max3f(alp.y, arp.y, 0.0f));
     const float2 am = make_float2(min3f(alm.x, arm.x, 0.0f), min3f(alm.y, arm.y, 0.0f));
-    const float2 inv = rcp2(sub2(ap, am));
-    // F = (fl ap - fr am + (ur - ul) ap am) / (ap - am), with wl + wr = 1
-    const float2 wl = mul2(ap, inv), wr = sub2(K[C_ONE], wl), wd = mul2(am, wl);
-#pragma unroll
-    for (int f = 0; f < NF; ++f) F[f] = fma2(sub2(ur[f], ul[f]), wd, fma2(fr[f], wr, mul2(fl[f], wl)));
-    const float2 tau_n = mul2(k, tn), tau_t = mul2(k, tt);
-    const float2 tx = AXIS == 0 ? tau_n : tau_t, ty = AXIS == 0 ? tau_t : tau_n;
-    F[1] = sub2(F[1], tx);
-    F[2] = sub2(F[2], ty);
-    if constexpr (NF == 4) F[3] = sub2(F[3], mul2(K[C_HALF], fma2(tx, vxs, mul2(ty, vys))));
+    const float2 wl = mul2(ap, rcp2(sub2(ap, am))), wr = sub2(K[C_ONE], wl), wd = mul2(am, wl);
+    const float2 ql = mul2(vl, wl), qr = mul2(vr, wr);
+    const float2 A = sub2(ql, wd), B = add2(qr, wd);
+    const float2 ml = mul2(pl[0], A), mr = mul2(pr[0], B);
+    F[0] = add2(ml, mr);
+    F[VT] = fma2(ml, pl[VT], mul2(mr, pr[VT]));
+    F[VN] = fma2(ml, vl, mul2(mr, vr));
+    if constexpr (NF == 3) {
+        F[VN] = fma2(cs2, fma2(pl[0], wl, mul2(pr[0], wr)), F[VN]);
+        F[VN] = fma2(k, tn, F[VN]);
+        F[VT] = fma2(k, tt, F[VT]);
+    } else {
+        F[VN] = fma2(pl[3], wl, fma2(pr[3], wr, F[VN]));
+        // energy: E = rho v^2 / 2 + p / (gamma - 1)
+        const float2 el = mul2(K[C_HALF], fma2(pl[1], pl[1], mul2(pl[2], pl[2])));
+        const float2 er = mul2(K[C_HALF], fma2(pr[1], pr[1], mul2(pr[2], pr[2])));
+        F[3] = fma2(pl[3], fma2(A, K[C_INV_GM1], ql), mul2(ml, el));
+        F[3] = fma2(pr[3], fma2(B, K[C_INV_GM1], qr), fma2(mr, er, F[3]));
+        const float2 sn = mul2(k, tn), st = mul2(k, tt);
+        F[VN] = add2(F[VN], sn);
+        F[VT] = add2(F[VT], st);
+        F[3] = fma2(K[C_HALF], fma2(sn, AXIS == 0 ? vxs : vys, mul2(st, AXIS == 0 ? vys : vxs)), F[3]);
+    }
 }
 
 // Sum K values (a power of two, K <= 32) over the 32 lanes of a warp by
@@ -394,11 +440,11 @@ template <int NF> __device__ __forceinline__ int ledger_word(int m)
 // under the strip the sums over the columns inside it, in the piece's slot of
 // the block's.  Out of line, so that it does not weigh on the row loop's
 // register allocation.
-template <int NF, int STORE>
+template <int NF, int STORE, int COPY>
 __device__ __noinline__ void flush_strip(const RunDev& rd, int stage, int strip, int ti, int brow, const float* sums,
-                                         const float* led, bool sinks, bool fake)
+                                         const float2* led, bool sinks, bool fake)
 {
-    using T = SWShape<NF, STORE>;
+    using T = SWShape<NF, STORE, COPY>;
     constexpr int NL = NITEMS * NF, K = NF == 3 ? 16 : 32;
     const int lane = threadIdx.x & 31;
     const int N = rd.N, bs = rd.bs;
@@ -413,7 +459,7 @@ __device__ __noinline__ void flush_strip(const RunDev& rd, int stage, int strip,
             const bool on = m < T::SINKS_AT || (m < (NF == 3 ? T::FAKE_AT : T::ITEMS) ? sinks : m < T::ITEMS && fake);
             v[m] = 0.0f;
             if (on) {
-                const float2 q = *(const float2*)((m < T::SINKS_AT ? sums + m * 64 : led + (m - T::SINKS_AT) * 64) + 2 * lane);
+                const float2 q = m < T::SINKS_AT ? *(const float2*)(sums + m * 64 + 2 * lane) : led[m - T::SINKS_AT];
                 v[m] = (inx ? q.x : 0.0f) + (iny ? q.y : 0.0f);
             }
         }
@@ -437,7 +483,15 @@ __device__ __forceinline__ const DevParamsF& params_for(const StageArgs& a, cons
 // Asynchronous copy of BYTES bytes (4, 8 or 16, aligned to it) from global to shared memory.
 template <int BYTES> __device__ __forceinline__ void copy_async(void* dst, const void* src)
 {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(BYTES) : "memory");
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_addr(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+// row + 16 place bytes, in one instruction
+__device__ __forceinline__ const void* chunk_at(const void* row, unsigned place)
+{
+    unsigned long long p;
+    asm("mad.wide.u32 %0, %1, 16, %2;" : "=l"(p) : "r"(place), "l"(row));
+    return (const void*)p;
 }
 __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING> __device__ __forceinline__ void copy_wait()
@@ -448,18 +502,18 @@ template <int PENDING> __device__ __forceinline__ void copy_wait()
 // A staged pair, and the pairs of all fields at the stencil's precision (an
 // FP64 state's by integer operations: the FP64 pipe converts two lanes a clock).
 __device__ __forceinline__ float2 pair_of(const float* p) { return *(const float2*)p; }
-template <int NF> __device__ __forceinline__ void pairs_of(const float* p, float2* u)
+template <int NF, int PITCH> __device__ __forceinline__ void pairs_of(const float* p, float2* u)
 {
 #pragma unroll
-    for (int f = 0; f < NF; ++f) u[f] = pair_of(p + f * 64);
+    for (int f = 0; f < NF; ++f) u[f] = pair_of(p + f * PITCH);
 }
-template <int NF> __device__ __forceinline__ void pairs_of(const double* p, float2* u)
+template <int NF, int PITCH> __device__ __forceinline__ void pairs_of(const double* p, float2* u)
 {
     double2 v[NF];
     bool ok = true;
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
-        v[f] = *(const double2*)(p + f * 64);
+        v[f] = *(const double2*)(p + f * PITCH);
         ok = ok && split_range(v[f].x) && split_range(v[f].y);
     }
     if (ok) {
@@ -472,11 +526,11 @@ template <int NF> __device__ __forceinline__ void pairs_of(const double* p, floa
 }
 
 // ---------------------------------------------------------------------------
-// EVEN: the mesh has an even number of columns, so that a pair is one aligned word.
-template <int NF, int STORE, bool SINGLE, bool EVEN>
-__global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_constant__ StageArgs a)
+template <int NF, int STORE, bool SINGLE, int COPY>
+__global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_kernel(const __grid_constant__ StageArgs a)
 {
-    using T = SWShape<NF, STORE>;
+    using T = SWShape<NF, STORE, COPY>;
+    constexpr bool EVEN = COPY != COPY_WORDS;               // a pair of columns is one aligned word
     using E = typename T::E;
     const int lane = threadIdx.x;
 
@@ -484,34 +538,42 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
     const int ri = SINGLE ? 0 : find_run(a, g);
     const RunDev& rd = a.runs[ri];
 
-    __shared__ DevParamsF Psh;
-    const DevParamsF& P = params_for<SINGLE>(a, Psh);
-    __shared__ Binary<float> B;
-    __shared__ float2 K[C_COUNT];
-    if (!SINGLE && lane == 10) Psh = rd.pf;
     extern __shared__ __align__(128) unsigned char smem_raw[];   // one declaration for every stage kernel
     poison_dynamic_smem(smem_raw);
-    __shared__ float B_lo[10];
+    unsigned smem_base = smem_addr(smem_raw);
+    asm volatile("" : "+r"(smem_base));
+    unsigned char* smem = (unsigned char*)__cvta_shared_to_generic(smem_base);
+    __builtin_assume(__isShared(smem));
+    typename T::Tables& S = *(typename T::Tables*)smem;
+    const DevParamsF& P = params_for<SINGLE>(a, S.P);
+    const Binary<float>& B = S.B;
+    const float2* K = S.K;
+    const float* B_lo = S.B_lo;
+    if (!SINGLE)
+        for (int k = lane; k < (int)(sizeof(DevParamsF) / 4); k += 32) ((unsigned*)&S.P)[k] = ((const unsigned*)&rd.pf)[k];
     if (lane < 10) {
         const double o = rd.orbit[a.stage * 10 + lane];
         const float hi = (float)o;
-        ((float*)&B)[lane] = hi;
-        B_lo[lane] = (float)(o - (double)hi);
+        ((float*)&S.B)[lane] = hi;
+        S.B_lo[lane] = (float)(o - (double)hi);
     }
     if (*(volatile unsigned long long*)a.err_key != ~0ull) return;   // an earlier stage failed: the advance is abandoned
     __syncwarp();
     const float dt = (float)*rd.dt;
     const float time = (float)rd.stage_time[a.stage];
+    const float itheta2 = P.plm != 0.0f ? __fdividef(0.5f, P.plm) : 0.0f;
     if (lane == 0) {
+        float2* K = S.K;
         const float visc = P.visc == 0 ? P.nu : (NF == 3 ? 1.0f : P.gamma), log2e = 1.4426950408889634f;
-        K[C_THETA2] = f2(2.0f * P.plm);
-        K[C_QUARTER] = f2(0.25f);
-        K[C_NQUARTER] = f2(-0.25f);
+        K[C_ITHETA2] = f2(itheta2);
+        K[C_EDGE] = f2(0.5f * P.plm);
+        K[C_NEDGE] = f2(-0.5f * P.plm);
+        K[C_NHALF] = f2(-0.5f);
         K[C_HALF] = f2(0.5f);
         K[C_ONE] = f2(1.0f);
         K[C_TN] = f2(4.0f / 3.0f + P.lambda);
         K[C_TT] = f2(-2.0f / 3.0f + P.lambda);
-        K[C_VISC] = f2(__fmul_rn(__fmul_rn(0.5f, visc), P.inv_dx));
+        K[C_VISC] = f2(__fmul_rn(__fmul_rn(P.plm, visc), P.inv_dx));
         K[C_CM1] = f2(__fmul_rn(B.p1.m, P.inv_mach2));
         K[C_CM2] = f2(__fmul_rn(B.p2.m, P.inv_mach2));
         K[C_M1] = f2(B.p1.m);
@@ -527,7 +589,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
         K[C_GM1] = f2(P.gm1);
         K[C_INV_GM1] = f2(P.inv_gm1);
         K[C_COOL] = f2(__fmul_rn(-dt, P.inv_cool_beta));
-        K[C_ALPHA] = f2(__fmul_rn(__fmul_rn(0.5f, P.nu), P.inv_sqrt_gm));
+        K[C_ALPHA] = f2(__fmul_rn(__fmul_rn(-0.5f, P.nu), P.inv_sqrt_gm));
     }
     __syncwarp();
 
@@ -546,56 +608,98 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
     const E* ubase = has_base ? (const E*)rd.slot[a.base_slot] : nullptr;
     const E* ubg = (const E*)rd.bg;
 
-    E* stencil = (E*)smem_raw;                              // [SW_SLOTS][NF][64]: this lane's pair at 2 lane
+    E* stencil = (E*)(smem + T::TABLES);                              // [SW_SLOTS][NF][64]: this lane's pair at 2 lane
     E* update = stencil + SW_SLOTS * T::STENCIL;            // [SW_USLOTS][NU][64]
-    float* led = (float*)(update + SW_USLOTS * T::UPDATE);  // [ITEMS - SINKS_AT][64]
-    E* my_stencil = stencil + 2 * lane;
-    E* my_update = update + 2 * lane;
+    float2 led[T::ITEMS - T::SINKS_AT];                     // the items that few warps have: local memory
+    E* my_stencil = stencil + T::S_FIRST + 2 * lane;        // this lane's pair
+    E* my_update = update + T::U_FIRST + 2 * lane;
 
     // ---- row staging -------------------------------------------------------------
     constexpr int PARTS = STORE == 1 ? 2 : 1;               // planes per field: hi and lo words
     const int colx = ((j0 + c0) % N + N) % N, coly = colx + 1 == N ? 0 : colx + 1;   // this lane's columns in the mesh
+    const unsigned bx = colx * (unsigned)sizeof(E), by = coly * (unsigned)sizeof(E);
     auto copy_pair = [&](E* dst, const E* row) {
-        if constexpr (EVEN) copy_async<2 * sizeof(E)>(dst, row + colx);
+        if constexpr (EVEN) copy_async<2 * sizeof(E)>(dst, (const char*)row + bx);
         else {
-            copy_async<sizeof(E)>(dst, row + colx);
-            copy_async<sizeof(E)>(dst + 1, row + coly);
+            copy_async<sizeof(E)>(dst, (const char*)row + bx);
+            copy_async<sizeof(E)>(dst + 1, (const char*)row + by);
         }
+    };
+    // Quads: lane l copies the chunks of four columns l, l + 32, ... of a row's planes of one kind,
+    // 17 a plane of the stencil, 15 of the update; their places from the row's start, in chunks.
+    constexpr int CHUNKS_S = 17 * NF, CHUNKS_U = 15 * NF;
+    unsigned quad_s[(CHUNKS_S + 31) / 32], quad_u[(CHUNKS_U + 31) / 32];
+    if constexpr (COPY == COPY_QUADS) {
+#pragma unroll
+        for (int k = 0; 32 * k < CHUNKS_S; ++k) {
+            const int c = min(lane + 32 * k, CHUNKS_S - 1), col = ((j0 - 4 + 4 * (c % 17)) % N + N) % N;
+            quad_s[k] = (unsigned)((PARTS * (c / 17) * nn + col) / 4);
+        }
+#pragma unroll
+        for (int k = 0; 32 * k < CHUNKS_U; ++k) {
+            const int c = min(lane + 32 * k, CHUNKS_U - 1), col = min(j0 + 4 * (c % 15), N - 4);
+            quad_u[k] = (unsigned)((PARTS * (c / 15) * nn + col) / 4);
+        }
+    }
+    // (the last lanes repeat the last chunk: a branch costs more)
+    const int last_s = 4 * (min(lane + CHUNKS_S / 32 * 32, CHUNKS_S - 1)), last_u = 4 * (min(lane + CHUNKS_U / 32 * 32, CHUNKS_U - 1));
+    auto copy_quads_s = [&](E* dst, const E* row) {
+#pragma unroll
+        for (int k = 0; 32 * k < CHUNKS_S; ++k)
+            copy_async<16>(dst + (32 * k + 32 <= CHUNKS_S ? 4 * lane + 128 * k : last_s), chunk_at(row, quad_s[k]));
+    };
+    auto copy_quads_u = [&](E* dst, const E* row) {
+#pragma unroll
+        for (int k = 0; 32 * k < CHUNKS_U; ++k)
+            copy_async<16>(dst + (32 * k + 32 <= CHUNKS_U ? 4 * lane + 128 * k : last_u), chunk_at(row, quad_u[k]));
     };
     // row rs of the stencil and row ru of the update, as one group
     int gi = wrap(wrap(i0 - 2, N), N);                      // mesh row of rs (a mesh may be one zone wide)
-    size_t row_s = (size_t)gi * N, row_u = (size_t)i0 * N;
+    const E *row_s = uin + (size_t)gi * N, *row_lo = uin + nn + (size_t)i0 * N, *row_bg = ubg + (size_t)i0 * N;
+    const E *row_b = has_base ? ubase + (size_t)i0 * N : nullptr;
     auto issue = [&](int rs, int ru) {
         if (rs <= TH + 1) {
-            const size_t row = row_s;
+            const E* row = row_s;
             row_s += N;
-            if (++gi == N) { gi = 0; row_s = 0; }
-            E* d = my_stencil + ((rs + 2) & (SW_SLOTS - 1)) * T::STENCIL;
+            if (++gi == N) { gi = 0; row_s = uin; }
+            const int at = ((rs + 2) & (SW_SLOTS - 1)) * T::STENCIL;
+            if constexpr (COPY == COPY_QUADS) copy_quads_s(stencil + at, row);
+            else {
 #pragma unroll
-            for (int f = 0; f < NF; ++f) copy_pair(d + f * 64, uin + (size_t)(PARTS * f) * nn + row);
+                for (int f = 0; f < NF; ++f) copy_pair(my_stencil + at + f * T::S_PITCH, row + (size_t)(PARTS * f) * nn);
+            }
         }
         if (ru >= 0 && ru < TH) {
-            const size_t row = row_u;
-            row_u += N;
-            E* d = my_update + (ru & 1) * T::UPDATE;
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                if constexpr (STORE == 1) copy_pair(d + f * 64, uin + (size_t)(2 * f + 1) * nn + row);
-                copy_pair(d + ((STORE == 1 ? NF : 0) + f) * 64, ubg + (size_t)(PARTS * f) * nn + row);
-            }
-            if (has_base) {
+            const int at = (ru & 1) * T::UPDATE;
+            constexpr int KIND = NF * T::U_PITCH;           // elements of the planes of one kind
+            if constexpr (COPY == COPY_QUADS) {
+                copy_quads_u(update + at, row_lo);
+                copy_quads_u(update + at + KIND, row_bg);
+                if (has_base) {
+                    copy_quads_u(update + at + 2 * KIND, row_b);
+                    copy_quads_u(update + at + 3 * KIND, row_b + nn);
+                }
+            } else {
 #pragma unroll
                 for (int f = 0; f < NF; ++f) {
-                    copy_pair(d + (PARTS * NF + f) * 64, ubase + (size_t)(PARTS * f) * nn + row);
-                    if constexpr (STORE == 1) copy_pair(d + (3 * NF + f) * 64, ubase + (size_t)(2 * f + 1) * nn + row);
+                    E* d = my_update + at + f * T::U_PITCH;
+                    if constexpr (STORE == 1) copy_pair(d, row_lo + (size_t)(2 * f) * nn);
+                    copy_pair(d + (STORE == 1 ? KIND : 0), row_bg + (size_t)(PARTS * f) * nn);
+                    if (has_base) {
+                        copy_pair(d + PARTS * KIND, row_b + (size_t)(PARTS * f) * nn);
+                        if constexpr (STORE == 1) copy_pair(d + 3 * KIND, row_b + (size_t)(2 * f + 1) * nn);
+                    }
                 }
             }
+            row_lo += N;
+            row_bg += N;
+            if (has_base) row_b += N;
         }
         copy_commit();
     };
     issue(-2, -1);
 
-    const float theta2 = 2.0f * P.plm, pdt = P.pdt;
+    const float pdt = P.pdt;
     const df32 w1{a.w1f.hi, a.w1f.lo}, wb{a.bff.hi, a.bff.lo};
     const bool half_avg = a.half_avg != 0;
     const bool want_amax = a.amax_flag != 0, fake_on = NF == 3 && P.fake_rate != 0.0f;
@@ -607,47 +711,44 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
     // in every row).
     auto at = [](int k, int n) { return min(max(k, 0), n); };
     auto from = [](float2 x, float hi, float lo) { return __fadd_rn(__fadd_rn(x.x, -hi), __fadd_rn(x.y, -lo)); };
-    __shared__ float2 dyc1[32], dyc2[32], dyv1[32], dyv2[32], sYc[32];   // of the pair's centres and left faces
     {
         const float2 ya = rd.xcf[at(j0 + c0, N - 1)], yb = rd.xcf[at(j0 + c0 + 1, N - 1)];
         const float2 va = rd.xvf[at(j0 + c0, N)], vb = rd.xvf[at(j0 + c0 + 1, N)];
-        sYc[lane] = make_float2(ya.x, yb.x);
-        dyc1[lane] = make_float2(from(ya, B.p1.y, B_lo[2]), from(yb, B.p1.y, B_lo[2]));
-        dyc2[lane] = make_float2(from(ya, B.p2.y, B_lo[7]), from(yb, B.p2.y, B_lo[7]));
-        dyv1[lane] = make_float2(from(va, B.p1.y, B_lo[2]), from(vb, B.p1.y, B_lo[2]));
-        dyv2[lane] = make_float2(from(va, B.p2.y, B_lo[7]), from(vb, B.p2.y, B_lo[7]));
+        S.yc[lane] = make_float2(ya.x, yb.x);
+        S.dyc1[lane] = make_float2(from(ya, B.p1.y, B_lo[2]), from(yb, B.p1.y, B_lo[2]));
+        S.dyc2[lane] = make_float2(from(ya, B.p2.y, B_lo[7]), from(yb, B.p2.y, B_lo[7]));
+        S.dyv1[lane] = make_float2(from(va, B.p1.y, B_lo[2]), from(vb, B.p1.y, B_lo[2]));
+        S.dyv2[lane] = make_float2(from(va, B.p2.y, B_lo[7]), from(vb, B.p2.y, B_lo[7]));
     }
-    __shared__ float2 rows[5][32];                          // dx1, dx2 and x^2 of zone rows, dx1, dx2 of the faces above
     enum { R_C1, R_C2, R_XX, R_F1, R_F2 };
     auto fill_rows = [&](int first) {
         const float2 xa = rd.xcf[at(i0 + first + lane, N - 1)], fa = rd.xvf[at(i0 + first + lane, N)];
         __syncwarp();
-        rows[R_C1][lane] = f2(from(xa, B.p1.x, B_lo[1]));
-        rows[R_C2][lane] = f2(from(xa, B.p2.x, B_lo[6]));
-        rows[R_XX][lane] = f2(__fmul_rn(xa.x, xa.x));
-        rows[R_F1][lane] = f2(from(fa, B.p1.x, B_lo[1]));
-        rows[R_F2][lane] = f2(from(fa, B.p2.x, B_lo[6]));
+        S.rows[R_C1][lane] = f2(from(xa, B.p1.x, B_lo[1]));
+        S.rows[R_C2][lane] = f2(from(xa, B.p2.x, B_lo[6]));
+        S.rows[R_XX][lane] = f2(__fmul_rn(xa.x, xa.x));
+        S.rows[R_F1][lane] = f2(from(fa, B.p1.x, B_lo[1]));
+        S.rows[R_F2][lane] = f2(from(fa, B.p2.x, B_lo[6]));
         __syncwarp();
     };
     const float near2 = (P.sink_r2 + P.soft2) * 1.0001f;    // the sinks' vote: softened distance, with a margin
-    // dy^2 + s^2 of the pair's left faces and of its centres to either body (isothermal)
-    constexpr int NPART = NF == 3 ? 4 : 1;
-    __shared__ float2 part[NPART][32];
+    constexpr int NPART = T::PARTIALS;
     if constexpr (NF == 3) {
         auto col_part = [&](float2 d) { return fma2(d, d, K[C_SOFT2]); };
-        part[0][lane] = col_part(dyv1[lane]);
-        part[1][lane] = col_part(dyv2[lane]);
-        part[2][lane] = col_part(dyc1[lane]);
-        part[3][lane] = col_part(dyc2[lane]);
+        S.part[0][lane] = col_part(S.dyv1[lane]);
+        S.part[1][lane] = col_part(S.dyv2[lane]);
+        S.part[2][lane] = col_part(S.dyc1[lane]);
+        S.part[3][lane] = col_part(S.dyc2[lane]);
     }
     // cs2 = -phi / M^2 (physics.rs:584-607) with the Plummer potential, of two faces dx1, dx2 from the bodies along x
     auto sound2 = [&](float2 dx1, float2 dx2, int which) {
-        const float2 r1 = rsqrt2(fma2(dx1, dx1, part[which % NPART][lane]));
-        const float2 r2 = rsqrt2(fma2(dx2, dx2, part[(which + 1) % NPART][lane]));
+        const float2 r1 = rsqrt2(fma2(dx1, dx1, S.part[which % NPART][lane]));
+        const float2 r2 = rsqrt2(fma2(dx2, dx2, S.part[(which + 1) % NPART][lane]));
         return fma2(K[C_CM1], r1, mul2(K[C_CM2], r2));
     };
 
-    float2 Pm1[NF], P0[NF];           // primitives of rows g - 1 and g
+    float2 dP[NF], P0[NF];            // primitives of row g, and less those of row g - 1
+    int trigger = 0;                  // rows whose densities are below the trigger: two bits for g - 1, for g and for g + 1
     float2 xl[NF], xtn, xtt;          // row g - 1: state at its lower x faces, stresses
     float2 div[NF];                   // row g - 1's y fluxes' difference less the flux through its upper x faces
     constexpr int NACC = T::SINKS_AT;
@@ -655,7 +756,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
 #pragma unroll
     for (int m = 0; m < NACC; ++m) acc[m] = f2(0.0f);
 #pragma unroll
-    for (int f = 0; f < NF; ++f) Pm1[f] = P0[f] = xl[f] = div[f] = f2(0.0f);
+    for (int f = 0; f < NF; ++f) dP[f] = P0[f] = xl[f] = div[f] = f2(0.0f);
     xtn = xtt = f2(0.0f);
     bool sinks_seen = false, fake_seen = false;
     float amax = 0.0f;
@@ -666,6 +767,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
 
     int next_fill = 0;
     for (int n = -2; n <= TH + 1; ++n) {
+        if constexpr (COPY == COPY_QUADS) __syncwarp();     // a slot is read by other lanes than those that fill it
         issue(n + 1, n - 1);
         const int gr = n - 1;
         if (gr == next_fill) {   // the table holds rows gr - 1 to gr + 30
@@ -678,9 +780,10 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
         float2 pn[NF];
         {
             copy_wait<1>();   // the row's group, and that of the update below
+            if constexpr (COPY == COPY_QUADS) __syncwarp();
             const E* sb = my_stencil + ((n + 2) & (SW_SLOTS - 1)) * T::STENCIL;
             float2 u[NF];
-            pairs_of<NF>(sb, u);
+            pairs_of<NF, T::S_PITCH>(sb, u);
             int ea = 0, eb = 0;
             if constexpr (NF == 3) {
                 if (P.has_density_floor) {
@@ -725,6 +828,11 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
             }
         }
 
+        float2 dn[NF];                                      // rows n less n - 1
+#pragma unroll
+        for (int f = 0; f < NF; ++f) dn[f] = sub2(pn[f], P0[f]);
+        if (pdt > 0.0f) trigger = trigger >> 2 | (pn[0].x < pdt ? 16 : 0) | (pn[0].y < pdt ? 32 : 0);
+
         if (gr >= -1) {
             // ---- slopes and stresses of row g (scheme.rs:216-254) ---------------------
             float lv[NF], rv[NF];                           // columns c0 - 1 and c0 + 2
@@ -737,18 +845,23 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                 if (lane == 0) lv[f] = poison_or(lv[f]);
                 if (lane == 31) rv[f] = poison_or(rv[f]);
             }
-            float2 thx = K[C_THETA2], thy = thx;
-            if (pdt > 0.0f) {   // (densities below 0 fail the advance before their slopes count)
-                thx = make_float2((Pm1[0].x < pdt || P0[0].x < pdt || pn[0].x < pdt) ? 0.0f : theta2,
-                                  (Pm1[0].y < pdt || P0[0].y < pdt || pn[0].y < pdt) ? 0.0f : theta2);
-                thy = make_float2((lv[0] < pdt || P0[0].x < pdt || P0[0].y < pdt) ? 0.0f : theta2,
-                                  (P0[0].x < pdt || P0[0].y < pdt || rv[0] < pdt) ? 0.0f : theta2);
-            }
-            float2 gx[NF], gy[NF];                          // twice the slopes
+            float2 gx[NF], gy[NF];                          // slopes over theta
 #pragma unroll
             for (int f = 0; f < NF; ++f) {
-                gx[f] = plm_gradient2(thx, Pm1[f], P0[f], pn[f]);
-                gy[f] = plm_gradient2(thy, make_float2(lv[f], P0[f].x), P0[f], make_float2(P0[f].y, rv[f]));
+                const float2 y = mul2(K[C_ITHETA2], add2(dP[f], dn[f]));
+                gx[f] = make_float2(minmod3(dP[f].x, y.x, dn[f].x), minmod3(dP[f].y, y.y, dn[f].y));
+                const float a0 = __fadd_rn(P0[f].x, -lv[f]), a1 = __fadd_rn(P0[f].y, -P0[f].x), a2 = __fadd_rn(rv[f], -P0[f].y);
+                const float t = __fmul_rn(itheta2, a1);
+                gy[f] = make_float2(minmod3(a0, fmaf(itheta2, a0, t), a1), minmod3(a1, fmaf(itheta2, a2, t), a2));
+            }
+            if (pdt > 0.0f) {   // (densities below 0 fail the advance before their slopes count)
+                const int below = (trigger | trigger >> 2 | trigger >> 4) & 3, own = trigger >> 2 & 3;
+                const bool yx = own || lv[0] < pdt, yy = own || rv[0] < pdt;
+#pragma unroll
+                for (int f = 0; f < NF; ++f) {
+                    gx[f] = make_float2(below & 1 ? 0.0f : gx[f].x, below & 2 ? 0.0f : gx[f].y);
+                    gy[f] = make_float2(yx ? 0.0f : gy[f].x, yy ? 0.0f : gy[f].y);
+                }
             }
             const float2 cv = mul2(K[C_VISC], P0[NF == 4 && P.visc != 0 ? NF - 1 : 0]);
             const float2 txx = mul2(cv, fma2(K[C_TN], gx[1], mul2(K[C_TT], gy[2])));
@@ -762,21 +875,21 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                     float2 pl[NF], pr[NF];
 #pragma unroll
                     for (int f = 0; f < NF; ++f) {
-                        const float2 e = fma2(gy[f], K[C_QUARTER], P0[f]);
+                        const float2 e = fma2(gy[f], K[C_EDGE], P0[f]);
                         pl[f] = make_float2(__shfl_up_sync(0xffffffffu, e.y, 1), e.x);
-                        pr[f] = fma2(gy[f], K[C_NQUARTER], P0[f]);
+                        pr[f] = fma2(gy[f], K[C_NEDGE], P0[f]);
                     }
                     const float2 tn = add2(make_float2(__shfl_up_sync(0xffffffffu, tyy.y, 1), tyy.x), tyy);
                     const float2 tt = add2(make_float2(__shfl_up_sync(0xffffffffu, txy.y, 1), txy.x), txy);
-                    float2 cs2 = f2(0.0f), k = K[C_HALF], vxs = f2(0.0f), vys = f2(0.0f);
-                    const float2 dx1 = rows[R_C1][rt], dx2 = rows[R_C2][rt];
+                    float2 cs2 = f2(0.0f), k = K[C_NHALF], vxs = f2(0.0f), vys = f2(0.0f);
+                    const float2 dx1 = S.rows[R_C1][rt], dx2 = S.rows[R_C2][rt];
                     if constexpr (NF == 3) cs2 = sound2(dx1, dx2, 0);
                     else {
                         vxs = add2(make_float2(lv[1], P0[1].x), P0[1]);
                         vys = add2(make_float2(lv[2], P0[2].x), P0[2]);
                     }
                     if (P.visc != 0) {
-                        k = alpha_half_k2(K, dx1, dx2, dyv1[lane], dyv2[lane]);
+                        k = alpha_nhalf_k2(K, dx1, dx2, S.dyv1[lane], S.dyv2[lane]);
                         if constexpr (NF == 3) k = mul2(k, cs2);
                     }
                     faces2<NF, 1>(K, pl, pr, cs2, k, tn, tt, vxs, vys, Fy);
@@ -791,16 +904,16 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                 {
                     float2 pr[NF];
 #pragma unroll
-                    for (int f = 0; f < NF; ++f) pr[f] = fma2(gx[f], K[C_NQUARTER], P0[f]);
-                    float2 cs2 = f2(0.0f), k = K[C_HALF], vxs = f2(0.0f), vys = f2(0.0f);
-                    const float2 dx1 = rows[R_F1][rt], dx2 = rows[R_F2][rt];
+                    for (int f = 0; f < NF; ++f) pr[f] = fma2(gx[f], K[C_NEDGE], P0[f]);
+                    float2 cs2 = f2(0.0f), k = K[C_NHALF], vxs = f2(0.0f), vys = f2(0.0f);
+                    const float2 dx1 = S.rows[R_F1][rt], dx2 = S.rows[R_F2][rt];
                     if constexpr (NF == 3) cs2 = sound2(dx1, dx2, 2);
                     else {
-                        vxs = add2(Pm1[1], P0[1]);
-                        vys = add2(Pm1[2], P0[2]);
+                        vxs = add2(P0[1], sub2(P0[1], dP[1]));
+                        vys = add2(P0[2], sub2(P0[2], dP[2]));
                     }
                     if (P.visc != 0) {
-                        k = alpha_half_k2(K, dx1, dx2, dyc1[lane], dyc2[lane]);
+                        k = alpha_nhalf_k2(K, dx1, dx2, S.dyc1[lane], S.dyc2[lane]);
                         if constexpr (NF == 3) k = mul2(k, cs2);
                     }
                     faces2<NF, 0>(K, xl, pr, cs2, k, add2(xtn, txx), add2(xtt, txy), vxs, vys, Fx);
@@ -811,47 +924,60 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                     const bool up_ok = ru >= 0;
                     const E* sb = my_stencil + ((ru + 2) & (SW_SLOTS - 1)) * T::STENCIL;
                     const E* q = my_update + (ru & 1) * T::UPDATE;
-                    const E* qg = q + (STORE == 1 ? NF * 64 : 0);                    // background
-                    const E* qb = qg + NF * 64;                                      // RK base
+                    const E* qg = q + (STORE == 1 ? NF * T::U_PITCH : 0);                    // background
+                    const E* qb = qg + NF * T::U_PITCH;                                      // RK base
                     float2 uc[NF], u0[NF];
-                    pairs_of<NF>(sb, uc);
-                    pairs_of<NF>(qg, u0);
+                    pairs_of<NF, T::S_PITCH>(sb, uc);
+                    pairs_of<NF, T::U_PITCH>(qg, u0);
                     // sources of the pair (Physics::source_terms, physics.rs:423-457;
                     // Isothermal 528-582, Euler 683-774)
-                    float2 tot[NF], it[NACC];
-                    const float2 dx1 = rows[R_C1][rt - 1], dx2 = rows[R_C2][rt - 1];
-                    const float2 dy1 = dyc1[lane], dy2 = dyc2[lane];
+                    float2 tot[NF];
+                    const float2 dx1 = S.rows[R_C1][rt - 1], dx2 = S.rows[R_C2][rt - 1];
+                    const float2 dy1 = S.dyc1[lane], dy2 = S.dyc2[lane];
                     // Plummer accelerations (kepler-two-body, restated): -m d / (d^2 + s^2)^(3/2)
-                    const float2 t1 = fma2(dx1, dx1, NF == 3 ? part[2 % NPART][lane] : fma2(dy1, dy1, K[C_SOFT2]));
-                    const float2 t2 = fma2(dx2, dx2, NF == 3 ? part[3 % NPART][lane] : fma2(dy2, dy2, K[C_SOFT2]));
+                    const float2 t1 = fma2(dx1, dx1, NF == 3 ? S.part[2 % NPART][lane] : fma2(dy1, dy1, K[C_SOFT2]));
+                    const float2 t2 = fma2(dx2, dx2, NF == 3 ? S.part[3 % NPART][lane] : fma2(dy2, dy2, K[C_SOFT2]));
                     const float2 r1 = rsqrt2(t1), r2 = rsqrt2(t2);
                     const float2 r13 = mul2(r1, mul2(r1, r1)), r23 = mul2(r2, mul2(r2, r2));
                     const float2 q1 = mul2(mul2(uc[0], K[C_NM1DT]), r13);
                     const float2 q2 = mul2(mul2(uc[0], K[C_NM2DT]), r23);
                     constexpr int G2 = NF - 1, BU = 2 * (NF - 1);
-                    it[0] = mul2(q1, dx1);
-                    it[1] = mul2(q1, dy1);
-                    it[G2] = mul2(q2, dx2);
-                    it[G2 + 1] = mul2(q2, dy2);
                     // buffer: 0.5 rate (1 + tanh(y)) Omega_outer, y = (r - R) / scale, 1 + tanh(y) = 2 / (1 + exp(-2y))
-                    const float2 yc2 = sYc[lane], rr2 = fma2(yc2, yc2, rows[R_XX][rt - 1]);
+                    const float2 yc2 = S.yc[lane], rr2 = fma2(yc2, yc2, S.rows[R_XX][rt - 1]);
                     const float2 yb = fma2(sqrt2(rr2), K[C_BUF_SLOPE], K[C_BUF_OFFSET]);
                     const float2 den = add2(K[C_ONE], make_float2(exp2_fast(yb.x), exp2_fast(yb.y)));
                     const float2 kb = mul2(K[C_BUF_RATE], rcp2(den));
 #pragma unroll
-                    for (int f = 0; f < NF; ++f) it[BU + f] = mul2(sub2(uc[f], u0[f]), kb);
-                    tot[0] = it[BU];
-                    tot[1] = add2(add2(it[0], it[G2]), it[BU + 1]);
-                    tot[2] = add2(add2(it[1], it[G2 + 1]), it[BU + 2]);
+                    for (int f = 0; f < NF; ++f) {
+                        tot[f] = mul2(sub2(uc[f], u0[f]), kb);
+                        acc[BU + f] = add2(acc[BU + f], tot[f]);
+                    }
+                    if constexpr (NF == 3) {
+                        tot[1] = fma2(q1, dx1, fma2(q2, dx2, tot[1]));
+                        tot[2] = fma2(q1, dy1, fma2(q2, dy2, tot[2]));
+                        acc[0] = fma2(q1, dx1, acc[0]);
+                        acc[1] = fma2(q1, dy1, acc[1]);
+                        acc[G2] = fma2(q2, dx2, acc[G2]);
+                        acc[G2 + 1] = fma2(q2, dy2, acc[G2 + 1]);
+                    }
                     if constexpr (NF == 4) {
                         // primitive velocities and specific internal energy (no floors, physics.rs:696)
                         const float2 ir = rcp2(uc[0]);
                         const float2 vx = mul2(uc[1], ir), vy = mul2(uc[2], ir);
                         const float2 v2 = fma2(vx, vx, mul2(vy, vy));
                         const float2 e0 = mul2(sub2(uc[3], mul2(mul2(K[C_HALF], uc[0]), v2)), ir);
-                        // the work of gravity
-                        it[2] = fma2(it[0], vx, mul2(it[1], vy));
-                        it[5] = fma2(it[3], vx, mul2(it[4], vy));
+                        // gravity and its work
+                        const float2 g1x = mul2(q1, dx1), g1y = mul2(q1, dy1), g2x = mul2(q2, dx2), g2y = mul2(q2, dy2);
+                        const float2 g1e = fma2(g1x, vx, mul2(g1y, vy)), g2e = fma2(g2x, vx, mul2(g2y, vy));
+                        tot[1] = add2(add2(g1x, g2x), tot[1]);
+                        tot[2] = add2(add2(g1y, g2y), tot[2]);
+                        tot[3] = add2(add2(g1e, g2e), tot[3]);
+                        acc[0] = add2(acc[0], g1x);
+                        acc[1] = add2(acc[1], g1y);
+                        acc[2] = add2(acc[2], g1e);
+                        acc[3] = add2(acc[3], g2x);
+                        acc[4] = add2(acc[4], g2y);
+                        acc[5] = add2(acc[5], g2e);
                         // Cooling of the specific internal energy, de = e_cooled - e0 formed directly
                         // (e0 (exp(-c) - 1), e0 ((1 + x)^(-1/3) - 1) through expm1 and log1p): as a
                         // difference of two near-equal energies it loses ~1e-7 / (c or x) of its value.
@@ -868,18 +994,21 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                             else
                                 dec = mul2(e0, expm1_small2(c));
                         } else {
-                            // T^4 law: e -> e (1 + 3 a e^3 dt)^(-1/3), a = coefficient / rho^n x slow start
-                            float d2[2];
-#pragma unroll
-                            for (int s = 0; s < 2; ++s) {
-                                const float rho = s ? uc[0].y : uc[0].x, e = s ? e0.y : e0.x;
-                                float rho_n = 1.0f;
-                                for (int m = 0; m < P.density_index; ++m) rho_n = __fmul_rn(rho_n, rho);
-                                const float ac = __fmul_rn(__fdividef(P.cool_coef, rho_n), slow);
-                                const float z = __fmul_rn(__fmul_rn(__fmul_rn(3.0f, ac), __fmul_rn(__fmul_rn(e, e), e)), dt);
-                                d2[s] = __fmul_rn(e, expm1f(__fmul_rn(log1pf(z), -1.0f / 3.0f)));
-                            }
-                            dec = make_float2(d2[0], d2[1]);
+                            // T^4 law: e -> e (1 + z)^(-1/3), z = 3 a e^3 dt, a = coefficient / rho^n x slow
+                            // start.  With y = (1 + z)^(-1/3), y - 1 = (y^3 - 1) / (y^2 + y + 1) =
+                            // -z / ((1 + z) (y^2 + y + 1)) without cancellation; y from the special
+                            // functions and a Newton step for y^-3 = 1 + z.
+                            float2 rho_n = K[C_ONE];
+                            for (int m = 0; m < P.density_index; ++m) rho_n = mul2(rho_n, uc[0]);
+                            const float2 ac = mul2(f2(__fmul_rn(P.cool_coef, slow)), rcp2(rho_n));
+                            float2 z = mul2(mul2(f2(__fmul_rn(3.0f, dt)), ac), mul2(mul2(e0, e0), e0));
+                            z = make_float2(z.x > 1e30f ? 1e30f : z.x, z.y > 1e30f ? 1e30f : z.y);   // y - 1 = -1
+                            const float2 s = add2(K[C_ONE], z);
+                            float2 y = make_float2(exp2_fast(__fmul_rn(log2_fast(s.x), -1.0f / 3.0f)),
+                                                   exp2_fast(__fmul_rn(log2_fast(s.y), -1.0f / 3.0f)));
+                            y = fma2(mul2(y, f2(1.0f / 3.0f)), sub2(K[C_ONE], mul2(mul2(s, y), mul2(y, y))), y);
+                            const float2 q = mul2(s, fma2(y, add2(y, K[C_ONE]), K[C_ONE]));
+                            dec = mul2(mul2(e0, mul2(z, rcp2(q))), f2(-1.0f));
                         }
                         if (P.has_mach_ceiling) {
                             // e >= 2 e_kinetic / (gamma (gamma - 1) M^2)
@@ -889,16 +1018,16 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                             if (ma != eca) dec.x = ma - e0.x;
                             if (mb != ecb) dec.y = mb - e0.y;
                         }
-                        it[10] = mul2(uc[0], dec);
-                        tot[3] = add2(add2(add2(it[2], it[5]), it[BU + 3]), it[10]);
+                        dec = mul2(uc[0], dec);
+                        acc[10] = add2(acc[10], dec);
+                        tot[3] = add2(tot[3], dec);
                     }
                     // sinks: only where a zone of the warp lies inside a sink radius
                     const bool near = inx && fminf(min3f(t1.x, t2.x, t1.y), t2.y) < near2;
                     if (__any_sync(0xffffffffu, near) && up_ok) {
-                        float* sl = led + 2 * lane;
                         if (!sinks_seen) {
 #pragma unroll
-                            for (int m = 0; m < 2 * NF; ++m) *(float2*)(sl + m * 64) = f2(0.0f);
+                            for (int m = 0; m < 2 * NF; ++m) led[m] = f2(0.0f);
                             sinks_seen = true;
                         }
 #pragma unroll
@@ -912,22 +1041,21 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                                 const float sk = s1[f] + s2[f];
                                 if (side) tot[f].y += sk;
                                 else tot[f].x += sk;
-                                sl[f * 64 + side] += s1[f];
-                                sl[(NF + f) * 64 + side] += s2[f];
+                                (side ? led[f].y : led[f].x) += s1[f];
+                                (side ? led[NF + f].y : led[NF + f].x) += s2[f];
                             }
                         }
                     }
                     // fake mass: u0 rate dt unless Sigma < Sigma_0 threshold
                     if (fake_on && up_ok) {
-                        float* sl = led + (T::FAKE_AT - T::SINKS_AT) * 64 + 2 * lane;
                         const bool offa = uc[0].x < u0[0].x * P.fake_thr, offb = uc[0].y < u0[0].y * P.fake_thr;
 #pragma unroll
                         for (int f = 0; f < 3; ++f) {
                             const float2 fk = mul2(mul2(u0[f], f2(P.fake_rate)), f2(dt));
                             const float2 on = make_float2(offa ? 0.0f : fk.x, offb ? 0.0f : fk.y);
                             tot[f] = add2(tot[f], on);
-                            float2* s = (float2*)(sl + f * 64);
-                            *s = fake_seen ? add2(*s, on) : on;
+                            float2& s = led[T::FAKE_AT - T::SINKS_AT + f];
+                            s = fake_seen ? add2(s, on) : on;
                         }
                         fake_seen = true;
                     }
@@ -937,13 +1065,14 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                         df2 o[NF];
 #pragma unroll
                         for (int f = 0; f < NF; ++f) {
-                            const float2 du = mul2(add2(Fx[f], div[f]), K[C_NDT_DX]);
-                            o[f] = df_add_f2(df2{uc[f], pair_of(q + f * 64)}, add2(du, tot[f]));
+                            const float2 inc = fma2(add2(Fx[f], div[f]), K[C_NDT_DX], tot[f]);
+                            o[f] = two_sum2(uc[f], inc);
+                            o[f].lo = add2(o[f].lo, pair_of(q + f * T::U_PITCH));
                         }
                         if (has_base) {
 #pragma unroll
                             for (int f = 0; f < NF; ++f) {
-                                const df2 b0{pair_of(qb + f * 64), pair_of(qb + (NF + f) * 64)};
+                                const df2 b0{pair_of(qb + f * T::U_PITCH), pair_of(qb + (NF + f) * T::U_PITCH)};
                                 if (half_avg) {
                                     const df2 sm = df_add2(o[f], b0);
                                     o[f] = {mul2(sm.hi, K[C_HALF]), mul2(sm.lo, K[C_HALF])};
@@ -952,6 +1081,9 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                                     o[f] = df_add2(x1, x2);
                                 }
                             }
+                        } else {
+#pragma unroll
+                            for (int f = 0; f < NF; ++f) o[f] = fast_two_sum2(o[f].hi, o[f].lo);
                         }
                         if (up_ok && inx) {
 #pragma unroll
@@ -974,9 +1106,8 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                         double2 o[NF];
 #pragma unroll
                         for (int f = 0; f < NF; ++f) {
-                            const float2 du = mul2(add2(Fx[f], div[f]), K[C_NDT_DX]);
-                            const float2 inc = add2(du, tot[f]);
-                            o[f] = *(const double2*)(sb + f * 64);
+                            const float2 inc = fma2(add2(Fx[f], div[f]), K[C_NDT_DX], tot[f]);
+                            o[f] = *(const double2*)(sb + f * T::S_PITCH);
                             o[f].x += widen(inc.x);
                             o[f].y += widen(inc.y);
                         }
@@ -984,7 +1115,7 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                             const double keep = -a.bf + 1.0;
 #pragma unroll
                             for (int f = 0; f < NF; ++f) {
-                                const double2 b0 = *(const double2*)(qb + f * 64);
+                                const double2 b0 = *(const double2*)(qb + f * T::U_PITCH);
                                 if (half_avg) o[f] = make_double2(halve(o[f].x + b0.x), halve(o[f].y + b0.y));
                                 else o[f] = make_double2(o[f].x * keep + b0.x * a.bf, o[f].y * keep + b0.y * a.bf);
                             }
@@ -1009,8 +1140,6 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                         }
                     }
                     if (up_ok) {
-#pragma unroll
-                        for (int m = 0; m < NACC; ++m) acc[m] = add2(acc[m], it[m]);
                         if (want_amax) {
                             float ua[NF], ub[NF], la[NF], lb[NF];
 #pragma unroll
@@ -1019,30 +1148,34 @@ __global__ void __launch_bounds__(32, SW_CTAS) stagew_kernel(const __grid_consta
                             if (iny) amax = fmaxf(max_speed_f32<NF>(P, ub, lb), amax);
                         }
                         if (ru + 1 == next_flush || ru + 1 == TH) {   // the end of a block row, or of the chunk
+                            if constexpr (COPY == COPY_QUADS) __syncwarp();   // it holds other lanes' columns
                             float* sums = (float*)(update + (ru & 1) * T::UPDATE);   // this row's, which is done with
 #pragma unroll
                             for (int m = 0; m < NACC; ++m) {
                                 *(float2*)(sums + m * 64 + 2 * lane) = acc[m];
                                 acc[m] = f2(0.0f);
                             }
-                            flush_strip<NF, STORE>(rd, a.stage, strip, ti, brow, sums, led, sinks_seen, fake_seen);
+                            flush_strip<NF, STORE, COPY>(rd, a.stage, strip, ti, brow, sums, led, sinks_seen, fake_seen);
                             sinks_seen = fake_seen = false;
                             ++brow;
                             next_flush += bs;
                         }
                         out += N;
+                    } else {
+#pragma unroll
+                        for (int m = 0; m < NACC; ++m) acc[m] = f2(0.0f);   // the row above the chunk's first
                     }
                 }
 #pragma unroll
                 for (int f = 0; f < NF; ++f) div[f] = sub2(dfy[f], Fx[f]);
             }
 #pragma unroll
-            for (int f = 0; f < NF; ++f) xl[f] = fma2(gx[f], K[C_QUARTER], P0[f]);
+            for (int f = 0; f < NF; ++f) xl[f] = fma2(gx[f], K[C_EDGE], P0[f]);
             xtn = txx;
             xtt = txy;
         }
 #pragma unroll
-        for (int f = 0; f < NF; ++f) { Pm1[f] = P0[f]; P0[f] = pn[f]; }
+        for (int f = 0; f < NF; ++f) { dP[f] = dn[f]; P0[f] = pn[f]; }
     }
 
     if (want_amax) {
