@@ -1892,7 +1892,8 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
         if (st != B2D_OK) return st;
     } else {
         // block-aligned chunks: every height that divides the blocks, but not
-        // so many chunks that they queue up behind one another
+        // so many chunks that they queue up behind one another, and none above
+        // one whose chunks take up half the GPU (they would only be longer)
         const long long slots = resident_ctas(ctx);
         int max_bs = 0;
         for (const RunHost& r : ctx->runs) max_bs = std::max(max_bs, r.bs);
@@ -1901,6 +1902,7 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
             if (h < 16 && 2 * h <= max_bs && chunk_ctas(ctx, h) > 2 * slots) continue;
             st = trial(h, 0);
             if (st != B2D_OK) return st;
+            if (2 * chunk_ctas(ctx, h) <= slots) break;
         }
         // chunks that cross block rows and fill whole waves
         const int h = best_h;
