@@ -47,12 +47,12 @@
 // waits 4.4 cycles per instruction and a scheduler has three), not memory (4.0
 // of 6.7 TB/s).  Measured per stage, with the kernels that it took the place of,
 // as this file began, and now:
-//   isothermal 2048^2          127 -> 109 -> 73 us (10 warps a CTA in step over 512 columns)
-//   isothermal 384^2            33 -> 22 -> 13 us
+//   isothermal 2048^2          127 -> 109 -> 72.7 us (10 warps a CTA in step over 512 columns)
+//   isothermal 384^2            33 -> 22 -> 12.6 us
 //   the sweep of 64 runs      1050 -> 690 -> 520 us
-//   Euler 4096^2               650 -> 550 -> 364 us
-//   Euler 768^2                 48 -> 42 -> 29.5 us
-//   blocks of 50^2, RK3, alpha 163 -> 25 -> 13.4 us (a thread per column of a block)
+//   Euler 4096^2               650 -> 550 -> 362 us
+//   Euler 768^2                 48 -> 42 -> 28.7 us
+//   blocks of 50^2, RK3, alpha 163 -> 25 -> 12.7 us (a thread per column of a block)
 //   FP64 state 1024^2          106 -> 94 -> 40 us
 // Of this, forming FP32 pairs of FP64 words and widening increments with integer
 // instructions gave the FP64 state 47 us where the FP64 pipe's conversions take 50
@@ -61,7 +61,9 @@
 // programmatic dependent launch (768^2: 47 against 40 us); 16 warps per SM with
 // 128 registers (85 against 78 us: more instructions, and four warps share what
 // three nearly fill); pairs carried from row to row as 64-bit values (76 against
-// 73 us: more moves).
+// 73 us: more moves); the row loop unrolled twice again, now without spills (76
+// to 78 us: 5 % fewer instructions, but waits for instructions nearly double);
+// the first rows converted before the loop, or requested four at once (75 to 76).
 #pragma once
 
 #include "split.cuh"
@@ -549,50 +551,6 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
     const Binary<float>& B = S.B;
     const float2* K = S.K;
     const float* B_lo = S.B_lo;
-    if (!SINGLE)
-        for (int k = lane; k < (int)(sizeof(DevParamsF) / 4); k += 32) ((unsigned*)&S.P)[k] = ((const unsigned*)&rd.pf)[k];
-    if (lane < 10) {
-        const double o = rd.orbit[a.stage * 10 + lane];
-        const float hi = (float)o;
-        ((float*)&S.B)[lane] = hi;
-        S.B_lo[lane] = (float)(o - (double)hi);
-    }
-    if (*(volatile unsigned long long*)a.err_key != ~0ull) return;   // an earlier stage failed: the advance is abandoned
-    __syncwarp();
-    const float dt = (float)*rd.dt;
-    const float time = (float)rd.stage_time[a.stage];
-    const float itheta2 = P.plm != 0.0f ? __fdividef(0.5f, P.plm) : 0.0f;
-    if (lane == 0) {
-        float2* K = S.K;
-        const float visc = P.visc == 0 ? P.nu : (NF == 3 ? 1.0f : P.gamma), log2e = 1.4426950408889634f;
-        K[C_ITHETA2] = f2(itheta2);
-        K[C_EDGE] = f2(0.5f * P.plm);
-        K[C_NEDGE] = f2(-0.5f * P.plm);
-        K[C_NHALF] = f2(-0.5f);
-        K[C_HALF] = f2(0.5f);
-        K[C_ONE] = f2(1.0f);
-        K[C_TN] = f2(4.0f / 3.0f + P.lambda);
-        K[C_TT] = f2(-2.0f / 3.0f + P.lambda);
-        K[C_VISC] = f2(__fmul_rn(__fmul_rn(P.plm, visc), P.inv_dx));
-        K[C_CM1] = f2(__fmul_rn(B.p1.m, P.inv_mach2));
-        K[C_CM2] = f2(__fmul_rn(B.p2.m, P.inv_mach2));
-        K[C_M1] = f2(B.p1.m);
-        K[C_M2] = f2(B.p2.m);
-        K[C_NM1DT] = f2(__fmul_rn(-B.p1.m, dt));
-        K[C_NM2DT] = f2(__fmul_rn(-B.p2.m, dt));
-        K[C_SOFT2] = f2(P.soft2);
-        K[C_BUF_SLOPE] = f2(__fmul_rn(-2.0f * P.inv_buffer_scale, log2e));
-        K[C_BUF_OFFSET] = f2(__fmul_rn(__fmul_rn(2.0f * P.inv_buffer_scale, log2e), P.domain_radius));
-        K[C_BUF_RATE] = f2(__fmul_rn(-2.0f * dt, P.half_rate_omega));
-        K[C_NDT_DX] = f2(__fmul_rn(-P.inv_dx, dt));
-        K[C_GAMMA] = f2(P.gamma);
-        K[C_GM1] = f2(P.gm1);
-        K[C_INV_GM1] = f2(P.inv_gm1);
-        K[C_COOL] = f2(__fmul_rn(-dt, P.inv_cool_beta));
-        K[C_ALPHA] = f2(__fmul_rn(__fmul_rn(-0.5f, P.nu), P.inv_sqrt_gm));
-    }
-    __syncwarp();
-
     const int N = rd.N, bs = rd.bs;
     const size_t nn = (size_t)N * N;
     // rows [i0, i0 + TH) of the strip from column j0: row chunk ti of C (chunk_start, runtime.cuh)
@@ -699,6 +657,59 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
     };
     issue(-2, -1);
 
+    // What else comes from memory, the first row already on its way, is asked for before any
+    // of it is used: on a small mesh a stage is little more than these latencies.
+    auto at = [](int k, int n) { return min(max(k, 0), n); };
+    const float2 ya = rd.xcf[at(j0 + c0, N - 1)], yb = rd.xcf[at(j0 + c0 + 1, N - 1)];
+    const float2 va = rd.xvf[at(j0 + c0, N)], vb = rd.xvf[at(j0 + c0 + 1, N)];
+    const float2 row_x = rd.xcf[at(i0 - 1 + lane, N - 1)], row_f = rd.xvf[at(i0 - 1 + lane, N)];
+    if (!SINGLE)
+        for (int k = lane; k < (int)(sizeof(DevParamsF) / 4); k += 32) ((unsigned*)&S.P)[k] = ((const unsigned*)&rd.pf)[k];
+    if (lane < 10) {
+        const double o = rd.orbit[a.stage * 10 + lane];
+        const float hi = (float)o;
+        ((float*)&S.B)[lane] = hi;
+        S.B_lo[lane] = (float)(o - (double)hi);
+    }
+    if (*(volatile unsigned long long*)a.err_key != ~0ull) {   // an earlier stage failed: the advance is abandoned
+        copy_wait<0>();
+        return;
+    }
+    __syncwarp();
+    const float dt = (float)*rd.dt;
+    const float time = (float)rd.stage_time[a.stage];
+    const float itheta2 = P.plm != 0.0f ? __fdividef(0.5f, P.plm) : 0.0f;
+    if (lane == 0) {
+        float2* K = S.K;
+        const float visc = P.visc == 0 ? P.nu : (NF == 3 ? 1.0f : P.gamma), log2e = 1.4426950408889634f;
+        K[C_ITHETA2] = f2(itheta2);
+        K[C_EDGE] = f2(0.5f * P.plm);
+        K[C_NEDGE] = f2(-0.5f * P.plm);
+        K[C_NHALF] = f2(-0.5f);
+        K[C_HALF] = f2(0.5f);
+        K[C_ONE] = f2(1.0f);
+        K[C_TN] = f2(4.0f / 3.0f + P.lambda);
+        K[C_TT] = f2(-2.0f / 3.0f + P.lambda);
+        K[C_VISC] = f2(__fmul_rn(__fmul_rn(P.plm, visc), P.inv_dx));
+        K[C_CM1] = f2(__fmul_rn(B.p1.m, P.inv_mach2));
+        K[C_CM2] = f2(__fmul_rn(B.p2.m, P.inv_mach2));
+        K[C_M1] = f2(B.p1.m);
+        K[C_M2] = f2(B.p2.m);
+        K[C_NM1DT] = f2(__fmul_rn(-B.p1.m, dt));
+        K[C_NM2DT] = f2(__fmul_rn(-B.p2.m, dt));
+        K[C_SOFT2] = f2(P.soft2);
+        K[C_BUF_SLOPE] = f2(__fmul_rn(-2.0f * P.inv_buffer_scale, log2e));
+        K[C_BUF_OFFSET] = f2(__fmul_rn(__fmul_rn(2.0f * P.inv_buffer_scale, log2e), P.domain_radius));
+        K[C_BUF_RATE] = f2(__fmul_rn(-2.0f * dt, P.half_rate_omega));
+        K[C_NDT_DX] = f2(__fmul_rn(-P.inv_dx, dt));
+        K[C_GAMMA] = f2(P.gamma);
+        K[C_GM1] = f2(P.gm1);
+        K[C_INV_GM1] = f2(P.inv_gm1);
+        K[C_COOL] = f2(__fmul_rn(-dt, P.inv_cool_beta));
+        K[C_ALPHA] = f2(__fmul_rn(__fmul_rn(-0.5f, P.nu), P.inv_sqrt_gm));
+    }
+    __syncwarp();
+
     const float pdt = P.pdt;
     const df32 w1{a.w1f.hi, a.w1f.lo}, wb{a.bff.hi, a.bff.lo};
     const bool half_avg = a.half_avg != 0;
@@ -709,20 +720,14 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
     // FP32 positions is off by 1e-6), as tables: per lane along y, in shared memory since registers
     // are scarce, and per row along x, 31 rows at a time (loads in the row loop would be waited for
     // in every row).
-    auto at = [](int k, int n) { return min(max(k, 0), n); };
     auto from = [](float2 x, float hi, float lo) { return __fadd_rn(__fadd_rn(x.x, -hi), __fadd_rn(x.y, -lo)); };
-    {
-        const float2 ya = rd.xcf[at(j0 + c0, N - 1)], yb = rd.xcf[at(j0 + c0 + 1, N - 1)];
-        const float2 va = rd.xvf[at(j0 + c0, N)], vb = rd.xvf[at(j0 + c0 + 1, N)];
-        S.yc[lane] = make_float2(ya.x, yb.x);
-        S.dyc1[lane] = make_float2(from(ya, B.p1.y, B_lo[2]), from(yb, B.p1.y, B_lo[2]));
-        S.dyc2[lane] = make_float2(from(ya, B.p2.y, B_lo[7]), from(yb, B.p2.y, B_lo[7]));
-        S.dyv1[lane] = make_float2(from(va, B.p1.y, B_lo[2]), from(vb, B.p1.y, B_lo[2]));
-        S.dyv2[lane] = make_float2(from(va, B.p2.y, B_lo[7]), from(vb, B.p2.y, B_lo[7]));
-    }
+    S.yc[lane] = make_float2(ya.x, yb.x);
+    S.dyc1[lane] = make_float2(from(ya, B.p1.y, B_lo[2]), from(yb, B.p1.y, B_lo[2]));
+    S.dyc2[lane] = make_float2(from(ya, B.p2.y, B_lo[7]), from(yb, B.p2.y, B_lo[7]));
+    S.dyv1[lane] = make_float2(from(va, B.p1.y, B_lo[2]), from(vb, B.p1.y, B_lo[2]));
+    S.dyv2[lane] = make_float2(from(va, B.p2.y, B_lo[7]), from(vb, B.p2.y, B_lo[7]));
     enum { R_C1, R_C2, R_XX, R_F1, R_F2 };
-    auto fill_rows = [&](int first) {
-        const float2 xa = rd.xcf[at(i0 + first + lane, N - 1)], fa = rd.xvf[at(i0 + first + lane, N)];
+    auto fill_rows = [&](float2 xa, float2 fa) {            // centres of 32 rows and faces below them, one each
         __syncwarp();
         S.rows[R_C1][lane] = f2(from(xa, B.p1.x, B_lo[1]));
         S.rows[R_C2][lane] = f2(from(xa, B.p2.x, B_lo[6]));
@@ -731,6 +736,7 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
         S.rows[R_F2][lane] = f2(from(fa, B.p2.x, B_lo[6]));
         __syncwarp();
     };
+    fill_rows(row_x, row_f);
     const float near2 = (P.sink_r2 + P.soft2) * 1.0001f;    // the sinks' vote: softened distance, with a margin
     constexpr int NPART = T::PARTIALS;
     if constexpr (NF == 3) {
@@ -765,13 +771,13 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
     __builtin_assume(__isGlobal(out));
     out += (size_t)i0 * N + j0 + c0;                        // this pair of row g - 1
 
-    int next_fill = 0;
+    int next_fill = 31;
     for (int n = -2; n <= TH + 1; ++n) {
         if constexpr (COPY == COPY_QUADS) __syncwarp();     // a slot is read by other lanes than those that fill it
         issue(n + 1, n - 1);
         const int gr = n - 1;
         if (gr == next_fill) {   // the table holds rows gr - 1 to gr + 30
-            fill_rows(gr - 1);
+            fill_rows(rd.xcf[at(i0 + gr - 1 + lane, N - 1)], rd.xvf[at(i0 + gr - 1 + lane, N)]);
             next_fill += 31;
         }
         const int rt = gr - (next_fill - 32);               // row g's place in it
