@@ -1097,21 +1097,25 @@ static std::vector<StagePlan> plan_advance(int rk, int fold, int start, int* fin
 // The ledgers of every block over one advance (compute_block_updated_solution,
 // scheme.rs:307-314), after the stage kernels, which only write their pieces
 // of each block's sums: folds and the serial FP64 perturbation stay out of
-// their tails.  Two kernels:
-//  * ledger_fold_kernel — one thread per (stage, block, item): the item's pieces,
-//    in order, to the block's stage sums ds·dx·dy, and for the gas items sink1,
-//    sink2, grav1, grav2 their perturbation (ItemizedChange::perturbation,
-//    state.rs:258-281).  An unbound perturbed orbit fails its stage with
-//    OrbitalEvolutionError, reported at position (0, 0) as in the reference.
-//    The reference converts every block's primitives before it updates any
-//    block, so within a stage a cons->prim failure anywhere wins: the key's
-//    block field is saturated and the failing block's index rides in the
-//    zone field; an earlier stage still wins through the stage field.
-//    Launched once per stage_window stages: once per advance, but for meshes
-//    of very many pieces.
-//  * ledger_sum_kernel — one thread per (block, ledger word or element
-//    component): the stages in order, x_out = x_in + change averaged like the
-//    state (state.rs:191-197), in the slot schedule of plan_advance.
+// their tails.  One CTA per block, in three steps:
+//  * a thread per (stage, ledger word): the word's pieces, in order, to the
+//    block's stage sums ds·dx·dy;
+//  * a thread per (stage, gas item) for sink1, sink2, grav1 and grav2: the
+//    perturbation (ItemizedChange::perturbation, state.rs:258-281).  An unbound
+//    perturbed orbit fails its stage with OrbitalEvolutionError, reported at
+//    position (0, 0) as in the reference.  The reference converts every block's
+//    primitives before it updates any block, so within a stage a cons->prim
+//    failure anywhere wins: the key's block field is saturated and the failing
+//    block's index rides in the zone field; an earlier stage still wins through
+//    the stage field;
+//  * a thread per ledger word or element component: the stages in order,
+//    x_out = x_in + change averaged like the state (state.rs:191-197), in the
+//    slot schedule of plan_advance.
+// Launched once per advance; meshes of very many pieces fold every stage_window
+// stages, and the last launch sums.  It is all latency, at the end of every
+// advance: as a launch of a thread per (stage, block, item) for the first two
+// steps and another for the third an advance of one step of 128^2 took 49 us, with
+// this 40 (a call of it 64 and 53).
 template <int NF> __device__ __forceinline__ void fold_item(const RunDev& rd, int s, int block, int item, double* ds)
 {
     constexpr int NL = NITEMS * NF;
@@ -1126,82 +1130,87 @@ template <int NF> __device__ __forceinline__ void fold_item(const RunDev& rd, in
     for (int f = 0; f < NF; ++f) ds[f] = v[f] * area;
 }
 
-__global__ void ledger_fold_kernel(const RunDev* runs, int first_stage, unsigned long long* err_key)
+__global__ void __launch_bounds__(256) ledger_kernel(const RunDev* runs, int first, int last, bool sum, int fold, int rk,
+                                                     int start, unsigned long long* err_key)
 {
-    const int run = blockIdx.z;
+    const int run = blockIdx.y, block = blockIdx.x;
     const RunDev& rd = runs[run];
-    const int s = first_stage + blockIdx.y;
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;   // block * 8 + item
-    const int block = id >> 3, item = id & 7;
-    if (block >= rd.nblocks || item >= NITEMS) return;
+    if (block >= rd.nblocks) return;
     if (rd.slab_hi > 0 && (block / rd.nb < rd.slab_lo || block / rd.nb >= rd.slab_hi)) return;   // another slab's
-    const int nf = rd.p.hydro == B2D_EULER ? 4 : 3;
-    double* ds = rd.stage_ds + ((size_t)s * rd.nblocks + block) * NITEMS * nf + item * nf;
-    if (nf == 3) fold_item<3>(rd, s, block, item, ds);
-    else fold_item<4>(rd, s, block, item, ds);
-    if (item >= 4) return;
-    const double* orbit = rd.orbit + 10 * s;
-    double* de = rd.stage_de + (((size_t)s * rd.nblocks + block) * 4 + item) * 4;
-    // pert1 (body 1: sink1, grav1) and pert2 (body 2: sink2, grav2), state.rs:261-269
-    const bool ok = (item == 0 || item == 2)
-                        ? perturb_elements(orbit, rd.el0, -ds[0], 0.0, -ds[1], 0.0, -ds[2], 0.0, de)
-                        : perturb_elements(orbit, rd.el0, 0.0, -ds[0], 0.0, -ds[1], 0.0, -ds[2], de);
-    if (!ok) {
-        de[0] = de[1] = de[2] = de[3] = 0.0;
-        const unsigned long long key = ((unsigned long long)s << 54) | ((unsigned long long)run << 46) |
-                                       (0xffffull << 30) | (0xfull << 26) | ((unsigned long long)block << 2) | 3ull;
-        atomicMin(err_key, key);
+    const int nf = rd.p.hydro == B2D_EULER ? 4 : 3, nl = NITEMS * nf, pieces = rd.tiles_per_block;
+    const size_t stride = (size_t)rd.nblocks * nl;
+    double* stage_ds = rd.stage_ds + (size_t)block * nl;
+    double* stage_de = rd.stage_de + (size_t)block * 16;
+    const double area = rd.p.dx * rd.p.dx;
+    for (int t = threadIdx.x; t < (last - first) * nl; t += blockDim.x) {
+        const int s = first + t / nl, k = t % nl;
+        const double* p = stage_pieces(rd, s, block, nl) + k;
+        double v = 0.0;
+#pragma unroll 16
+        for (int q = 0; q < pieces; ++q) v += p[q * nl];
+        stage_ds[s * stride + k] = v * area;
     }
-}
-
-__global__ void ledger_sum_kernel(const RunDev* runs, int fold, int rk, int start)
-{
-    const int run = blockIdx.y;
-    const RunDev& rd = runs[run];
-    const int id = blockIdx.x * blockDim.x + threadIdx.x;   // ledger words [block][7 nf], then elements [block][7][4]
-    const int nl = NITEMS * (rd.p.hydro == B2D_EULER ? 4 : 3), words = rd.nblocks * nl;
-    if (id >= words + rd.nblocks * NITEMS * 4) return;
-    const bool elements = id >= words;
-    const int w = elements ? id - words : id;
-    const int block = w / (elements ? NITEMS * 4 : nl), k = w % (elements ? NITEMS * 4 : nl);
-    if (rd.slab_hi > 0 && (block / rd.nb < rd.slab_lo || block / rd.nb >= rd.slab_hi)) return;
-    double* const* slots = elements ? rd.elements : rd.ledger;
-    // the change of each stage; only the gas items perturb the orbit
-    const double* change = elements ? (k < 16 ? rd.stage_de + (size_t)block * 16 + k : nullptr) : rd.stage_ds + (size_t)block * nl + k;
-    const size_t stride = (size_t)rd.nblocks * (elements ? 16 : nl);
-    double e[NSLOTS];
-    e[start] = slots[start][w];
-    int s = 0;
-    auto stage = [&](int in, int base_slot, int out, double bf) {
-        double v = e[in] + (change ? change[s * stride] : 0.0);
-        if (base_slot >= 0) v = v * (-bf + 1.0) + e[base_slot] * bf;
-        e[out] = v;
-        ++s;
-    };
-    // the schedule of plan_advance
-    int base = start;
-    for (int f = 0; f < fold; ++f) {
-        if (rk == 1) {
-            const int a = free_slot(start, base, -1);
-            stage(base, -1, a, 0.0);
-            base = a;
-        } else if (rk == 2) {
-            const int a = free_slot(start, base, -1);
-            stage(base, -1, a, 0.0);
-            const int b = free_slot(start, base, a);
-            stage(a, base, b, 0.5);
-            base = b;
-        } else {
-            const int a = free_slot(start, base, -1);
-            stage(base, -1, a, 0.0);
-            const int b = free_slot(start, base, a);
-            stage(a, base, b, 0.75);
-            const int c = free_slot(start, base, b);
-            stage(b, base, c, 1.0 / 3.0);
-            base = c;
+    __syncthreads();
+    for (int t = threadIdx.x; t < (last - first) * 4; t += blockDim.x) {
+        const int s = first + t / 4, item = t % 4;
+        const double* orbit = rd.orbit + 10 * s;
+        const double* ds = stage_ds + s * stride + item * nf;
+        double* de = stage_de + (size_t)s * rd.nblocks * 16 + item * 4;
+        // pert1 (body 1: sink1, grav1) and pert2 (body 2: sink2, grav2), state.rs:261-269
+        const bool ok = (item == 0 || item == 2)
+                            ? perturb_elements(orbit, rd.el0, -ds[0], 0.0, -ds[1], 0.0, -ds[2], 0.0, de)
+                            : perturb_elements(orbit, rd.el0, 0.0, -ds[0], 0.0, -ds[1], 0.0, -ds[2], de);
+        if (!ok) {
+            de[0] = de[1] = de[2] = de[3] = 0.0;
+            const unsigned long long key = ((unsigned long long)s << 54) | ((unsigned long long)run << 46) |
+                                           (0xffffull << 30) | (0xfull << 26) | ((unsigned long long)block << 2) | 3ull;
+            atomicMin(err_key, key);
         }
     }
-    slots[base][w] = e[base];
+    if (!sum) return;
+    __syncthreads();
+    for (int t = threadIdx.x; t < nl + NITEMS * 4; t += blockDim.x) {   // ledger words [7 nf], then elements [7][4]
+        const bool elements = t >= nl;
+        const int k = elements ? t - nl : t;
+        const size_t w = (size_t)block * (elements ? NITEMS * 4 : nl) + k;
+        double* const* slots = elements ? rd.elements : rd.ledger;
+        // the change of each stage; only the gas items perturb the orbit
+        const double* change = elements ? (k < 16 ? stage_de + k : nullptr) : stage_ds + k;
+        const size_t stage_stride = (size_t)rd.nblocks * (elements ? 16 : nl);
+        double e[NSLOTS];
+        e[start] = slots[start][w];
+        int s = 0;
+        auto stage = [&](int in, int base_slot, int out, double bf) {
+            double v = e[in] + (change ? change[s * stage_stride] : 0.0);
+            if (base_slot >= 0) v = v * (-bf + 1.0) + e[base_slot] * bf;
+            e[out] = v;
+            ++s;
+        };
+        // the schedule of plan_advance
+        int base = start;
+        for (int f = 0; f < fold; ++f) {
+            if (rk == 1) {
+                const int a = free_slot(start, base, -1);
+                stage(base, -1, a, 0.0);
+                base = a;
+            } else if (rk == 2) {
+                const int a = free_slot(start, base, -1);
+                stage(base, -1, a, 0.0);
+                const int b = free_slot(start, base, a);
+                stage(a, base, b, 0.5);
+                base = b;
+            } else {
+                const int a = free_slot(start, base, -1);
+                stage(base, -1, a, 0.0);
+                const int b = free_slot(start, base, a);
+                stage(a, base, b, 0.75);
+                const int c = free_slot(start, base, b);
+                stage(b, base, c, 1.0 / 3.0);
+                base = c;
+            }
+        }
+        slots[base][w] = e[base];
+    }
 }
 
 static int max_blocks(const b2d_ctx* ctx)
@@ -1430,26 +1439,23 @@ static b2d_status launch_tracers(b2d_ctx* ctx, const StagePlan& sp, bool count)
     return B2D_OK;
 }
 
-// Fold the ledger pieces once stage s has filled their buffers, or was the last of nstages.
-static b2d_status launch_fold(b2d_ctx* ctx, int s, int nstages, bool count)
+// Stages [first, last) of the advance's ledgers, and with `sum` the sums over its stages.
+static b2d_status launch_ledgers(b2d_ctx* ctx, int first, int last, bool sum, int fold, int start, bool count)
 {
-    const int first = s / ctx->stage_window * ctx->stage_window;
-    if (s + 1 != nstages && s + 1 != first + ctx->stage_window) return B2D_OK;
-    const dim3 grid((unsigned)((max_blocks(ctx) * 8 + 127) / 128), (unsigned)(s + 1 - first), (unsigned)ctx->nruns);
-    ledger_fold_kernel<<<grid, 128, 0, ctx->stream>>>(ctx->rdev, first, ctx->d_err_key);
+    const int nl = NITEMS * ctx->nf, work = std::max((last - first) * nl, nl + NITEMS * 4);
+    const int threads = std::min((work + 31) / 32 * 32, 256);
+    ledger_kernel<<<dim3((unsigned)max_blocks(ctx), (unsigned)ctx->nruns), threads, 0, ctx->stream>>>(
+        ctx->rdev, first, last, sum, fold, ctx->rk, start, ctx->d_err_key);
     CUDA_TRY(cudaGetLastError());
     if (count) ctx->launches++;
     return B2D_OK;
 }
 
-// The ledgers' sums over an advance's stages, after the last fold.
-static b2d_status launch_ledgers(b2d_ctx* ctx, int fold, int start, bool count)
+// The first of the stages up to s whose pieces are to be folded after it, or -1.
+static int fold_due(const b2d_ctx* ctx, int s, int nstages)
 {
-    const dim3 grid((unsigned)((max_blocks(ctx) * NITEMS * (4 + ctx->nf) + 127) / 128), (unsigned)ctx->nruns);
-    ledger_sum_kernel<<<grid, 128, 0, ctx->stream>>>(ctx->rdev, fold, ctx->rk, start);
-    CUDA_TRY(cudaGetLastError());
-    if (count) ctx->launches++;
-    return B2D_OK;
+    const int first = s / ctx->stage_window * ctx->stage_window;
+    return s + 1 == nstages || s + 1 == first + ctx->stage_window ? first : -1;
 }
 
 static b2d_status enqueue_advance(b2d_ctx* ctx, int fold, int start, int* final_slot, bool count)
@@ -1475,10 +1481,11 @@ static b2d_status enqueue_advance(b2d_ctx* ctx, int fold, int start, int* final_
         if (count) ctx->launches++;
         st = launch_tracers(ctx, plan[s], count);
         if (st != B2D_OK) return st;
-        st = launch_fold(ctx, (int)s, (int)plan.size(), count);
+        const int first = fold_due(ctx, (int)s, (int)plan.size());
+        if (first >= 0) st = launch_ledgers(ctx, first, (int)s + 1, s + 1 == plan.size(), fold, start, count);
         if (st != B2D_OK) return st;
     }
-    return launch_ledgers(ctx, fold, start, count);
+    return B2D_OK;
 }
 
 extern "C" b2d_status b2d_set_tracers(b2d_ctx* ctx, int32_t run, int64_t n, const double* xy)
@@ -1738,7 +1745,7 @@ extern "C" int64_t b2d_launches_per_advance(const b2d_ctx* ctx, int32_t fold)
     int with_tracers = 0;
     for (const RunDev& d : ctx->rdev_h) with_tracers += d.ntracers > 0 ? 1 : 0;
     const int64_t stages = (int64_t)fold * ctx->rk, window = std::min<int64_t>(ctx->stage_window, stages);
-    return 2 + (stages + window - 1) / window + stages * (1 + with_tracers);
+    return 1 + (stages + window - 1) / window + stages * (1 + with_tracers);
 }
 
 extern "C" b2d_status b2d_set_instrument(b2d_ctx* ctx, int32_t enable)
@@ -1998,7 +2005,8 @@ extern "C" b2d_status b2d_slab_stage(b2d_ctx* ctx)
     ctx->launches++;
     st = launch_tracers(ctx, ctx->slab_plan[s], true);
     if (st != B2D_OK) return st;
-    st = launch_fold(ctx, s, (int)ctx->slab_plan.size(), true);
+    const int first = fold_due(ctx, s, (int)ctx->slab_plan.size());
+    if (first >= 0) st = launch_ledgers(ctx, first, s + 1, false, ctx->slab_fold, ctx->slab_start, true);
     if (st != B2D_OK) return st;
     ctx->slab_next++;
     return B2D_OK;
@@ -2008,7 +2016,7 @@ extern "C" b2d_status b2d_slab_end(b2d_ctx* ctx, double* dt_out, b2d_error* err_
 {
     if (!ctx || ctx->slab_next != (int)ctx->slab_plan.size() || ctx->slab_plan.empty())
         return fail(B2D_ERR_INVALID, "the slab advance has stages left to run");
-    b2d_status st = launch_ledgers(ctx, ctx->slab_fold, ctx->slab_start, true);
+    b2d_status st = launch_ledgers(ctx, 0, 0, true, ctx->slab_fold, ctx->slab_start, true);
     ctx->slab_next = -1;
     if (st != B2D_OK) return st;
     return finish_advance(ctx, ctx->slab_final, dt_out, err_out);
