@@ -290,7 +290,7 @@ class Runtime:
 
     def set_strip_rows(self, rows: int = 0):
         """Row chunks of at most `rows` rows, crossing block boundaries, for the
-        paired FP32 kernel (0: block-aligned tiles of the tile height)."""
+        FP32 stage kernel (0: block-aligned chunks of the tile height)."""
         _check(self.lib.b2d_set_strip_rows(self.ctx, int(rows)))
 
     def strip_rows(self) -> int:

@@ -480,8 +480,8 @@ static void split_blocks(RunDev& d, int bs, int th, int tw, int per_cta)
 
 static bool tile_ok(const b2d_ctx* ctx, int tw, int th)
 {
-    // the paired FP32 kernels' 128-, 256- and 512-column tiles may also span
-    // whole blocks side by side (blocks of 64 columns or more)
+    // (a width has no effect on the kernels: the FP64 kernel picks its own sub-tiles, the FP32 kernel's strips
+    // are 60 columns.  128-, 256- and 512-column tiles may also span whole blocks side by side.)
     const bool span = ctx->precision == B2D_PREC_FP32_COMP && (tw == 128 || tw == 256 || tw == 512);
     if (tw < 1 || th < 1 || tw > (span ? 512 : 256)) return false;
     for (const RunHost& r : ctx->runs) {
@@ -2059,7 +2059,7 @@ extern "C" b2d_status b2d_slab_rows(b2d_ctx* ctx, int32_t run, int32_t row0, int
 // embedded runtime.  They hand over every input and
 // output buffer themselves; the scratch the stage kernel needs (its run
 // descriptor, the binary at the stage time, per-tile ledger partials, block
-// counters, the max-speed word and the failure key) lives in the file-scope
+// the max-speed word and the failure key) lives in the file-scope
 // array below, which every GPU that loads this library holds until the
 // process exits.
 constexpr size_t B2D_NOALLOC_SCRATCH_BYTES = 4u << 20;   // 4 MiB
@@ -2136,7 +2136,7 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
         return fail(B2D_ERR_INVALID, "b2d_stage_noalloc: block_size " + std::to_string(bs) +
                                          " must be a multiple of 32 or at most 256");
 
-    // scratch layout: run descriptor | control words | counters | ledger pieces | geometry tables.  A CTA takes
+    // scratch layout: run descriptor | control words | (unused, one word a block) | ledger pieces | geometry tables.  A CTA takes
     // several sub-tiles of a block where one piece per sub-tile would not fit.
     const size_t off_run = 0, off_ctl = 2048, off_cnt = 2304;
     const size_t off_part = off_cnt + ((sizeof(unsigned) * (size_t)nblocks + 255) / 256) * 256;

@@ -72,8 +72,8 @@ def link_bandwidth(torch, host_src, host_dst):
     return out
 
 
-PROFILES = {("disk_2048", "fp32_comp"): "stage3_kernel_fp32comp_disk2048.md",
-            ("euler_4096", "fp32_comp"): "stage3e_kernel_fp32comp_euler4096.md"}
+PROFILES = {("disk_2048", "fp32_comp"): "stagew_kernel_fp32comp_disk2048.md",
+            ("euler_4096", "fp32_comp"): "stagew_kernel_fp32comp_euler4096.md"}
 
 
 def ncu_profile(workload, precision, key):
@@ -655,7 +655,7 @@ def main():
     ap.add_argument("--workload", default="disk_2048")
     ap.add_argument("--tile", default="", help="WxH: fixed tile instead of the autotuner")
     ap.add_argument("--strip-rows", type=int, default=0,
-                    help="with --tile: row chunks across block rows for the paired FP32 kernel (0: off)")
+                    help="with --tile: row chunks across block rows for the FP32 kernel (0: off)")
     ap.add_argument("--sweep-runs", type=int, default=64)
     ap.add_argument("--tracers", type=int, default=-1, help="tracer particles (-1: workload default)")
     ap.add_argument("--cpu-seconds", type=float, default=10.0)
