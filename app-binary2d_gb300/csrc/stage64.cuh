@@ -29,7 +29,8 @@
 //    per zone instead of once per side of each of its four faces.
 //  * The buffer's rate depends on the place only: it is a table of the context.
 //  * A warp evaluates sinks only if one of its zones lies in a sink radius,
-//    and only the upwind state of faces that are all supersonic.
+//    and only the upwind state of faces that are all supersonic, whose flux
+//    times and over the wave speed takes three operations (ThereAndBack).
 //
 // Work decomposition.  A CTA takes sub-tiles of TH x TW zones of one mesh
 // block (at most 16 x 32; blocks are split evenly, so any block size does) and
@@ -40,10 +41,12 @@
 // three (85 registers) or one of 512 threads were 1-19 % slower.
 //
 // Measured per stage, against the marching kernel it took the place of (one
-// thread per column of a block's 64 rows): isothermal 2048^2 10.6 -> 3.2 ms,
-// 384^2 (6 x 6 blocks of 64^2) 2.97 -> 0.14 ms; Euler 256^2 with the T^4 law
-// 3.79 -> 0.13 ms.  At 2048^2 the FP64 pipe is 84 % busy with about 395
-// operations per zone; 2.65 ms would be all of it.
+// thread per column of a block's 64 rows): isothermal 2048^2 10.6 -> 3.15 ms,
+// 384^2 (6 x 6 blocks of 64^2) 2.97 -> 0.131 ms; Euler 256^2 with the T^4 law
+// 3.79 -> 0.119 ms (of which the upwind fluxes' quotients and y loops that begin
+// with the warps that had fewer x faces: 3.18 -> 3.15, 0.134 -> 0.131 and 0.123 ->
+// 0.119 ms).  At 2048^2 the FP64 pipe is 84 % busy with about 395 operations per
+// zone; 2.65 ms would be all of it.
 #pragma once
 
 #include "stage.cuh"
@@ -117,6 +120,31 @@ struct Divisor {
         if (!(ok && moderate(x))) return plain_div(x, d);
         const double q = __dmul_rn(x, r);
         return __fma_rn(__fma_rn(-q, d, x), r, q);
+    }
+};
+
+// (f w) / w, both rounded.  The quotient is f but for the rounding of x = f w:
+// with e = x - f w (exact in a fused step) it is f + e / w, which one fused step
+// rounds.  1 / w to rounding: the 20 bits of the approximate reciprocal and one
+// cubic step, 1 + d + d^2 of the residual d (Householder).  Equal to the two
+// operations in each of 2e8 random pairs; three operations a quotient and three
+// for w in place of four and a division.
+struct ThereAndBack {
+    double w, r;
+    bool ok;
+    __device__ __forceinline__ explicit ThereAndBack(double w_) : w(w_), ok(moderate(w_) && w_ != 0.0)
+    {
+        double r0;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(w));
+        const double d = __fma_rn(-w, r0, 1.0);
+        r = __fma_rn(r0, __fma_rn(d, d, d), r0);
+    }
+    __device__ __forceinline__ double operator()(double f) const
+    {
+        if (!(ok && moderate(f))) return plain_div(f * w, w);
+        const double x = __dmul_rn(f, w);
+        const double q = __fma_rn(__fma_rn(-f, w, x), r, f);
+        return zero(f) ? f : q;   // (the sign of a zero)
     }
 };
 
@@ -249,6 +277,8 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
     const double inv_dx = P.inv_dx;
     const bool const_nu = P.visc == 0, with_bulk = P.lambda != 0.0;
     const double lam_nu = P.lambda * P.nu;
+    // this thread's first item of a loop that follows one of n items: the warps take turns on from its last
+    auto after = [&](int n) { return (t - (n + 31) / 32 * 32 % NT + NT) % NT; };
     const bool trigger = P.pdt > 0.0;      // densities below 0 fail the advance before their slopes count
 
     double acc[K0];                        // this thread's zones' sums of the items that are live everywhere
@@ -357,7 +387,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
                 sDX[f * DXS + e] = trigger ? d : theta * d;
             }
         }
-        for (int e = t; e < DYS; e += NT) {
+        for (int e = after(DXS); e < DYS; e += NT) {
             const int r = e / DW, c = e % DW;
             const int o = (r + 1) * PW + c;
 #pragma unroll
@@ -499,10 +529,9 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
 #pragma unroll
                 for (int k = 0; k < NF; ++k) pu[k] = from_l ? pl[k] : pr[k];
                 side64<NF, AX>(pu, from_l ? pgl : pgr, by_gm1, u, f);
-                const double w = from_l ? ap : am;
-                const Divisor by_w(w);
+                const ThereAndBack through(from_l ? ap : am);
 #pragma unroll
-                for (int k = 0; k < NF; ++k) F[k] = by_w(f[k] * w);
+                for (int k = 0; k < NF; ++k) F[k] = through(f[k]);
             } else {
                 double ul[NF], ur[NF], fl[NF], fr[NF];
                 side64<NF, AX>(pl, pgl, by_gm1, ul, fl);
@@ -528,7 +557,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
             const int rl = r * CW + c + 1, pl = (r + 1) * PW + c + 2;
             face(std::integral_constant<int, 0>(), rl, rl + CW, pl, pl + PW, q[0], q[1], w[0], w[1], sFX + e, FXS);
         }
-        for (int e = t; e < FYS; e += NT) {
+        for (int e = after(FXS); e < FYS; e += NT) {
             const int r = e / FW, c = e % FW;               // face between columns c - 1 and c
             const double* q = gr + 7 * r;
             const double* w = gc + 7 * TW + 5 * c;
