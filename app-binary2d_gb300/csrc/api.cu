@@ -1810,8 +1810,10 @@ extern "C" b2d_status b2d_set_device(int32_t device)
 // Tile autotuner: time every tile shape that divides the block size with CUDA
 // events on the context's stream, keep the fastest.  The advances run from
 // the current slot, which the slot schedule never overwrites, so the state is
-// unchanged afterwards (the max signal speed is recomputed).
-static b2d_status time_tile(b2d_ctx* ctx, int fold, int reps, double* ms)
+// unchanged afterwards (the max signal speed is recomputed).  A tiling that is
+// a quarter slower than `best` in its warm-up, or a twentieth in a repetition,
+// is not repeated.
+static b2d_status time_tile(b2d_ctx* ctx, int fold, int reps, double best, double* ms)
 {
     ctx->instrument = true;
     ctx->stage_ms_total = 0.0;
@@ -1822,16 +1824,20 @@ static b2d_status time_tile(b2d_ctx* ctx, int fold, int reps, double* ms)
         b2d_status st = enqueue_advance(ctx, fold, ctx->cur, &fs, true);
         if (st != B2D_OK) { ctx->instrument = false; return st; }
         CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        if (r == 0) continue;  // warm-up
+        double total = 0.0;
         for (size_t s = 0; s < plan.size(); ++s) {
             float m = 0;
             CUDA_TRY(cudaEventElapsedTime(&m, ctx->ev[2 * s], ctx->ev[2 * s + 1]));
-            ctx->stage_ms_total += m;
-            ctx->stage_count++;
+            total += m;
         }
+        if (r > 0) {
+            ctx->stage_ms_total += total;
+            ctx->stage_count += (long long)plan.size();
+        }
+        *ms = r > 0 ? ctx->stage_ms_total / ctx->stage_count : total / plan.size();
+        if (*ms > best * (r > 0 ? 1.05 : 1.25)) break;
     }
     ctx->instrument = false;
-    *ms = ctx->stage_ms_total / std::max<long long>(ctx->stage_count, 1);
     return B2D_OK;
 }
 
@@ -1899,7 +1905,7 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
         ctx->strip_rows = rows;
         b2d_status s = sync_rundev(ctx);
         double ms = 0;
-        if (s == B2D_OK) s = time_tile(ctx, fold, reps, &ms);
+        if (s == B2D_OK) s = time_tile(ctx, fold, reps, best, &ms);
         if (s == B2D_OK && ms < best * AUTOTUNE_MARGIN) { best = ms; best_h = th; best_rows = rows; }
         return s;
     };
@@ -1909,13 +1915,15 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
     } else {
         // block-aligned chunks: every height that divides the blocks, but not
         // so many chunks that they queue up behind one another, and none above
-        // one whose chunks take up half the GPU (they would only be longer)
+        // one whose chunks take up half the GPU (they would only be longer), nor
+        // below a quarter of one that still fills it (four guard rows a chunk)
         const long long slots = resident_ctas(ctx);
         int max_bs = 0;
         for (const RunHost& r : ctx->runs) max_bs = std::max(max_bs, r.bs);
         for (int h = 1; h <= std::min(max_bs, 128); ++h) {
             if (!tile_ok(ctx, ctx->tw, h)) continue;
             if (h < 16 && 2 * h <= max_bs && chunk_ctas(ctx, h) > 2 * slots) continue;
+            if (4 * h <= max_bs && chunk_ctas(ctx, 4 * h) > slots) continue;
             st = trial(h, 0);
             if (st != B2D_OK) return st;
             if (2 * chunk_ctas(ctx, h) <= slots) break;
