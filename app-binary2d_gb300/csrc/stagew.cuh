@@ -47,23 +47,26 @@
 // waits 4.4 cycles per instruction and a scheduler has three), not memory (4.0
 // of 6.7 TB/s).  Measured per stage, with the kernels that it took the place of,
 // as this file began, and now:
-//   isothermal 2048^2          127 -> 109 -> 72.7 us (10 warps a CTA in step over 512 columns)
-//   isothermal 384^2            33 -> 22 -> 12.6 us
-//   the sweep of 64 runs      1050 -> 690 -> 520 us
-//   Euler 4096^2               650 -> 550 -> 362 us
-//   Euler 768^2                 48 -> 42 -> 28.7 us
-//   blocks of 50^2, RK3, alpha 163 -> 25 -> 12.7 us (a thread per column of a block)
-//   FP64 state 1024^2          106 -> 94 -> 40 us
+//   isothermal 2048^2          127 -> 109 -> 71 us (10 warps a CTA in step over 512 columns)
+//   isothermal 384^2            33 -> 22 -> 12.1 us
+//   the sweep of 64 runs      1050 -> 690 -> 512 us
+//   Euler 4096^2               650 -> 550 -> 361 us
+//   Euler 768^2                 48 -> 42 -> 26.6 us
+//   blocks of 50^2, RK3, alpha 163 -> 25 -> 11.9 us (a thread per column of a block)
+//   FP64 state 1024^2          106 -> 94 -> 39 us
 // Of this, forming FP32 pairs of FP64 words and widening increments with integer
 // instructions gave the FP64 state 47 us where the FP64 pipe's conversions take 50
-// to 70.  Tried and slower: the row loop unrolled twice (104 against 98 us at
-// 2048^2: spills); the run's descriptor as a kernel argument (99 against 92);
-// programmatic dependent launch (768^2: 47 against 40 us); 16 warps per SM with
-// 128 registers (85 against 78 us: more instructions, and four warps share what
-// three nearly fill); pairs carried from row to row as 64-bit values (76 against
-// 73 us: more moves); the row loop unrolled twice again, now without spills (76
-// to 78 us: 5 % fewer instructions, but waits for instructions nearly double);
-// the first rows converted before the loop, or requested four at once (75 to 76).
+// to 70, and letting a stage begin in the last row of the one before 12.5 -> 12.1
+// us at 384^2 and 12.6 -> 11.9 on blocks of 50^2.
+//
+// Tried and slower: the row loop unrolled twice (104 against 98 us at 2048^2:
+// spills); the same later without spills (76 to 78 against 73 us: 5 % fewer
+// instructions, but waits for instructions nearly double); the run's descriptor as
+// a kernel argument (99 against 92); letting the next stage in from the start
+// (768^2: 47 against 40 us); 16 warps per SM with 128 registers (85 against 78 us:
+// more instructions, and four warps share what three nearly fill); pairs carried
+// from row to row as 64-bit values (76 against 73 us: more moves); the first rows
+// converted before the loop, or requested four at once (75 to 76).
 #pragma once
 
 #include "split.cuh"
@@ -482,6 +485,13 @@ __device__ __forceinline__ const DevParamsF& params_for(const StageArgs& a, cons
     else return shared_copy;
 }
 
+// Programmatic dependent launch: once every CTA of a stage has let the next
+// start (or is gone), the next stage's CTAs may take the places of those that
+// finish; they wait for the whole stage, and for its writes, before they touch
+// anything that a stage writes.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Asynchronous copy of BYTES bytes (4, 8 or 16, aligned to it) from global to shared memory.
 template <int BYTES> __device__ __forceinline__ void copy_async(void* dst, const void* src)
 {
@@ -655,21 +665,22 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
         }
         copy_commit();
     };
-    issue(-2, -1);
-
-    // What else comes from memory, the first row already on its way, is asked for before any
-    // of it is used: on a small mesh a stage is little more than these latencies.
+    // What else comes from memory is asked for before any of it is used: on a small mesh a stage
+    // is little more than these latencies.  None of this is written by a stage, so it does not
+    // wait for the previous one, of which the last rows may still be running.
     auto at = [](int k, int n) { return min(max(k, 0), n); };
     const float2 ya = rd.xcf[at(j0 + c0, N - 1)], yb = rd.xcf[at(j0 + c0 + 1, N - 1)];
     const float2 va = rd.xvf[at(j0 + c0, N)], vb = rd.xvf[at(j0 + c0 + 1, N)];
     const float2 row_x = rd.xcf[at(i0 - 1 + lane, N - 1)], row_f = rd.xvf[at(i0 - 1 + lane, N)];
+    const double orbit_word = lane < 10 ? rd.orbit[a.stage * 10 + lane] : 0.0;
+    wait_for_previous();
+    issue(-2, -1);
     if (!SINGLE)
         for (int k = lane; k < (int)(sizeof(DevParamsF) / 4); k += 32) ((unsigned*)&S.P)[k] = ((const unsigned*)&rd.pf)[k];
     if (lane < 10) {
-        const double o = rd.orbit[a.stage * 10 + lane];
-        const float hi = (float)o;
+        const float hi = (float)orbit_word;
         ((float*)&S.B)[lane] = hi;
-        S.B_lo[lane] = (float)(o - (double)hi);
+        S.B_lo[lane] = (float)(orbit_word - (double)hi);
     }
     if (*(volatile unsigned long long*)a.err_key != ~0ull) {   // an earlier stage failed: the advance is abandoned
         copy_wait<0>();
@@ -775,6 +786,8 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
     for (int n = -2; n <= TH + 1; ++n) {
         if constexpr (COPY == COPY_QUADS) __syncwarp();     // a slot is read by other lanes than those that fill it
         issue(n + 1, n - 1);
+        // (in the Euler kernel after the loop: here it costs its schedule 4 %)
+        if (NF == 3 && n == TH + 1) let_next_start();
         const int gr = n - 1;
         if (gr == next_fill) {   // the table holds rows gr - 1 to gr + 30
             fill_rows(rd.xcf[at(i0 + gr - 1 + lane, N - 1)], rd.xvf[at(i0 + gr - 1 + lane, N)]);
@@ -1183,6 +1196,8 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
 #pragma unroll
         for (int f = 0; f < NF; ++f) { dP[f] = dn[f]; P0[f] = pn[f]; }
     }
+
+    if (NF == 4) let_next_start();
 
     if (want_amax) {
         const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));   // amax >= 0: its bits are in order
