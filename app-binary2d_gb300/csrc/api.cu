@@ -546,7 +546,10 @@ static int side_divisor(const b2d_ctx* ctx)
 
 // Buffers for the ledger pieces of as many stages as PIECE_BYTES hold (at
 // least one, at most an advance's capacity), and the run descriptors and first
-// CTAs on the device.  Graphs that hold the old descriptors go.
+// CTAs on the device.  Graphs that hold the old descriptors go.  Like every copy
+// and clear of a context these go through its stream: that stream does not wait
+// for the legacy one, and a stage that sees new first CTAs beside old
+// descriptors would compute tiles out of range.
 static b2d_status alloc_pieces(b2d_ctx* ctx)
 {
     constexpr size_t PIECE_BYTES = 64u << 20;
@@ -569,12 +572,13 @@ static b2d_status alloc_pieces(b2d_ctx* ctx)
             CUDA_TRY(cudaMalloc(&r.partial, bytes));
             r.partial_bytes = bytes;
         }
-        CUDA_TRY(cudaMemset(r.partial, 0, bytes));   // the words of items that are always zero are never written
+        CUDA_TRY(cudaMemsetAsync(r.partial, 0, bytes, ctx->stream));   // the words of items that are always zero are never written
         d.partial = r.partial;
         d.stage_window = ctx->stage_window;
     }
-    CUDA_TRY(cudaMemcpy(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * ctx->nruns, cudaMemcpyHostToDevice));
-    CUDA_TRY(cudaMemcpy(ctx->d_bases, bases.data(), sizeof(int) * ctx->nruns, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * ctx->nruns, cudaMemcpyHostToDevice, ctx->stream));
+    CUDA_TRY(cudaMemcpyAsync(ctx->d_bases, bases.data(), sizeof(int) * ctx->nruns, cudaMemcpyHostToDevice, ctx->stream));
+    CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
     ctx->graphs.clear();
     return B2D_OK;
@@ -621,6 +625,7 @@ static b2d_status ensure_stage_capacity(b2d_ctx* ctx, int fold)
     int need = fold * ctx->rk;
     if (need <= ctx->max_stages) return B2D_OK;
     int cap = std::max(need, 64);
+    CUDA_TRY(cudaStreamSynchronize(ctx->stream));   // queued advances use what is replaced here
     for (int i = 0; i < ctx->nruns; ++i) {
         RunHost& r = ctx->runs[i];
         CUDA_TRY(cudaFree(r.stage_time));
@@ -683,14 +688,14 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
     ctx->ctl_words = 2 + (size_t)nruns * (2 + 2 * NSLOTS);
     CREATE_TRY(cudaMalloc(&ctx->d_ctl, sizeof(unsigned long long) * ctx->ctl_words));
     CREATE_TRY(cudaMallocHost(&ctx->h_ctl, sizeof(unsigned long long) * ctx->ctl_words));
-    CREATE_TRY(cudaMemset(ctx->d_ctl, 0, sizeof(unsigned long long) * ctx->ctl_words));
+    CREATE_TRY(cudaMemsetAsync(ctx->d_ctl, 0, sizeof(unsigned long long) * ctx->ctl_words, ctx->stream));
     ctx->d_err_key = ctx->d_ctl;
     ctx->d_adv_count = (long long*)(ctx->d_ctl + 1);
     ctx->d_amax = ctx->d_ctl + 2;
     ctx->d_dt = (double*)(ctx->d_amax + nruns);
     ctx->d_time = ctx->d_dt + nruns;
     ctx->d_iter = (long long*)(ctx->d_time + (size_t)nruns * NSLOTS);
-    CREATE_TRY(cudaMemset(ctx->d_err_key, 0xff, sizeof(unsigned long long)));
+    CREATE_TRY(cudaMemsetAsync(ctx->d_err_key, 0xff, sizeof(unsigned long long), ctx->stream));
 
     ctx->runs.resize(nruns);
     ctx->rdev_h.resize(nruns);
@@ -708,14 +713,14 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
         r.state_bytes = store == 1 ? nn * ctx->nf * 2 * sizeof(float) : nn * ctx->nf * sizeof(double);
         for (int s = 0; s < NSLOTS; ++s) {
             CREATE_TRY(cudaMalloc(&r.slot[s], r.state_bytes));
-            CREATE_TRY(cudaMemset(r.slot[s], 0, r.state_bytes));
+            CREATE_TRY(cudaMemsetAsync(r.slot[s], 0, r.state_bytes, ctx->stream));
             CREATE_TRY(cudaMalloc(&r.ledger[s], sizeof(double) * r.nblocks * NITEMS * ctx->nf));
-            CREATE_TRY(cudaMemset(r.ledger[s], 0, sizeof(double) * r.nblocks * NITEMS * ctx->nf));
+            CREATE_TRY(cudaMemsetAsync(r.ledger[s], 0, sizeof(double) * r.nblocks * NITEMS * ctx->nf, ctx->stream));
             CREATE_TRY(cudaMalloc(&r.elements[s], sizeof(double) * r.nblocks * NITEMS * 4));
-            CREATE_TRY(cudaMemset(r.elements[s], 0, sizeof(double) * r.nblocks * NITEMS * 4));
+            CREATE_TRY(cudaMemsetAsync(r.elements[s], 0, sizeof(double) * r.nblocks * NITEMS * 4, ctx->stream));
         }
         CREATE_TRY(cudaMalloc(&r.bg, r.state_bytes));
-        CREATE_TRY(cudaMemset(r.bg, 0, r.state_bytes));
+        CREATE_TRY(cudaMemsetAsync(r.bg, 0, r.state_bytes, ctx->stream));
         // geometry tables
         std::vector<double> xc(r.N), xv((size_t)r.nb * (r.bs + 1));
         for (int b = 0; b < r.nb; ++b) {
@@ -739,10 +744,10 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
         CREATE_TRY(cudaMalloc(&r.xv, sizeof(double) * xv.size()));
         CREATE_TRY(cudaMalloc(&r.xcf, sizeof(float2) * xcf.size()));
         CREATE_TRY(cudaMalloc(&r.xvf, sizeof(float2) * xvf.size()));
-        CREATE_TRY(cudaMemcpy(r.xc, xc.data(), sizeof(double) * xc.size(), cudaMemcpyHostToDevice));
-        CREATE_TRY(cudaMemcpy(r.xv, xv.data(), sizeof(double) * xv.size(), cudaMemcpyHostToDevice));
-        CREATE_TRY(cudaMemcpy(r.xcf, xcf.data(), sizeof(float2) * xcf.size(), cudaMemcpyHostToDevice));
-        CREATE_TRY(cudaMemcpy(r.xvf, xvf.data(), sizeof(float2) * xvf.size(), cudaMemcpyHostToDevice));
+        CREATE_TRY(cudaMemcpyAsync(r.xc, xc.data(), sizeof(double) * xc.size(), cudaMemcpyHostToDevice, ctx->stream));
+        CREATE_TRY(cudaMemcpyAsync(r.xv, xv.data(), sizeof(double) * xv.size(), cudaMemcpyHostToDevice, ctx->stream));
+        CREATE_TRY(cudaMemcpyAsync(r.xcf, xcf.data(), sizeof(float2) * xcf.size(), cudaMemcpyHostToDevice, ctx->stream));
+        CREATE_TRY(cudaMemcpyAsync(r.xvf, xvf.data(), sizeof(float2) * xvf.size(), cudaMemcpyHostToDevice, ctx->stream));
 
         d.N = r.N; d.bs = r.bs; d.nb = r.nb; d.nblocks = r.nblocks;
         d.xc = r.xc; d.xv = r.xv; d.xcf = r.xcf; d.xvf = r.xvf;
@@ -800,7 +805,7 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
             ctx->rdev_h[i].buffer = r.buffer;
         }
         CREATE_TRY(cudaStreamSynchronize(ctx->stream));
-        CREATE_TRY(cudaMemcpy(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * nruns, cudaMemcpyHostToDevice));
+        CREATE_TRY(cudaMemcpyAsync(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * nruns, cudaMemcpyHostToDevice, ctx->stream));
     }
     if (ensure_stage_capacity(ctx, 16) != B2D_OK) { *status = B2D_ERR_CUDA; free_ctx(ctx); return nullptr; }
     *status = B2D_OK;
@@ -1500,10 +1505,11 @@ extern "C" b2d_status b2d_set_tracers(b2d_ctx* ctx, int32_t run, int64_t n, cons
     d.ntracers = 0;
     if (n > 0) {
         for (int s = 0; s < NSLOTS; ++s) CUDA_TRY(cudaMalloc(&d.tracers[s], sizeof(double) * 2 * (size_t)n));
-        CUDA_TRY(cudaMemcpy(d.tracers[ctx->cur], xy, sizeof(double) * 2 * (size_t)n, cudaMemcpyHostToDevice));
+        CUDA_TRY(cudaMemcpyAsync(d.tracers[ctx->cur], xy, sizeof(double) * 2 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
         d.ntracers = n;
     }
-    CUDA_TRY(cudaMemcpy(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * ctx->nruns, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemcpyAsync(ctx->rdev, ctx->rdev_h.data(), sizeof(RunDev) * ctx->nruns, cudaMemcpyHostToDevice, ctx->stream));
+    CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
     ctx->graphs.clear();
     return B2D_OK;
@@ -1581,6 +1587,13 @@ static double failure_value(const b2d_config& c, const double* u, int code)
     return p[3];
 }
 
+// A copy to the host in the order of `stream`, waited for.
+static cudaError_t read_back(void* dst, const void* src, size_t bytes, cudaStream_t stream)
+{
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(stream);
+}
+
 static b2d_status decode_failure(b2d_ctx* ctx, unsigned long long key, const std::vector<StagePlan>& plan,
                                  b2d_error* e)
 {
@@ -1600,8 +1613,8 @@ static b2d_status decode_failure(b2d_ctx* ctx, unsigned long long key, const std
         // the failing block's index is carried in the zone field.
         e->block_i = zone / nb;
         e->block_j = zone % nb;
-        CUDA_TRY(cudaMemcpy(&e->time, r.stage_time + stage, sizeof(double), cudaMemcpyDeviceToHost));
-        CUDA_TRY(cudaMemcpy(orb, r.orbit + 10 * stage, sizeof orb, cudaMemcpyDeviceToHost));
+        CUDA_TRY(read_back(&e->time, r.stage_time + stage, sizeof(double), ctx->stream));
+        CUDA_TRY(read_back(orb, r.orbit + 10 * stage, sizeof orb, ctx->stream));
         e->binary[0] = orb[1]; e->binary[1] = orb[2]; e->binary[2] = orb[6]; e->binary[3] = orb[7];
         return B2D_OK;
     }
@@ -1618,17 +1631,17 @@ static b2d_status decode_failure(b2d_ctx* ctx, unsigned long long key, const std
     double u[4] = {0, 0, 0, 0};
     for (int f = 0; f < ctx->nf; ++f) {
         if (store_of(ctx) == 0) {
-            CUDA_TRY(cudaMemcpy(&u[f], (const double*)r.slot[slot] + f * nn + idx, sizeof(double), cudaMemcpyDeviceToHost));
+            CUDA_TRY(read_back(&u[f], (const double*)r.slot[slot] + f * nn + idx, sizeof(double), ctx->stream));
         } else {
             float hl[2];
-            CUDA_TRY(cudaMemcpy(&hl[0], (const float*)r.slot[slot] + (2 * f) * nn + idx, sizeof(float), cudaMemcpyDeviceToHost));
-            CUDA_TRY(cudaMemcpy(&hl[1], (const float*)r.slot[slot] + (2 * f + 1) * nn + idx, sizeof(float), cudaMemcpyDeviceToHost));
+            CUDA_TRY(read_back(&hl[0], (const float*)r.slot[slot] + (2 * f) * nn + idx, sizeof(float), ctx->stream));
+            CUDA_TRY(read_back(&hl[1], (const float*)r.slot[slot] + (2 * f + 1) * nn + idx, sizeof(float), ctx->stream));
             u[f] = (double)hl[0] + (double)hl[1];
         }
     }
     e->value = failure_value(r.cfg, u, e->code);
-    CUDA_TRY(cudaMemcpy(&e->time, r.stage_time + stage, sizeof(double), cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemcpy(orb, r.orbit + 10 * stage, sizeof orb, cudaMemcpyDeviceToHost));
+    CUDA_TRY(read_back(&e->time, r.stage_time + stage, sizeof(double), ctx->stream));
+    CUDA_TRY(read_back(orb, r.orbit + 10 * stage, sizeof orb, ctx->stream));
     e->binary[0] = orb[1]; e->binary[1] = orb[2]; e->binary[2] = orb[6]; e->binary[3] = orb[7];
     return B2D_OK;
 }
@@ -1937,10 +1950,10 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
     }
     // discard what the trial advances left behind
     long long count = 0;
-    CUDA_TRY(cudaMemcpy(&count, ctx->d_adv_count, sizeof count, cudaMemcpyDeviceToHost));
+    CUDA_TRY(read_back(&count, ctx->d_adv_count, sizeof count, ctx->stream));
     ctx->adv_base = count;
     ctx->window.clear();
-    CUDA_TRY(cudaMemset(ctx->d_err_key, 0xff, sizeof(unsigned long long)));
+    CUDA_TRY(cudaMemsetAsync(ctx->d_err_key, 0xff, sizeof(unsigned long long), ctx->stream));
     ctx->tw = best_w;
     ctx->th = best_h;
     ctx->strip_rows = best_rows;
@@ -2271,9 +2284,8 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     err.time = time;
     double u[4] = {0, 0, 0, 0}, orb[10];
     for (int f = 0; f < nf; ++f)
-        CUDA_TRY(cudaMemcpy(&u[f], d_in + (size_t)f * N * N + (size_t)gi * N + gj, sizeof(double),
-                            cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemcpy(orb, orbit, sizeof orb, cudaMemcpyDeviceToHost));
+        CUDA_TRY(read_back(&u[f], d_in + (size_t)f * N * N + (size_t)gi * N + gj, sizeof(double), stream));
+    CUDA_TRY(read_back(orb, orbit, sizeof orb, stream));
     err.value = failure_value(*cfg, u, err.code);
     err.binary[0] = orb[1]; err.binary[1] = orb[2]; err.binary[2] = orb[6]; err.binary[3] = orb[7];
     if (err_out) *err_out = err;
