@@ -122,6 +122,9 @@ template <int NF, int STORE, int COPY> struct SWShape {
     static constexpr int UPDATE = NU * U_PITCH;
     static constexpr int BYTES = TABLES + (SW_SLOTS * STENCIL + SW_USLOTS * UPDATE + (COPY == COPY_QUADS ? 4 : 0)) * (int)sizeof(E);
     static constexpr int CTAS = 12;   // per SM
+    // A lane's items' sums (words 2 lane, 2 lane + 1 of rows of 64 FP32 words) cover only words that it alone
+    // copies and reads: not where the planes' words are FP64, or lie at another pitch.
+    static constexpr bool SUMS_OVER_OWN = STORE == 1 && COPY != COPY_QUADS;
     static_assert(SINKS_AT * 64 * 4 <= UPDATE * (int)sizeof(E), "a consumed update row takes the items' sums");
 };
 
@@ -1167,7 +1170,7 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
                             if (iny) amax = fmaxf(max_speed_f32<NF>(P, ub, lb), amax);
                         }
                         if (ru + 1 == next_flush || ru + 1 == TH) {   // the end of a block row, or of the chunk
-                            if constexpr (COPY == COPY_QUADS) __syncwarp();   // it holds other lanes' columns
+                            if constexpr (!T::SUMS_OVER_OWN) __syncwarp();   // others may not have read theirs yet
                             float* sums = (float*)(update + (ru & 1) * T::UPDATE);   // this row's, which is done with
 #pragma unroll
                             for (int m = 0; m < NACC; ++m) {
