@@ -356,11 +356,17 @@ __device__ __forceinline__ float2 alpha_nhalf_k2(const float2* K, float2 dx1, fl
 //   F = fl wl + fr wr - (ur - ul) b wl,
 // and f = u v + pressure terms, so that the states enter through two products,
 //   F = ul A + ur B + pressure terms, A = wl (vl + b), B = wr (vr - a+):
-// 12 packed operations of an isothermal face pair where forming the conserved
-// states and the fluxes on either side takes 22.  Where the flow is supersonic
-// the downwind state's weight is a product with a zero, so that it drops out
-// exactly, whichever way the flow goes: as 1 - wl it is 1e-7 of that state,
-// which beside a light zone is no small part of the flux.
+// 16 packed operations of an isothermal face pair where forming the conserved
+// states and the fluxes on either side takes 22.
+//
+// Where the flow is supersonic the downwind state's weight is a product with a
+// zero, so that it drops out exactly, whichever way the flow goes: as 1 - wl it
+// is 1e-7 of that state, which beside a light zone is no small part of the flux.
+// What the two rounded weights miss to 1 is then shared out over them (a weight
+// of 0 stays 0, that of a state on its own becomes 1): without that the flux is
+// off by the reciprocal's rounding, and over 40 disks of 256^2 and 512^2 the
+// state's error against 64 bits 3 to 14 % larger (2048^2 without it 29.9 ms a
+// pass, with it 30.3).
 template <int NF, int AXIS>
 __device__ __forceinline__ void faces2(const float2* K, const float2* pl, const float2* pr, float2 cs2, float2 k,
                                        float2 tn, float2 tt, float2 vxs, float2 vys, float2* F)
@@ -377,7 +383,8 @@ __device__ __forceinline__ void faces2(const float2* K, const float2* pl, const 
     const float2 alp = add2(vl, csl), arp = add2(vr, csr), blm = sub2(csl, vl), brm = sub2(csr, vr);
     const float2 ap = make_float2(max3f(alp.x, arp.x, 0.0f), max3f(alp.y, arp.y, 0.0f));
     const float2 bm = make_float2(max3f(blm.x, brm.x, 0.0f), max3f(blm.y, brm.y, 0.0f));
-    const float2 r = rcp2(add2(ap, bm)), wl = mul2(ap, r), wr = mul2(bm, r);
+    const float2 r = rcp2(add2(ap, bm)), wl1 = mul2(ap, r), wr1 = mul2(bm, r);
+    const float2 miss = sub2(K[C_ONE], add2(wl1, wr1)), wl = fma2(wl1, miss, wl1), wr = fma2(wr1, miss, wr1);
     const float2 A = mul2(wl, add2(vl, bm)), B = mul2(wr, sub2(vr, ap));
     const float2 ml = mul2(pl[0], A), mr = mul2(pr[0], B);
     F[0] = add2(ml, mr);
