@@ -89,13 +89,17 @@ __device__ void kepler_orbit(const RunDev& rd, double t, double* o)
 // steps (try_advance_rk stamps t + dt, scheme.rs:168-170; weighted_average
 // averages time, state.rs:213-214), and the binary at each stage time.
 __global__ void prologue_kernel(const RunDev* runs, int fold, int rk, int start, int final_slot,
-                                const unsigned long long* err_key, long long* adv_count)
+                                Failure* failure, long long* adv_count)
 {
     const RunDev& rd = runs[blockIdx.x];
     const int stages = rk;
     __shared__ int failed;
-    // a failure is pending: this advance and every later one are abandoned
-    if (threadIdx.x == 0) failed = (*(volatile const unsigned long long*)err_key != ~0ull);
+    // a failure is pending: this advance and every later one are abandoned.  Their kernels leave every
+    // slot alone, since the one that the failing advance began from comes up again as an output slot.
+    if (threadIdx.x == 0) {
+        failed = (*(volatile unsigned long long*)&failure->key != ~0ull);
+        if (blockIdx.x == 0) failure->abandoned = failed;
+    }
     __syncthreads();
     if (failed) return;
     if (threadIdx.x == 0 && blockIdx.x == 0) *adv_count += 1;
@@ -320,7 +324,7 @@ struct b2d_ctx {
     double* d_time = nullptr;         // [nruns][NSLOTS]
     long long* d_iter = nullptr;      // [nruns][NSLOTS]
     unsigned long long* d_amax = nullptr;  // [nruns]
-    unsigned long long* d_err_key = nullptr;  // failure key (~0: none)
+    Failure* d_failure = nullptr;
     long long* d_adv_count = nullptr;       // advances begun without a pending failure
     long long adv_base = 0;
     std::vector<std::pair<int, std::vector<StagePlan>>> window;  // advances since the last check
@@ -685,17 +689,17 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
     CREATE_TRY(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
     CREATE_TRY(cudaMalloc(&ctx->rdev, sizeof(RunDev) * nruns));
     CREATE_TRY(cudaMalloc(&ctx->d_bases, sizeof(int) * nruns));
-    ctx->ctl_words = 2 + (size_t)nruns * (2 + 2 * NSLOTS);
+    ctx->ctl_words = 3 + (size_t)nruns * (2 + 2 * NSLOTS);
     CREATE_TRY(cudaMalloc(&ctx->d_ctl, sizeof(unsigned long long) * ctx->ctl_words));
     CREATE_TRY(cudaMallocHost(&ctx->h_ctl, sizeof(unsigned long long) * ctx->ctl_words));
     CREATE_TRY(cudaMemsetAsync(ctx->d_ctl, 0, sizeof(unsigned long long) * ctx->ctl_words, ctx->stream));
-    ctx->d_err_key = ctx->d_ctl;
-    ctx->d_adv_count = (long long*)(ctx->d_ctl + 1);
-    ctx->d_amax = ctx->d_ctl + 2;
+    ctx->d_failure = (Failure*)ctx->d_ctl;
+    ctx->d_adv_count = (long long*)(ctx->d_ctl + 2);
+    ctx->d_amax = ctx->d_ctl + 3;
     ctx->d_dt = (double*)(ctx->d_amax + nruns);
     ctx->d_time = ctx->d_dt + nruns;
     ctx->d_iter = (long long*)(ctx->d_time + (size_t)nruns * NSLOTS);
-    CREATE_TRY(cudaMemsetAsync(ctx->d_err_key, 0xff, sizeof(unsigned long long), ctx->stream));
+    CREATE_TRY(cudaMemsetAsync(&ctx->d_failure->key, 0xff, sizeof(unsigned long long), ctx->stream));
 
     ctx->runs.resize(nruns);
     ctx->rdev_h.resize(nruns);
@@ -1136,11 +1140,11 @@ template <int NF> __device__ __forceinline__ void fold_item(const RunDev& rd, in
 }
 
 __global__ void __launch_bounds__(256) ledger_kernel(const RunDev* runs, int first, int last, bool sum, int fold, int rk,
-                                                     int start, unsigned long long* err_key)
+                                                     int start, Failure* failure)
 {
     const int run = blockIdx.y, block = blockIdx.x;
     const RunDev& rd = runs[run];
-    if (block >= rd.nblocks) return;
+    if (block >= rd.nblocks || failure->abandoned) return;
     if (rd.slab_hi > 0 && (block / rd.nb < rd.slab_lo || block / rd.nb >= rd.slab_hi)) return;   // another slab's
     const int nf = rd.p.hydro == B2D_EULER ? 4 : 3, nl = NITEMS * nf, pieces = rd.tiles_per_block;
     const size_t stride = (size_t)rd.nblocks * nl;
@@ -1169,7 +1173,7 @@ __global__ void __launch_bounds__(256) ledger_kernel(const RunDev* runs, int fir
             de[0] = de[1] = de[2] = de[3] = 0.0;
             const unsigned long long key = ((unsigned long long)s << 54) | ((unsigned long long)run << 46) |
                                            (0xffffull << 30) | (0xfull << 26) | ((unsigned long long)block << 2) | 3ull;
-            atomicMin(err_key, key);
+            atomicMin(&failure->key, key);
         }
     }
     if (!sum) return;
@@ -1249,7 +1253,7 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
     a.half_avg = sp.bf == 0.5;
     a.w1f = split_df(-sp.bf + 1.0);
     a.bff = split_df(sp.bf);
-    a.err_key = ctx->d_err_key;
+    a.failure = ctx->d_failure;
     cudaError_t e;
     if (ctx->precision == B2D_PREC_FP64)
         e = launch_stage_f64(ctx->nf, a, ctx->total_tiles, stage_f64_smem(ctx->nf, ctx->sub_h, ctx->sub_w), ctx->stream);
@@ -1343,11 +1347,11 @@ __device__ __forceinline__ double tracer_move(double x, float xh, float xl, floa
 // bf: the base's weight; w: 1 - bf as FP32 high and low words.
 template <int MODE>
 __global__ void __launch_bounds__(256) tracer_kernel(const RunDev* runs, int run, int in_slot, int base_slot, int out_slot,
-                                                     double bf, float2 w)
+                                                     double bf, float2 w, const Failure* failure)
 {
     const RunDev& rd = runs[run];
     const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (k >= rd.ntracers) return;
+    if (k >= rd.ntracers || failure->abandoned) return;
     const double R = rd.p.domain_radius, dx = rd.p.dx, dt = *rd.dt;
     const int N = rd.N;
     const double2 at = ((const double2*)rd.tracers[in_slot])[k];
@@ -1433,11 +1437,11 @@ static b2d_status launch_tracers(b2d_ctx* ctx, const StagePlan& sp, bool count)
         const int threads = 256;
         const unsigned grid = (unsigned)((n + threads - 1) / threads);
         if (ctx->precision == B2D_PREC_FP64)
-            tracer_kernel<0><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w);
+            tracer_kernel<0><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w, ctx->d_failure);
         else if (ctx->precision == B2D_PREC_FP32_STATE64)
-            tracer_kernel<1><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w);
+            tracer_kernel<1><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w, ctx->d_failure);
         else
-            tracer_kernel<2><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w);
+            tracer_kernel<2><<<grid, threads, 0, ctx->stream>>>(ctx->rdev, r, sp.in, sp.base, sp.out, sp.bf, w, ctx->d_failure);
         CUDA_TRY(cudaGetLastError());
         if (count) ctx->launches++;
     }
@@ -1450,7 +1454,7 @@ static b2d_status launch_ledgers(b2d_ctx* ctx, int first, int last, bool sum, in
     const int nl = NITEMS * ctx->nf, work = std::max((last - first) * nl, nl + NITEMS * 4);
     const int threads = std::min((work + 31) / 32 * 32, 256);
     ledger_kernel<<<dim3((unsigned)max_blocks(ctx), (unsigned)ctx->nruns), threads, 0, ctx->stream>>>(
-        ctx->rdev, first, last, sum, fold, ctx->rk, start, ctx->d_err_key);
+        ctx->rdev, first, last, sum, fold, ctx->rk, start, ctx->d_failure);
     CUDA_TRY(cudaGetLastError());
     if (count) ctx->launches++;
     return B2D_OK;
@@ -1466,7 +1470,7 @@ static int fold_due(const b2d_ctx* ctx, int s, int nstages)
 static b2d_status enqueue_advance(b2d_ctx* ctx, int fold, int start, int* final_slot, bool count)
 {
     std::vector<StagePlan> plan = plan_advance(ctx->rk, fold, start, final_slot);
-    prologue_kernel<<<ctx->nruns, 32, 0, ctx->stream>>>(ctx->rdev, fold, ctx->rk, start, *final_slot, ctx->d_err_key,
+    prologue_kernel<<<ctx->nruns, 32, 0, ctx->stream>>>(ctx->rdev, fold, ctx->rk, start, *final_slot, ctx->d_failure,
                                                          ctx->d_adv_count);
     CUDA_TRY(cudaGetLastError());
     if (count) ctx->launches++;
@@ -1650,7 +1654,7 @@ static b2d_status finish_advance(b2d_ctx* ctx, int final_slot, double* dt_out, b
 {
     const ControlRead control(ctx);
     if (control.status != B2D_OK) return control.status;
-    const unsigned long long key = control(ctx->d_err_key);
+    const unsigned long long key = control(&ctx->d_failure->key);
     const long long count = control(ctx->d_adv_count);
     auto window = std::move(ctx->window);
     ctx->window.clear();
@@ -1666,7 +1670,7 @@ static b2d_status finish_advance(b2d_ctx* ctx, int final_slot, double* dt_out, b
         b2d_status s = decode_failure(ctx, key, window[k].second, &err);
         if (s != B2D_OK) return s;
         if (err_out) *err_out = err;
-        CUDA_TRY(cudaMemsetAsync(ctx->d_err_key, 0xff, sizeof(unsigned long long), ctx->stream));
+        CUDA_TRY(cudaMemsetAsync(&ctx->d_failure->key, 0xff, sizeof(unsigned long long), ctx->stream));
         ctx->cur = start;
         for (int r = 0; r < ctx->nruns; ++r) {
             s = launch_max_speed(ctx, r, start);
@@ -1953,7 +1957,7 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
     CUDA_TRY(read_back(&count, ctx->d_adv_count, sizeof count, ctx->stream));
     ctx->adv_base = count;
     ctx->window.clear();
-    CUDA_TRY(cudaMemsetAsync(ctx->d_err_key, 0xff, sizeof(unsigned long long), ctx->stream));
+    CUDA_TRY(cudaMemsetAsync(&ctx->d_failure->key, 0xff, sizeof(unsigned long long), ctx->stream));
     ctx->tw = best_w;
     ctx->th = best_h;
     ctx->strip_rows = best_rows;
@@ -2017,7 +2021,7 @@ extern "C" b2d_status b2d_slab_begin(b2d_ctx* ctx, int32_t fold, const double* a
     ctx->slab_start = start;
     ctx->slab_next = 0;
     ctx->window.emplace_back(start, ctx->slab_plan);
-    prologue_kernel<<<ctx->nruns, 32, 0, ctx->stream>>>(ctx->rdev, fold, ctx->rk, start, ctx->slab_final, ctx->d_err_key,
+    prologue_kernel<<<ctx->nruns, 32, 0, ctx->stream>>>(ctx->rdev, fold, ctx->rk, start, ctx->slab_final, ctx->d_failure,
                                                          ctx->d_adv_count);
     CUDA_TRY(cudaGetLastError());
     ctx->launches++;
@@ -2201,7 +2205,7 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     double* times = orbit + 12;                            // 4 doubles (unused by the stage)
     long long* iters = (long long*)(orbit + 16);           // 4 (unused by the stage)
     unsigned long long* amax = (unsigned long long*)(orbit + 20);
-    unsigned long long* err_key = amax + 1;
+    Failure* failure = (Failure*)(amax + 1);
     double* partial = (double*)(base + off_part);
 
     std::vector<double> xc(N), xv((size_t)nb * (bs + 1));
@@ -2237,7 +2241,8 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     CUDA_TRY(cudaMemcpyAsync(d_xc, xc.data(), sizeof(double) * xc.size(), cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemcpyAsync(d_xv, xv.data(), sizeof(double) * xv.size(), cudaMemcpyHostToDevice, stream));
     CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(unsigned long long), stream));
-    CUDA_TRY(cudaMemsetAsync(err_key, 0xff, sizeof(unsigned long long), stream));
+    CUDA_TRY(cudaMemsetAsync(failure, 0, sizeof(Failure), stream));
+    CUDA_TRY(cudaMemsetAsync(&failure->key, 0xff, sizeof(unsigned long long), stream));
     noalloc_setup_kernel<<<1, 32, 0, stream>>>(d_run, time, dt);
     CUDA_TRY(cudaGetLastError());
 
@@ -2256,7 +2261,7 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     a.half_avg = a.bf == 0.5;
     a.w1f = split_df(-a.bf + 1.0);
     a.bff = split_df(a.bf);
-    a.err_key = err_key;
+    a.failure = failure;
     cudaError_t e = launch_stage_f64(nf, a, rd.ntiles, stage_f64_smem(nf, sub_h, sub_w), stream);
     if (e != cudaSuccess) return fail(B2D_ERR_CUDA, std::string("stage kernel launch: ") + cudaGetErrorString(e));
     noalloc_ledger_kernel<<<(nblocks * NITEMS + 127) / 128, 128, 0, stream>>>(d_run, a.base_slot, a.bf);
@@ -2264,7 +2269,7 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     if (d_max_speed) CUDA_TRY(cudaMemcpyAsync(d_max_speed, amax, sizeof(double), cudaMemcpyDeviceToDevice, stream));
 
     unsigned long long key = ~0ull;
-    CUDA_TRY(cudaMemcpyAsync(&key, err_key, sizeof key, cudaMemcpyDeviceToHost, stream));
+    CUDA_TRY(cudaMemcpyAsync(&key, &failure->key, sizeof key, cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaStreamSynchronize(stream));
     if (key == ~0ull) return B2D_OK;
 

@@ -53,6 +53,12 @@ struct RunDev {
     DevParamsF pf;   // FP32 kernels
 };
 
+// A context's failure words.
+struct Failure {
+    unsigned long long key;         // of the earliest failing zone (error_key, stage.cuh), ~0 when none failed
+    unsigned long long abandoned;   // the advance found a failure pending when it began: it changes nothing
+};
+
 struct StageArgs {
     const RunDev* runs;
     const int* tile_bases;   // [nruns] first CTA of each run
@@ -64,7 +70,7 @@ struct StageArgs {
     double bf;               // weight of the RK base state (br of godunov-core)
     int half_avg;            // bf is 1/2
     b2d::df32w w1f, bff;     // 1 - bf and bf as double-float
-    unsigned long long* err_key;  // failure key, ~0 when no zone failed
+    Failure* failure;
     DevParamsF pf1;          // FP32 parameters of a single-run context, read as kernel arguments
 };
 

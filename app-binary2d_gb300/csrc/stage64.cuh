@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
     for (int i = t; i < NW * NL; i += NT) led[i / NL][i % NL] = 0.0;
     if (t == 0) P = rd.p;
     // an earlier stage failed: the advance is abandoned (the caller keeps its state)
-    if (t == 0) failed = (*(volatile unsigned long long*)a.err_key != ~0ull);
+    if (t == 0) failed = (*(volatile unsigned long long*)&a.failure->key != ~0ull);
     __syncthreads();
     if (failed) return;
     if (t < 10) orb[t] = rd.orbit[a.stage * 10 + t];
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
                 }
             }
             if (err && r >= 0 && r < TH && c >= 0 && c < TW)
-                atomicMin(a.err_key, error_key(a.stage, ri, rd, gi, gj, err));
+                atomicMin(&a.failure->key, error_key(a.stage, ri, rd, gi, gj, err));
 #pragma unroll
             for (int f = 0; f < NF; ++f) sP[f * PS + e] = p[f];
         }

@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
         ((float*)&S.B)[lane] = hi;
         S.B_lo[lane] = (float)(orbit_word - (double)hi);
     }
-    if (*(volatile unsigned long long*)a.err_key != ~0ull) {   // an earlier stage failed: the advance is abandoned
+    if (*(volatile unsigned long long*)&a.failure->key != ~0ull) {   // an earlier stage failed: the advance is abandoned
         copy_wait<0>();
         return;
     }
@@ -854,8 +854,8 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
                 eb = pn[0].y < 0.0f ? 1 : (pn[3].y <= 0.0f ? 2 : 0);
             }
             if (__any_sync(0xffffffffu, ea || eb) && n >= 0 && n < TH) {
-                if (ea && inx) atomicMin(a.err_key, error_key(a.stage, ri, rd, i0 + n, j0 + c0, ea));
-                if (eb && iny) atomicMin(a.err_key, error_key(a.stage, ri, rd, i0 + n, j0 + c0 + 1, eb));
+                if (ea && inx) atomicMin(&a.failure->key, error_key(a.stage, ri, rd, i0 + n, j0 + c0, ea));
+                if (eb && iny) atomicMin(&a.failure->key, error_key(a.stage, ri, rd, i0 + n, j0 + c0 + 1, eb));
             }
         }
 
