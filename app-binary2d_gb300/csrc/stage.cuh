@@ -37,4 +37,15 @@ __device__ __forceinline__ unsigned long long error_key(int stage, int run, cons
     return best;
 }
 
+// Whether stage `stage` is to be left out: the advance was abandoned when it
+// began, or an earlier stage of it failed.  A failure in this stage does not
+// count, whoever found it: all of its zones are looked at, so that the smallest
+// key does not depend on which CTAs run first.
+__device__ __forceinline__ bool left_out(const Failure* failure, int stage)
+{
+    const volatile Failure* f = failure;
+    const unsigned long long key = f->key, abandoned = f->abandoned;
+    return abandoned || key < (unsigned long long)stage << 54;
+}
+
 }  // namespace b2d

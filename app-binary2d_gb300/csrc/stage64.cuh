@@ -241,15 +241,14 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
 
     __shared__ DevParams P;
     __shared__ double orb[10];
-    __shared__ int failed;
+    __shared__ int skip;
     __shared__ double led[NW][NL];
     __shared__ double wmax[NW];
     for (int i = t; i < NW * NL; i += NT) led[i / NL][i % NL] = 0.0;
     if (t == 0) P = rd.p;
-    // an earlier stage failed: the advance is abandoned (the caller keeps its state)
-    if (t == 0) failed = (*(volatile unsigned long long*)&a.failure->key != ~0ull);
+    if (t == 0) skip = left_out(a.failure, a.stage);   // (the caller keeps its state)
     __syncthreads();
-    if (failed) return;
+    if (skip) return;
     if (t < 10) orb[t] = rd.orbit[a.stage * 10 + t];
     extern __shared__ __align__(128) unsigned char smem_raw[];   // one declaration for every stage kernel
     poison_dynamic_smem(smem_raw);

@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
         ((float*)&S.B)[lane] = hi;
         S.B_lo[lane] = (float)(orbit_word - (double)hi);
     }
-    if (*(volatile unsigned long long*)&a.failure->key != ~0ull) {   // an earlier stage failed: the advance is abandoned
+    if (left_out(a.failure, a.stage)) {
         copy_wait<0>();
         return;
     }
