@@ -87,6 +87,8 @@ __device__ __forceinline__ bool moderate(double x)
     const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
     return h - 0x26f00000u < 0x32000000u || (h | (unsigned)__double2loint(x)) == 0u;
 }
+// a magnitude below 2^100: neither infinite nor NaN, and products of a few such values are not either
+__device__ __forceinline__ bool bounded(double x) { return ((unsigned)__double2hiint(x) & 0x7fffffffu) < 0x46300000u; }
 // max(0, x), 0 for NaN
 __device__ __forceinline__ unsigned long long positive_part(unsigned long long b) { return b <= D_INF ? b : 0ull; }
 // max(0, a, b) and min(0, a, b) of fmax and fmin, which pass over NaN
@@ -521,9 +523,13 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
             const double ap = max_0(vl + csl, vr + csr), am = min_0(vl - csl, vr - csr);
             double F[NF];
             // All faces of the warp supersonic: (fl ap - fr am - (ul - ur) ap am) / (ap - am) is
-            // then (fl ap) / ap with am = 0, (fr am) / am with ap = 0, and the other side drops out.
+            // then (fl ap) / ap with am = 0, (fr am) / am with ap = 0, and the other side drops out
+            // (unless its terms are infinite or NaN: those times 0 are NaN).
             const bool from_l = zero(am);
-            if (__all_sync(__activemask(), from_l || zero(ap))) {
+            bool one_side = from_l || zero(ap);
+#pragma unroll
+            for (int f = 0; f < NF; ++f) one_side = one_side && bounded(pl[f]) && bounded(pr[f]);
+            if (__all_sync(__activemask(), one_side)) {
                 double pu[NF], u[NF], f[NF];
 #pragma unroll
                 for (int k = 0; k < NF; ++k) pu[k] = from_l ? pl[k] : pr[k];
@@ -609,7 +615,13 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
             }
             constexpr int IB = 2 * (NF - 1);               // the buffer's items in acc
             const double kb = -dt * br;
-            const bool buffer_on = __any_sync(0xffffffffu, !zero(br));
+            // items with a rate of 0 are left out where none of the warp's zones has another rate: not
+            // where a zone's values could make NaN of that 0
+            bool odd = false;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) odd = odd || !bounded(u[f]) || !bounded(u0[f]);
+            odd = __any_sync(0xffffffffu, odd);
+            const bool buffer_on = odd || __any_sync(0xffffffffu, !zero(br));
 #pragma unroll
             for (int f = 0; f < NF; ++f) it[IB + f] = buffer_on ? (u[f] - u0[f]) * kb : 0.0;
             // cooling (Euler::source_terms, physics.rs:701-738; beta-cooling is new)
@@ -644,7 +656,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
             // those that are zero
             const bool near = dbits(s1) < dbits(P.sink_r2) || dbits(s2) < dbits(P.sink_r2);
             tot[0] = it[IB];
-            if (__any_sync(0xffffffffu, near)) {
+            if (odd || __any_sync(0xffffffffu, near)) {
                 // sink_kernel and the sink terms (physics.rs:388-397, 423-457)
                 auto rate = [&](double r2) {
                     if (!(r2 < P.sink_r2)) return 0.0;
@@ -700,7 +712,7 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
             if constexpr (NF == 4) {
 #pragma unroll
                 for (int f = 1; f < 4; ++f) tot[f] = tot[f] + it[IB + 3 + f];
-            } else if (P.fake_rate != 0.0) {
+            } else if (odd || P.fake_rate != 0.0) {
                 double fk[4] = {0.0, 0.0, 0.0, 0.0};
                 if (!(u[0] < u0[0] * P.fake_thr)) {
 #pragma unroll
@@ -729,6 +741,8 @@ __global__ void __launch_bounds__(S64_THREADS, 2) stage64_kernel(const __grid_co
                 for (int f = 0; f < NF; ++f) uout[f * nn + idx] = out[f];
 #pragma unroll
                 for (int k = 0; k < IB + (NF == 4 ? 7 : 3); ++k) acc[k] += it[k];
+                if constexpr (NF == 4)
+                    if (odd) acc[IB + 7] += u[0] - u[0];   // the mass of cooling
                 if (a.amax_flag) {
                     // max(|vx|, |vy|) + c (physics.rs:521-526, 679-681); NaN speeds are passed over, as f64::max does
                     const Divisor by_rho(out[0]);
