@@ -4,7 +4,7 @@
 // and SM; an integer instruction takes a thirty-second of that.  These give
 // the values of the conversions (round to nearest, ties to even) for
 // magnitudes in [2^-70, 2^127) and leave the others, zero included, to the
-// conversion itself.
+// conversion itself (tests/test_gpu_exact_helpers.py).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -87,6 +87,8 @@ __device__ __forceinline__ bool moderate(double x)
     const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
     return h - 0x26f00000u < 0x32000000u || (h | (unsigned)__double2loint(x)) == 0u;
 }
+// in [2^-400, 2^400)
+__device__ __forceinline__ bool moderate_positive(double x) { return (unsigned)__double2hiint(x) - 0x26f00000u < 0x32000000u; }
 // a magnitude below 2^100: neither infinite nor NaN, and products of a few such values are not either
 __device__ __forceinline__ bool bounded(double x) { return ((unsigned)__double2hiint(x) & 0x7fffffffu) < 0x46300000u; }
 // max(0, x), 0 for NaN
@@ -110,18 +112,19 @@ __device__ __noinline__ double plain_div(double a, double b) { return a / b; }
 // (Markstein 1990, IBM J. Res. Dev. 34; with the divisor known in advance:
 // Brisebarre, Muller & Raina 2004, IEEE Trans. Comput. 53).  Equal to the
 // division in each of 4e8 random quotients, among them divisors and dividends
-// next to powers of two.  Magnitudes far from 1, infinities and NaN take the
-// division itself.
+// next to powers of two (tests/test_gpu_exact_helpers.py).  Negative divisors,
+// magnitudes far from 1, infinities and NaN take the division itself.
 struct Divisor {
     double d, r;
     bool ok;
-    __device__ __forceinline__ explicit Divisor(double d_) : d(d_), r(1.0 / d_), ok(moderate(d_) && d_ != 0.0) {}
-    __device__ __forceinline__ Divisor(double d_, double r_) : d(d_), r(r_), ok(moderate(d_) && d_ != 0.0) {}
+    __device__ __forceinline__ explicit Divisor(double d_) : Divisor(d_, 1.0 / d_) {}
+    __device__ __forceinline__ Divisor(double d_, double r_)
+        : d(d_), r(r_), ok(moderate_positive(d_)) {}
     __device__ __forceinline__ double operator()(double x) const
     {
         if (!(ok && moderate(x))) return plain_div(x, d);
         const double q = __dmul_rn(x, r);
-        return __fma_rn(__fma_rn(-q, d, x), r, q);
+        return __fma_rn(-__fma_rn(q, d, -x), r, q);   // (as q + (x - q d) r, -0 / d would come out as +0)
     }
 };
 
@@ -129,8 +132,8 @@ struct Divisor {
 // with e = x - f w (exact in a fused step) it is f + e / w, which one fused step
 // rounds.  1 / w to rounding: the 20 bits of the approximate reciprocal and one
 // cubic step, 1 + d + d^2 of the residual d (Householder).  Equal to the two
-// operations in each of 2e8 random pairs; three operations a quotient and three
-// for w in place of four and a division.
+// operations in each of 2e8 random pairs (tests/test_gpu_exact_helpers.py); three
+// operations a quotient and three for w in place of four and a division.
 struct ThereAndBack {
     double w, r;
     bool ok;
