@@ -1935,12 +1935,15 @@ extern "C" b2d_status b2d_autotune(b2d_ctx* ctx, int32_t fold, int32_t reps, int
         // one whose chunks take up half the GPU (they would only be longer), nor
         // below a quarter of one that still fills it (four guard rows a chunk)
         const long long slots = resident_ctas(ctx);
-        int max_bs = 0;
-        for (const RunHost& r : ctx->runs) max_bs = std::max(max_bs, r.bs);
-        for (int h = 1; h <= std::min(max_bs, 128); ++h) {
-            if (!tile_ok(ctx, ctx->tw, h)) continue;
-            if (h < 16 && 2 * h <= max_bs && chunk_ctas(ctx, h) > 2 * slots) continue;
-            if (4 * h <= max_bs && chunk_ctas(ctx, 4 * h) > slots) continue;
+        auto divides = [&](int h) {
+            return std::all_of(ctx->runs.begin(), ctx->runs.end(), [h](const RunHost& r) { return r.bs % h == 0; });
+        };
+        int tallest = 128;   // of those that divide the blocks of every run: it is always tried
+        while (!divides(tallest)) --tallest;
+        for (int h = 1; h <= tallest; ++h) {
+            if (!divides(h)) continue;
+            if (h < 16 && 2 * h <= tallest && chunk_ctas(ctx, h) > 2 * slots) continue;
+            if (4 * h <= tallest && chunk_ctas(ctx, 4 * h) > slots) continue;
             st = trial(h, 0);
             if (st != B2D_OK) return st;
             if (2 * chunk_ctas(ctx, h) <= slots) break;
