@@ -1319,7 +1319,7 @@ static __device__ __noinline__ double tracer_wrap(double xo, double R)
 // x + (hi + lo), or with a base xb + w (x + (hi + lo) - xb) on the base's
 // periodic image, wrapped into [-R, R).
 __device__ __forceinline__ double tracer_move(double x, float xh, float xl, float d, bool has_base, double xb, float2 w,
-                                              double R, float Rf)
+                                              double R, float2 Rf)
 {
     double xo;
     if (!has_base) xo = x + widen(d);
@@ -1330,8 +1330,9 @@ __device__ __forceinline__ double tracer_move(double x, float xh, float xl, floa
         float dd = __fadd_rn(xh, -bh);
         const float ee = __fadd_rn(dd, -xh);
         float l = __fadd_rn(__fadd_rn(__fadd_rn(xh, -__fadd_rn(dd, -ee)), -__fadd_rn(bh, ee)), __fadd_rn(xl, -bl));
-        if (dd > Rf) dd = __fadd_rn(dd, -2.0f * Rf);
-        else if (dd < -Rf) dd = __fadd_rn(dd, 2.0f * Rf);
+        // (exact in the high word; the radius has a low one too)
+        if (dd > Rf.x) { dd = __fadd_rn(dd, -2.0f * Rf.x); l = __fadd_rn(l, -2.0f * Rf.y); }
+        else if (dd < -Rf.x) { dd = __fadd_rn(dd, 2.0f * Rf.x); l = __fadd_rn(l, 2.0f * Rf.y); }
         const float h = __fadd_rn(dd, d), bb = __fadd_rn(h, -dd);
         l = __fadd_rn(l, __fadd_rn(__fadd_rn(dd, -__fadd_rn(h, -bb)), __fadd_rn(d, -bb)));
         // times w
@@ -1420,7 +1421,8 @@ __global__ void __launch_bounds__(256) tracer_kernel(const RunDev* runs, int run
         const float w00 = bx * by, w10 = ax * by, w01 = bx * ay, w11 = ax * ay;
         const float vx = w00 * v00.x + w10 * v10.x + w01 * v01.x + w11 * v11.x;
         const float vy = w00 * v00.y + w10 * v10.y + w01 * v01.y + w11 * v11.y;
-        const float dtf = narrow(dt), Rf = rd.tracer_radius.x;
+        const float dtf = narrow(dt);
+        const float2 Rf = rd.tracer_radius;
         xo = tracer_move(at.x, xh, xl, dtf * vx, base_slot >= 0, base.x, w, R, Rf);
         yo = tracer_move(at.y, yh, yl, dtf * vy, base_slot >= 0, base.y, w, R, Rf);
     }
