@@ -287,12 +287,6 @@ struct RunHost {
     std::vector<double> hxc;
 };
 
-// Host mirror of the per-context control block in device memory.
-struct Control {
-    b2d_error err;
-    int pad_[2];
-};
-
 struct StagePlan {
     int in, base, out;
     double bf;
@@ -343,7 +337,6 @@ struct b2d_ctx {
     std::map<std::pair<int, int>, cudaGraphExec_t> graphs;
     long long launches = 0;
     int total_tiles = 0;
-    int pending_final = -1;
     // instrumentation
     bool instrument = false;
     std::vector<cudaEvent_t> ev;
@@ -528,8 +521,6 @@ static void free_ctx(b2d_ctx* ctx)
     delete ctx;
 }
 
-constexpr int STRIP_COLS = 60;   // SW_COLS of the FP32 kernel (stagew.cuh)
-
 // Row chunks per column strip of a run: block-aligned tiles of height th, or,
 // with strip rows set, ceil(N / rows) chunks that may cross block boundaries.
 static int row_chunks(const b2d_ctx* ctx, const RunHost& r)
@@ -611,13 +602,7 @@ static b2d_status sync_rundev(b2d_ctx* ctx)
             d.tiles_j = (r.N + STRIP_COLS - 1) / STRIP_COLS;
             d.ntiles = d.tiles_i * d.tiles_j;
             base += d.ntiles;
-            // ledger pieces of the block with the most: the chunks of its rows times the strips of its columns
-            int rows = 0, cols = 0;
-            for (int b = 0; b < r.nb; ++b) {
-                rows = std::max(rows, chunks_in_block_row(b, r.bs, r.N, d.chunks));
-                cols = std::max(cols, (b * r.bs + r.bs - 1) / STRIP_COLS - b * r.bs / STRIP_COLS + 1);
-            }
-            d.tiles_per_block = rows * cols;
+            d.tiles_per_block = most_strip_pieces(r.bs, r.nb, d.chunks);
         }
     }
     ctx->total_tiles = base;
@@ -1243,7 +1228,6 @@ static b2d_status launch_stage(b2d_ctx* ctx, const StagePlan& sp, int stage, int
     a.tile_bases = ctx->d_bases;
     a.nruns = ctx->nruns;
     a.pf1 = ctx->rdev_h[0].pf;
-    a.th = ctx->th;
     a.in_slot = sp.in;
     a.base_slot = sp.base;
     a.out_slot = sp.out;
@@ -2256,7 +2240,6 @@ extern "C" b2d_status b2d_stage_noalloc(const b2d_config* cfg, const double* d_i
     a.tile_bases = nullptr;
     a.nruns = 1;
     a.pf1 = rd.pf;
-    a.th = sub_h;
     a.in_slot = 0;
     a.base_slot = d_base ? 1 : -1;
     a.out_slot = 2;

@@ -63,7 +63,6 @@ struct StageArgs {
     const RunDev* runs;
     const int* tile_bases;   // [nruns] first CTA of each run
     int nruns;
-    int th;
     int in_slot, base_slot, out_slot;
     int stage;
     int amax_flag;
@@ -90,6 +89,26 @@ __host__ __device__ inline int chunk_of_row(int r, int N, int C)
 __host__ __device__ inline int chunks_in_block_row(int b, int bs, int N, int C)
 {
     return chunk_of_row((b + 1) * bs - 1, N, C) - chunk_of_row(b * bs, N, C) + 1;
+}
+
+// The FP32 kernel's strips are this many columns wide.  Its ledger piece of a
+// strip and chunk for a block under both: the block's strips from left to right,
+// and the chunks of its rows (nc of them from `first`) in each.
+constexpr int STRIP_COLS = 60;
+__host__ __device__ inline int strip_piece(int strip, int chunk, int block_column, int bs, int nc, int first)
+{
+    return (strip - block_column * bs / STRIP_COLS) * nc + chunk - first;
+}
+// pieces of the block that has the most
+inline int most_strip_pieces(int bs, int nb, int C)
+{
+    int rows = 0, cols = 0;
+    for (int b = 0; b < nb; ++b) {
+        const int n = chunks_in_block_row(b, bs, nb * bs, C), m = (b * bs + bs - 1) / STRIP_COLS - b * bs / STRIP_COLS + 1;
+        if (n > rows) rows = n;
+        if (m > cols) cols = m;
+    }
+    return rows * cols;
 }
 
 // The ledger pieces of a block in a stage.

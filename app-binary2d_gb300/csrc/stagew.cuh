@@ -74,7 +74,6 @@
 
 namespace b2d {
 
-constexpr int SW_COLS = 60;              // columns of a strip
 constexpr int SW_SLOTS = 4;              // stencil ring: rows n - 2 (for its update) to n + 1
 constexpr int SW_USLOTS = 2;             // update rows: one in use, one ahead
 
@@ -465,7 +464,7 @@ __device__ __noinline__ void flush_strip(const RunDev& rd, int stage, int strip,
     constexpr int NL = NITEMS * NF, K = NF == 3 ? 16 : 32;
     const int lane = threadIdx.x & 31;
     const int N = rd.N, bs = rd.bs;
-    const int j0 = strip * SW_COLS, w = min(SW_COLS, N - j0), c0 = 2 * lane - 2;
+    const int j0 = strip * STRIP_COLS, w = min(STRIP_COLS, N - j0), c0 = 2 * lane - 2;
     const int nc = chunks_in_block_row(brow, bs, N, rd.chunks), first_chunk = chunk_of_row(brow * bs, N, rd.chunks);
     for (int b = j0 / bs; b <= (j0 + w - 1) / bs; ++b) {
         const int lo = max(b * bs - j0, 0), hi = min(b * bs + bs - j0, w);
@@ -482,7 +481,7 @@ __device__ __noinline__ void flush_strip(const RunDev& rd, int stage, int strip,
         }
         const float s = warp_sum_items<K>(v, lane);
         const int m = item_of_lane<K>(lane);
-        const int piece = (strip - b * bs / SW_COLS) * nc + ti - first_chunk;
+        const int piece = strip_piece(strip, ti, b, bs, nc, first_chunk);
         if ((lane & (32 / K - 1)) == 0 && m < T::ITEMS)
             stage_pieces(rd, stage, brow * rd.nb + b, NL)[(size_t)piece * NL + ledger_word<NF>(m)] = (double)s;
     }
@@ -579,7 +578,7 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
     const int lt = g - rd.tile_base;
     const int strip = lt % rd.tiles_j, ti = rd.chunk0 + lt / rd.tiles_j;
     const int i0 = chunk_start(ti, N, rd.chunks), TH = chunk_start(ti + 1, N, rd.chunks) - i0;
-    const int j0 = strip * SW_COLS, w = min(SW_COLS, N - j0);
+    const int j0 = strip * STRIP_COLS, w = min(STRIP_COLS, N - j0);
     const int c0 = 2 * lane - 2;                            // this lane's columns c0, c0 + 1
     const bool inx = c0 >= 0 && c0 < w, iny = EVEN ? inx : c0 >= 0 && c0 + 1 < w;
     const bool has_base = a.base_slot >= 0;
