@@ -783,7 +783,10 @@ extern "C" b2d_ctx* b2d_create(const b2d_config* cfgs, int32_t nruns, int32_t pr
         // the buffer's rate depends on the zone's place only, and takes an
         // FP64 root, division and tanh: a table, 8 bytes a zone beside the
         // run's 144 or 192 (without the memory for it, the stages compute it)
-        for (int i = 0; i < nruns; ++i) {
+        size_t tables = 0, free_bytes = 0, total_bytes = 0;
+        for (const RunHost& r : ctx->runs) tables += sizeof(double) * (size_t)r.N * r.N;
+        CREATE_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+        for (int i = 0; i < nruns && room_for_tables(free_bytes, total_bytes, tables); ++i) {
             RunHost& r = ctx->runs[i];
             if (cudaMalloc(&r.buffer, sizeof(double) * (size_t)r.N * r.N) != cudaSuccess) {
                 cudaGetLastError();

@@ -111,6 +111,15 @@ inline int most_strip_pieces(int bs, int nb, int C)
     return rows * cols;
 }
 
+// Whether a context keeps tables that its stages can do without: where they
+// leave half of the GPU's memory free.  Pipelined transfers allocate two thirds
+// of what a context holds after it was made, tracers 64 bytes each; a mesh that
+// fits with them must not fail for a table.
+inline bool room_for_tables(size_t free_bytes, size_t total_bytes, size_t tables)
+{
+    return free_bytes >= tables && free_bytes - tables >= total_bytes / 2;
+}
+
 // The ledger pieces of a block in a stage.
 __host__ __device__ inline double* stage_pieces(const RunDev& rd, int stage, int block, int words)
 {
