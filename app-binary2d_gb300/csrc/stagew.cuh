@@ -87,7 +87,7 @@ enum {
     C_TN, C_TT, C_VISC,      // 4/3 + lambda, -2/3 + lambda; theta c / dx of the cell's stress
     C_CM1, C_CM2,            // m / Mach^2
     C_M1, C_M2, C_NM1DT, C_NM2DT, C_SOFT2,
-    C_BUF_SLOPE, C_BUF_OFFSET, C_BUF_RATE, C_NDT_DX, C_GAMMA, C_GM1, C_INV_GM1, C_COOL, C_ALPHA, C_COUNT
+    C_BUF_SLOPE, C_RADIUS, C_BUF_RATE, C_NDT_DX, C_GAMMA, C_GM1, C_INV_GM1, C_COOL, C_ALPHA, C_COUNT
 };
 
 // How a warp copies its rows: a word, a pair of columns or four columns at a
@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
         K[C_NM2DT] = f2(__fmul_rn(-B.p2.m, dt));
         K[C_SOFT2] = f2(P.soft2);
         K[C_BUF_SLOPE] = f2(__fmul_rn(-2.0f * P.inv_buffer_scale, log2e));
-        K[C_BUF_OFFSET] = f2(__fmul_rn(__fmul_rn(2.0f * P.inv_buffer_scale, log2e), P.domain_radius));
+        K[C_RADIUS] = f2(P.domain_radius);
         K[C_BUF_RATE] = f2(__fmul_rn(-2.0f * dt, P.half_rate_omega));
         K[C_NDT_DX] = f2(__fmul_rn(-P.inv_dx, dt));
         K[C_GAMMA] = f2(P.gamma);
@@ -974,7 +974,8 @@ __global__ void __launch_bounds__(32, SWShape<NF, STORE, COPY>::CTAS) stagew_ker
                     constexpr int G2 = NF - 1, BU = 2 * (NF - 1);
                     // buffer: 0.5 rate (1 + tanh(y)) Omega_outer, y = (r - R) / scale, 1 + tanh(y) = 2 / (1 + exp(-2y))
                     const float2 yc2 = S.yc[lane], rr2 = fma2(yc2, yc2, S.rows[R_XX][rt - 1]);
-                    const float2 yb = fma2(sqrt2(rr2), K[C_BUF_SLOPE], K[C_BUF_OFFSET]);
+                    // (r - R first: r / scale - R / scale is NaN for a scale of 0, a sharp edge, and rounds twice)
+                    const float2 yb = mul2(sub2(sqrt2(rr2), K[C_RADIUS]), K[C_BUF_SLOPE]);
                     const float2 den = add2(K[C_ONE], make_float2(exp2_fast(yb.x), exp2_fast(yb.y)));
                     const float2 kb = mul2(K[C_BUF_RATE], rcp2(den));
 #pragma unroll
