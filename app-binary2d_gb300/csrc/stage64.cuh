@@ -41,12 +41,12 @@
 // three (85 registers) or one of 512 threads were 1-19 % slower.
 //
 // Measured per stage, against the marching kernel it took the place of (one
-// thread per column of a block's 64 rows): isothermal 2048^2 10.6 -> 3.15 ms,
-// 384^2 (6 x 6 blocks of 64^2) 2.97 -> 0.131 ms; Euler 256^2 with the T^4 law
+// thread per column of a block's 64 rows): isothermal 2048^2 10.6 -> 3.10 ms,
+// 384^2 (6 x 6 blocks of 64^2) 2.97 -> 0.130 ms; Euler 256^2 with the T^4 law
 // 3.79 -> 0.119 ms (of which the upwind fluxes' quotients and y loops that begin
 // with the warps that had fewer x faces: 3.18 -> 3.15, 0.134 -> 0.131 and 0.123 ->
-// 0.119 ms).  At 2048^2 the FP64 pipe is 84 % busy with about 395 operations per
-// zone; 2.65 ms would be all of it.
+// 0.119 ms; one range test fewer in the quotients: 3.15 -> 3.10 ms).  With about
+// 395 operations per zone 2.65 ms would be all of the FP64 pipe at 2048^2.
 #pragma once
 
 #include "stage.cuh"

@@ -41,19 +41,19 @@
 //    pieces of all stages are folded, in order, after the last of them: a fence,
 //    a counter and a fold in the stage's tail cost it about 5 us.
 //
-// What bounds it: instruction issue (680 warp instructions per row of 60
+// What bounds it: instruction issue (620 warp instructions per row of 60
 // columns and isothermal first stage, guard rows and set-up included, 290 of
 // them packed or special-function arithmetic and min / max; a warp in flight
-// waits 4.4 cycles per instruction and a scheduler has three), not memory (4.0
-// of 6.7 TB/s).  Measured per stage, with the kernels that it took the place of,
-// as this file began, and now:
+// waits 4.5 cycles per instruction and a scheduler has three), not memory (4.0
+// of 6.7 TB/s).  Measured per stage of queued advances, with the kernels that it
+// took the place of, as this file began, and now:
 //   isothermal 2048^2          127 -> 109 -> 71 us (10 warps a CTA in step over 512 columns)
-//   isothermal 384^2            33 -> 22 -> 12.1 us
-//   the sweep of 64 runs      1050 -> 690 -> 512 us
-//   Euler 4096^2               650 -> 550 -> 361 us
-//   Euler 768^2                 48 -> 42 -> 26.6 us
-//   blocks of 50^2, RK3, alpha 163 -> 25 -> 11.9 us (a thread per column of a block)
-//   FP64 state 1024^2          106 -> 94 -> 39 us
+//   isothermal 384^2            33 -> 22 -> 11.6 us
+//   the sweep of 64 runs      1050 -> 690 -> 520 us
+//   Euler 4096^2               650 -> 550 -> 365 us
+//   Euler 768^2                 48 -> 42 -> 26.0 us
+//   blocks of 50^2, RK3, alpha 163 -> 25 -> 10.3 us (a thread per column of a block)
+//   FP64 state 1024^2          106 -> 94 -> 38 us
 // Of this, forming FP32 pairs of FP64 words and widening increments with integer
 // instructions gave the FP64 state 47 us where the FP64 pipe's conversions take 50
 // to 70, and letting a stage begin in the last row of the one before 12.5 -> 12.1
